@@ -2,10 +2,11 @@
 // internal force with the J2 return map, Gauss-point stress, material-point
 // batch update and the adjoint sensitivity.
 //
-// Assembly is deterministic without floating-point atomics: elements are
-// processed colour by colour (no two elements of one colour share a node), and
-// inside a colour every matrix or vector entry has exactly one writer, so each
-// entry receives its contributions in the fixed colour order.
+// Assembly is deterministic without floating-point atomics: the stiffness is
+// assembled by block rows, each value summed by one thread in ascending element
+// order and written once; the vector scatters process elements colour by colour
+// (no two elements of one colour share a node), so every entry receives its
+// contributions in the fixed colour order.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -18,137 +19,510 @@ namespace ufc {
 
 namespace {
 
-constexpr int kWarpsPerCta = 4;
+// ---- stiffness assembly by block rows
+//
+// Every stored block (i, j) is the sum, over the elements that hold both nodes,
+// of sum_gp w detJ B_i^T D B_j.  A CTA owns half a SELL slice (16 block rows),
+// accumulates them in shared memory and writes each stored value once; nothing
+// is read back and no two threads touch the same entry, so there are no
+// atomics, no colour passes and no zero fill, and each entry receives its
+// contributions in ascending element order (bitwise reproducible).
+//
+// A warp works on 4 rows at a time, 8 lanes per row.  For the row's k-th
+// element, lane t first takes Gauss point t (its scaled inverse Jacobian
+// adj(J)/sqrt(detJ) goes to shared memory: with that scaling on both sides the
+// weight detJ needs no separate product), then takes the element's node t and
+// forms the block (row node, node t) over the 8 Gauss points.  Lane t's node
+// is the one whose natural coordinates have the sign bits t, and the trilinear
+// factor of node t at Gauss point g equals that of node g at Gauss point t, so
+// one table of 12 products per lane serves the Jacobian and the gradients.
+// The linear-elastic block is formed from G = sum_gp g_a (x) g_b as
+// lam G + mu G^T + mu tr(G) I (72 + 21 FP64 operations per block instead of
+// about 320 when D is applied at every Gauss point); the J2 block as
+// sum_gp (D B_a)^T B_b with D B_a formed once per (row, element, Gauss point).
+//
+// What bounds it: FP64 issue and the shared-memory pipe, about equally (per row
+// and element 250 FP64 operations a lane and some 150 shared-memory wavefronts a
+// warp).  Recomputing an element's Jacobians for each of its 8 rows costs less
+// than the read-modify-write of the values that an element-wise scatter needs
+// (16.6 GB at 192x96x96, in 8 colour passes).
+constexpr int kAsmRows = 16;                // rows per CTA
+constexpr int kAsmWarps = kAsmRows / 4;
+constexpr int kAsmMaxSmem = 227 * 1024;     // dynamic shared memory of one CTA
 
-// Node pairs (a <= b) of the upper triangle of the 8x8 block grid of Ke.
-__constant__ int8_t c_pair_a[36];
-__constant__ int8_t c_pair_b[36];
+// Lane t's node (Abaqus order) has the natural-coordinate sign bits t; the map is its own inverse.
+__host__ __device__ constexpr int bits_node(int t) { return t ^ ((t >> 1) & 1); }
 
-struct PairTable {
-  int8_t a[36], b[36];
-  PairTable() {
-    int k = 0;
-    for (int i = 0; i < 8; ++i)
-      for (int j = i; j < 8; ++j) {
-        a[k] = (int8_t)i;
-        b[k] = (int8_t)j;
-        ++k;
-      }
-  }
+// Upper triangle of a symmetric 6x6, row by row: entry (i, j), i <= j.
+__host__ __device__ constexpr int tri6(int i, int j) {
+  const int lo = i < j ? i : j, hi = i < j ? j : i;
+  return lo * 6 - lo * (lo - 1) / 2 + hi - lo;
+}
+
+// Shared memory of one warp.
+template <typename T, bool kTangent>
+struct AsmWarp {
+  T X[4][26];                             // element coordinates by sign bits, [row][3 bits + i], padded
+  T P[4][8][kTangent ? 28 : 10];          // [row][gp]: scaled inverse Jacobian (9), then D B_a (18) for J2
 };
 
 template <typename T>
-struct WarpSmem {
-  T X[24];
-  T g[8][8][3];  // [gp][node][dir] physical gradients
-  T wdet[8];
-  T D[8][36];    // per-Gauss-point tangent (J2 only)
+__device__ __forceinline__ T flip_if(T v, bool neg) {
+  return neg ? -v : v;
+}
+
+// Writes the accumulated block rows [half, half + ROWS) of a slice to the SELL
+// values (each written once, ROWS consecutive values per warp load) and the
+// Jacobi diagonal; val_r and dinv_r, when given, take the values rounded to
+// FP32.  Entries in a row or a column of a Dirichlet DOF are zero, its diagonal
+// 1 (symmetric elimination).  init() reads the Dirichlet flags of the first
+// kAhead entries of each thread, so that their latency passes behind the
+// accumulation.
+template <typename T, int ROWS, int THREADS>
+struct RowWriter {
+  static constexpr int kAhead = 8, kStep = THREADS / ROWS;
+  int r, j0, dj;       // row in the tile, first entry of this thread, entry of the diagonal (or -1)
+  int64_t R, P0;       // block row, position of its entry 0
+  unsigned fr, fc;     // Dirichlet flags: of the row (3 bits), of the columns of the first kAhead entries
+
+  __device__ __forceinline__ unsigned flags(const uint8_t* __restrict__ fixed, int64_t node) const {
+    return (fixed[3 * node] ? 1u : 0u) | (fixed[3 * node + 1] ? 2u : 0u) | (fixed[3 * node + 2] ? 4u : 0u);
+  }
+
+  __device__ __forceinline__ void init(int32_t N, int64_t s, int half, int64_t base, int len,
+                                       const int32_t* __restrict__ scol, const int32_t* __restrict__ dpos,
+                                       const uint8_t* __restrict__ fixed) {
+    r = threadIdx.x & (ROWS - 1);
+    j0 = threadIdx.x / ROWS;
+    R = s * kSlice + half + r;
+    P0 = base + half + r;
+    const bool real = R < N;
+    int32_t col[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) col[q] = j0 + q * kStep < len ? scol[P0 + 32 * (int64_t)(j0 + q * kStep)] : 0;
+    fr = real ? flags(fixed, R) : 0u;
+    dj = real ? (int)((dpos[R] - P0) >> 5) : -1;
+    fc = 0;
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) fc |= flags(fixed, col[q]) << (3 * q);
+  }
+
+  __device__ __forceinline__ void write(int len, const int32_t* __restrict__ scol, const uint8_t* __restrict__ fixed,
+                                        const T* acc, int stride, T* __restrict__ val, T* __restrict__ dinv,
+                                        float* __restrict__ val_r, float* __restrict__ dinv_r) const {
+    unsigned f = fc;
+    int q = 0;
+    for (int j = j0; j < len; j += kStep, ++q, f >>= 3) {
+      const int64_t P = P0 + 32 * (int64_t)j;
+      const unsigned m = q < kAhead ? f & 7u : flags(fixed, scol[P]);
+      const T* a = acc + r * stride + 9 * j;
+      const int64_t p = vpos(P, 0);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int jj = 0; jj < 3; ++jj) {
+          T v = (((fr >> i) | (m >> jj)) & 1u) ? T(0) : a[3 * i + jj];
+          if (j == dj && i == jj && ((fr >> i) & 1u)) v = T(1);
+          val[p + 32 * (3 * i + jj)] = v;
+          if (val_r) val_r[p + 32 * (3 * i + jj)] = (float)v;
+          if (j == dj && i == jj) {
+            // Jacobi diag_inv = 1/K_ii, or 1 when |K_ii| <= 1e-30 (NM_LinSolv_Prec_Jacobi_Build,
+            // ufc_core/L2_NM/Solver/LinSolv/NM_Solv_LinPrec.f90:328-353; NM_Solver_PCG uses 1e-30)
+            const T di = fabs((double)v) > 1e-30 ? T(1) / v : T(1);
+            dinv[3 * R + i] = di;
+            if (dinv_r) dinv_r[3 * R + i] = (float)di;
+          }
+        }
+    }
+  }
 };
 
-// Stiffness block K_ab (3x3, row-major) contribution of one Gauss point.
 template <typename T, bool kTangent>
-__device__ __forceinline__ void block_gp(const T* ga, const T* gb, T wd, T lam, T mu, const T* D, T K[9]) {
-  if (!kTangent) {
-    const T dot = ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2];
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        T v = lam * ga[i] * gb[j] + mu * ga[j] * gb[i];
-        if (i == j) v += mu * dot;
-        K[i * 3 + j] += wd * v;
-      }
-  } else {
-    // B column j of a node has non-zeros at Voigt rows kIdx[j][m] with gradient
-    // component kCmp[j][m] (B matrix of PH_Elem_ShapeFunc.f90:225-244).
-    constexpr int kIdx[3][3] = {{0, 3, 5}, {1, 3, 4}, {2, 4, 5}};
-    constexpr int kCmp[3][3] = {{0, 1, 2}, {1, 0, 2}, {2, 1, 0}};
-    T DB[6][3];
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-        DB[k][j] = D[k * 6 + kIdx[j][0]] * gb[kCmp[j][0]] + D[k * 6 + kIdx[j][1]] * gb[kCmp[j][1]] +
-                   D[k * 6 + kIdx[j][2]] * gb[kCmp[j][2]];
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-        K[i * 3 + j] += wd * (ga[kCmp[i][0]] * DB[kIdx[i][0]][j] + ga[kCmp[i][1]] * DB[kIdx[i][1]][j] +
-                              ga[kCmp[i][2]] * DB[kIdx[i][2]][j]);
-  }
-}
+__global__ void __launch_bounds__(kAsmWarps * 32)
+    k_assemble_rows(int32_t N, const int32_t* __restrict__ nptr, const int32_t* __restrict__ nelem,
+                    const double* __restrict__ coords, const int32_t* __restrict__ conn,
+                    const double* __restrict__ lame, const double* __restrict__ Dt, const int32_t* __restrict__ slot,
+                    const int64_t* __restrict__ sptr, const int32_t* __restrict__ scol,
+                    const int32_t* __restrict__ dpos, const uint8_t* __restrict__ fixed, int stride,
+                    T* __restrict__ val, T* __restrict__ dinv, float* __restrict__ val_r, float* __restrict__ dinv_r,
+                    int32_t* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char asm_smem[];
+  using Warp = AsmWarp<T, kTangent>;
+  Warp* wsm = reinterpret_cast<Warp*>(asm_smem);
+  T* acc = reinterpret_cast<T*>(asm_smem + sizeof(Warp) * kAsmWarps);  // [row][stride], 9 per entry, stride odd
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, rr = lane >> 3, t = lane & 7;
+  const int64_t s = blockIdx.x >> 1;
+  const int half = (blockIdx.x & 1) * kAsmRows;
+  const int64_t base = sptr[s];
+  const int len = (int)((sptr[s + 1] - base) >> 5);
+  RowWriter<T, kAsmRows, kAsmWarps * 32> out;
+  out.init(N, s, half, base, len, scol, dpos, fixed);
+  for (int q = threadIdx.x; q < kAsmRows * stride; q += kAsmWarps * 32) acc[q] = T(0);
+  __syncthreads();
 
-// One warp per element of the given colour: Ke = sum_gp w detJ B^T D B, block by
-// block, added into the SELL values of the stiffness.  Entries in a row or a
-// column of a Dirichlet DOF are skipped (symmetric elimination).
-template <typename T, bool kTangent>
-__global__ void __launch_bounds__(kWarpsPerCta * 32)
-    k_assemble(const int32_t* __restrict__ elems, int32_t ne, const double* __restrict__ coords,
-               const int32_t* __restrict__ conn, const double* __restrict__ props, int nprops,
-               const double* __restrict__ Dt, const int32_t* __restrict__ slot, const uint8_t* __restrict__ fixed,
-               T* __restrict__ val, int32_t* __restrict__ err) {
-  __shared__ WarpSmem<T> sm[kWarpsPerCta];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t idx = (int64_t)blockIdx.x * kWarpsPerCta + w;
-  if (idx >= ne) return;
-  const int64_t e = elems[idx];
-  WarpSmem<T>& s = sm[w];
-  if (lane < 24) s.X[lane] = (T)coords[(int64_t)conn[e * 8 + lane / 3] * 3 + lane % 3];
-  if (kTangent) {
-    for (int k = lane; k < 288; k += 32) (&s.D[0][0])[k] = (T)Dt[e * 288 + k];
-  }
-  __syncwarp();
-  if (lane < 8) {
-    T inv[9];
-    const T det = jacobian_inv<T>(s.X, lane, inv);
-    if (!(det > T(0))) atomicOr(err, (int)kDevBadJacobian);
-    s.wdet[lane] = det;
+  Warp& sm = wsm[w];
+  const int64_t row = s * kSlice + half + 4 * w + rr;
+  T* arow = acc + (4 * w + rr) * stride;
+  const int node_t = bits_node(t);
+  // trilinear factors of lane t: c[d][m] = (1/8) prod over the two other
+  // directions of (1 + s_t s_m g), m = the bits of those directions in order
+  const T g = T(0.57735026918962576451);
+  T c[3][4];
+  {
+    const T f0[2] = {T(1) + ((t & 1) ? -g : g), T(1) + ((t & 1) ? g : -g)};
+    const T f1[2] = {T(1) + ((t & 2) ? -g : g), T(1) + ((t & 2) ? g : -g)};
+    const T f2[2] = {T(1) + ((t & 4) ? -g : g), T(1) + ((t & 4) ? g : -g)};
 #pragma unroll
-    for (int a = 0; a < 8; ++a) grad_x<T>(inv, lane, a, s.g[lane][a]);
+    for (int m = 0; m < 4; ++m) {
+      c[0][m] = T(0.125) * f1[m & 1] * f2[m >> 1];
+      c[1][m] = T(0.125) * f0[m & 1] * f2[m >> 1];
+      c[2][m] = T(0.125) * f0[m & 1] * f1[m >> 1];
+    }
   }
-  __syncwarp();
-  T lam = T(0), mu = T(0);
-  if (!kTangent) lame<T>((T)props[e * nprops], (T)props[e * nprops + 1], lam, mu);
-  for (int p = lane; p < 36; p += 32) {
-    const int a = c_pair_a[p], b = c_pair_b[p];
+  const int32_t kb = row < N ? nptr[row] : 0, ke = row < N ? nptr[row + 1] : 0;
+  const int kmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)(ke - kb));
+  bool bad = false;
+  // the element of step k + 1 is fetched while step k is worked on
+  int32_t el = 0, pos = 0;
+  T x0 = T(0), x1 = T(0), x2 = T(0);
+  auto fetch = [&](int k) {
+    if (kb + k >= ke) return;
+    el = nelem[kb + k];
+    const int64_t e = el >> 3;
+    const int64_t nd = conn[e * 8 + node_t];
+    pos = slot[e * 64 + (el & 7) * 8 + node_t];
+    x0 = (T)coords[nd * 3];
+    x1 = (T)coords[nd * 3 + 1];
+    x2 = (T)coords[nd * 3 + 2];
+  };
+  fetch(0);
+  for (int k = 0; k < kmax; ++k) {
+    const bool on = kb + k < ke;
+    const int64_t e = el >> 3;
+    const int ta = bits_node(el & 7);  // the row's own node in sign bits
+    const int j = (int)((pos - base) >> 5);
+    sm.X[rr][3 * t] = x0;
+    sm.X[rr][3 * t + 1] = x1;
+    sm.X[rr][3 * t + 2] = x2;
+    T lam = T(0), mu = T(0), D[kTangent ? 21 : 1];
+    if (on) {
+      if (kTangent) {
+#pragma unroll
+        for (int q = 0; q < 21; ++q) D[kTangent ? q : 0] = (T)Dt[(e * 21 + q) * 8 + t];
+      } else {
+        lam = (T)lame[2 * e];
+        mu = (T)lame[2 * e + 1];
+      }
+    }
+    fetch(k + 1);
+    __syncwarp();
+    if (on) {
+      // Gauss point t: J_di = dx_i / dxi_d from the 4 edges along d
+      const T* X = sm.X[rr];
+      T J[9];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        J[i] = J[3 + i] = J[6 + i] = T(0);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          const int m0 = m & 1, m1 = m >> 1;
+          J[i] += c[0][m] * (X[3 * (1 + 2 * m0 + 4 * m1) + i] - X[3 * (2 * m0 + 4 * m1) + i]);
+          J[3 + i] += c[1][m] * (X[3 * (m0 + 2 + 4 * m1) + i] - X[3 * (m0 + 4 * m1) + i]);
+          J[6 + i] += c[2][m] * (X[3 * (m0 + 2 * m1 + 4) + i] - X[3 * (m0 + 2 * m1) + i]);
+        }
+      }
+      const T a0 = J[4] * J[8] - J[5] * J[7], a3 = J[5] * J[6] - J[3] * J[8], a6 = J[3] * J[7] - J[4] * J[6];
+      const T det = J[0] * a0 + J[1] * a3 + J[2] * a6;
+      bad |= !(det > T(0));
+      const T q = rsqrt(det);
+      T inv[9] = {a0 * q, (J[2] * J[7] - J[1] * J[8]) * q, (J[1] * J[5] - J[2] * J[4]) * q,
+                  a3 * q, (J[0] * J[8] - J[2] * J[6]) * q, (J[2] * J[3] - J[0] * J[5]) * q,
+                  a6 * q, (J[1] * J[6] - J[0] * J[7]) * q, (J[0] * J[4] - J[1] * J[3]) * q};
+      T* P = sm.P[rr][t];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) P[i] = inv[i];
+      if (kTangent) {
+        // D B_a of the row's node at this Gauss point
+        const T b0 = T(1) + ((((ta ^ t) & 1) != 0) ? -g : g), b1 = T(1) + ((((ta ^ t) & 2) != 0) ? -g : g),
+                b2 = T(1) + ((((ta ^ t) & 4) != 0) ? -g : g);
+        const T d0 = flip_if(T(0.125) * b1 * b2, !(ta & 1)), d1 = flip_if(T(0.125) * b0 * b2, !(ta & 2)),
+                d2 = flip_if(T(0.125) * b0 * b1, !(ta & 4));
+        T ga[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) ga[i] = inv[3 * i] * d0 + inv[3 * i + 1] * d1 + inv[3 * i + 2] * d2;
+        // B column i of a node has non-zeros at Voigt rows kIdx[i][m] with
+        // gradient component kCmp[i][m] (PH_Elem_ShapeFunc.f90:225-244)
+        constexpr int kIdx[3][3] = {{0, 3, 5}, {1, 3, 4}, {2, 4, 5}};
+        constexpr int kCmp[3][3] = {{0, 1, 2}, {1, 0, 2}, {2, 1, 0}};
+#pragma unroll
+        for (int v = 0; v < 6; ++v)
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+            P[(kTangent ? 9 : 0) + v * 3 + i] = D[kTangent ? tri6(v, kIdx[i][0]) : 0] * ga[kCmp[i][0]] +
+                                                D[kTangent ? tri6(v, kIdx[i][1]) : 0] * ga[kCmp[i][1]] +
+                                                D[kTangent ? tri6(v, kIdx[i][2]) : 0] * ga[kCmp[i][2]];
+      }
+    }
+    __syncwarp();
     T K[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) K[k] = T(0);
-    if (kTangent) {
-#pragma unroll 1
-      for (int gp = 0; gp < 8; ++gp) block_gp<T, true>(s.g[gp][a], s.g[gp][b], s.wdet[gp], lam, mu, s.D[gp], K);
-    } else {
+    for (int i = 0; i < 9; ++i) K[i] = T(0);
 #pragma unroll
-      for (int gp = 0; gp < 8; ++gp) block_gp<T, false>(s.g[gp][a], s.g[gp][b], s.wdet[gp], lam, mu, s.D[gp], K);
+    for (int gp = 0; gp < 8; ++gp) {
+      const T* P = sm.P[rr][gp];
+      const int p0 = gp & 1, p1 = (gp >> 1) & 1, p2 = gp >> 2;
+      const T d0 = flip_if(c[0][p1 + 2 * p2], !(t & 1)), d1 = flip_if(c[1][p0 + 2 * p2], !(t & 2)),
+              d2 = flip_if(c[2][p0 + 2 * p1], !(t & 4));
+      T gb[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) gb[i] = P[3 * i] * d0 + P[3 * i + 1] * d1 + P[3 * i + 2] * d2;
+      if (kTangent) {
+        constexpr int kIdx[3][3] = {{0, 3, 5}, {1, 3, 4}, {2, 4, 5}};
+        constexpr int kCmp[3][3] = {{0, 1, 2}, {1, 0, 2}, {2, 1, 0}};
+        const T* M = P + (kTangent ? 9 : 0);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int jj = 0; jj < 3; ++jj)
+            K[3 * i + jj] += M[kIdx[jj][0] * 3 + i] * gb[kCmp[jj][0]] + M[kIdx[jj][1] * 3 + i] * gb[kCmp[jj][1]] +
+                             M[kIdx[jj][2] * 3 + i] * gb[kCmp[jj][2]];
+      } else {
+        T ga[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) ga[i] = __shfl_sync(0xffffffffu, gb[i], ta, 8);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int jj = 0; jj < 3; ++jj) K[3 * i + jj] += ga[i] * gb[jj];
+      }
     }
-    const int64_t na = conn[e * 8 + a], nb = conn[e * 8 + b];
-    const int64_t P = slot[e * 64 + a * 8 + b];
-    bool fa[3], fb[3];
+    if (on) {
+      T* d = arow + 9 * j;
+      if (kTangent) {
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      fa[r] = fixed[3 * na + r] != 0;
-      fb[r] = fixed[3 * nb + r] != 0;
+        for (int i = 0; i < 9; ++i) d[i] += K[i];
+      } else {
+        const T tr = mu * (K[0] + K[4] + K[8]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int jj = 0; jj < 3; ++jj) {
+            T v = lam * K[3 * i + jj] + mu * K[3 * jj + i];
+            if (i == jj) v += tr;
+            d[3 * i + jj] += v;
+          }
+      }
     }
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if (!fa[r] && !fb[c]) val[vpos(P, r * 3 + c)] += K[r * 3 + c];
-    if (a != b) {
-      const int64_t Q = slot[e * 64 + b * 8 + a];
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          if (!fb[r] && !fa[c]) val[vpos(Q, r * 3 + c)] += K[c * 3 + r];
-    }
+    __syncwarp();  // the warp's shared memory is consumed
   }
+  if (bad) atomicOr(err, (int)kDevBadJacobian);
+  __syncthreads();
+
+  out.write(len, scol, fixed, acc, stride, val, dinv, val_r, dinv_r);
 }
 
-__global__ void k_round_values(int64_t n, const double* __restrict__ v64, float* __restrict__ v32) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    v32[i] = (float)v64[i];
+// The linear-elastic assembly with one thread per (block row, element): the
+// whole element is worked through in registers (72 accumulators of the row's 8
+// blocks), so the lanes exchange nothing and shared memory only takes the
+// element coordinates and the finished blocks.  A CTA owns one SELL slice of 32
+// rows; warp q takes the elements k = q, q + 4, ... of all 32 rows, and the
+// warps add their blocks in turn (named barriers pass the turn on), so each
+// entry still receives its contributions in ascending element order.  The
+// coordinates of a thread's next element come by cp.async while the current one
+// is worked on.
+constexpr int kIsoWarps = 4;
+constexpr int kIsoThreads = kIsoWarps * 32;
+constexpr int kIsoXBytes = kIsoWarps * 2 * 24 * 32 * (int)sizeof(double);  // [warp][stage][coordinate][lane]
+
+__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+               : "memory");
+}
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kIsoThreads, 2)
+    k_assemble_iso(int32_t N, const int32_t* __restrict__ nptr, const int32_t* __restrict__ nelem,
+                   const double* __restrict__ coords, const int32_t* __restrict__ conn,
+                   const double* __restrict__ lame, const int32_t* __restrict__ slot,
+                   const int64_t* __restrict__ sptr, const int32_t* __restrict__ scol,
+                   const int32_t* __restrict__ dpos, const uint8_t* __restrict__ fixed, int stride,
+                   T* __restrict__ val, T* __restrict__ dinv, float* __restrict__ val_r, float* __restrict__ dinv_r,
+                   int32_t* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char asm_smem[];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double* xs = reinterpret_cast<double*>(asm_smem) + w * (2 * 24 * 32) + lane;
+  T* acc = reinterpret_cast<T*>(asm_smem + kIsoXBytes);  // [row][stride]
+  const int64_t s = blockIdx.x;
+  const int64_t base = sptr[s];
+  const int len = (int)((sptr[s + 1] - base) >> 5);
+  for (int i = threadIdx.x; i < kSlice * stride; i += kIsoThreads) acc[i] = T(0);
+  const int64_t row = s * kSlice + lane;
+  const int32_t ke = row < N ? nptr[row + 1] : 0;
+  int32_t k = (row < N ? nptr[row] : 0) + w;
+  const int rounds =
+      ((int)__reduce_max_sync(0xffffffffu, (unsigned)(row < N ? ke - (k - w) : 0)) + kIsoWarps - 1) / kIsoWarps;
+  const T g = T(0.57735026918962576451);
+  const T hp = T(0.5) + T(0.5) * g, hm = T(0.5) - T(0.5) * g;  // (1 +- g) / 2
+  bool bad = false;
+  // an element's coordinates into this thread's column of stage r, by sign bits (xi fastest)
+  auto load_x = [&](const int4& n0, const int4& n1, int r) {
+    const int32_t nd[8] = {n0.x, n0.y, n0.w, n0.z, n1.x, n1.y, n1.w, n1.z};
+    double* dst = xs + (r & 1) * (24 * 32);
+#pragma unroll
+    for (int m = 0; m < 8; ++m)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) cp_async8(dst + 32 * (3 * m + i), coords + (int64_t)nd[m] * 3 + i);
+  };
+  int32_t el = k < ke ? nelem[k] : 0, el_next = k + kIsoWarps < ke ? nelem[k + kIsoWarps] : 0;
+  if (k < ke) {
+    const int4* cn = reinterpret_cast<const int4*>(conn + (int64_t)(el >> 3) * 8);
+    load_x(cn[0], cn[1], 0);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  RowWriter<T, kSlice, kIsoThreads> out;
+  out.init(N, s, 0, base, len, scol, dpos, fixed);
+  __syncthreads();
+#pragma unroll 1
+  for (int r = 0; r < rounds; ++r) {
+    const bool on = k < ke, more = k + kIsoWarps < ke;
+    const int64_t e = el >> 3;
+    const int a = el & 7, ta = bits_node(a);
+    const double* X = xs + (r & 1) * (24 * 32);
+    int4 n0 = make_int4(0, 0, 0, 0), n1 = n0;
+    if (more) {
+      const int4* cn = reinterpret_cast<const int4*>(conn + (int64_t)(el_next >> 3) * 8);
+      n0 = cn[0];
+      n1 = cn[1];
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    T G[8][9];
+#pragma unroll
+    for (int b = 0; b < 8; ++b)
+#pragma unroll
+      for (int i = 0; i < 9; ++i) G[b][i] = T(0);
+#pragma unroll 1
+    for (int iz = 0; iz < 2; ++iz) {
+      const T fz = ((ta >> 2) == iz) ? hp : hm;  // factors (1 + s g) / 2 of the row's node
+      const T tz = iz ? hp : hm;                 // the Gauss point's position on the edge
+#pragma unroll 1
+      for (int iy = 0; iy < 2; ++iy) {
+        if (!on) continue;
+        const T fy = (((ta >> 1) & 1) == iy) ? hp : hm, ty = iy ? hp : hm;
+        // at the Gauss point's eta and zeta, for xi = -1 and +1: value, half
+        // eta-derivative, half zeta-derivative of the coordinates
+        T v[2][3], dy[2][3], dz[2][3];
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const T x00 = (T)X[32 * (3 * x + i)], x10 = (T)X[32 * (3 * (x + 2) + i)],
+                    x01 = (T)X[32 * (3 * (x + 4) + i)], x11 = (T)X[32 * (3 * (x + 6) + i)];
+            const T d0 = x01 - x00, d1 = x11 - x10;
+            const T v0 = x00 + tz * d0, v1 = x10 + tz * d1;
+            dz[x][i] = T(0.5) * (d0 + ty * (d1 - d0));
+            dy[x][i] = T(0.5) * (v1 - v0);
+            v[x][i] = v0 + ty * (v1 - v0);
+          }
+        // products of the element nodes' factors in eta and zeta: [same or opposite side of the Gauss point]
+        const T pyz[4] = {T(0.5) * ((iy ? hm : hp) * (iz ? hm : hp)), T(0.5) * ((iy ? hp : hm) * (iz ? hm : hp)),
+                          T(0.5) * ((iy ? hm : hp) * (iz ? hp : hm)), T(0.5) * ((iy ? hp : hm) * (iz ? hp : hm))};
+#pragma unroll 1
+        for (int ix = 0; ix < 2; ++ix) {
+          const T fx = ((ta & 1) == ix) ? hp : hm, tx = ix ? hp : hm;
+          T J[9];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            J[i] = T(0.5) * (v[1][i] - v[0][i]);
+            J[3 + i] = dy[0][i] + tx * (dy[1][i] - dy[0][i]);
+            J[6 + i] = dz[0][i] + tx * (dz[1][i] - dz[0][i]);
+          }
+          const T c0 = J[4] * J[8] - J[5] * J[7], c3 = J[5] * J[6] - J[3] * J[8], c6 = J[3] * J[7] - J[4] * J[6];
+          const T det = J[0] * c0 + J[1] * c3 + J[2] * c6;
+          bad |= !(det > T(0));
+          const T sc = rsqrt(det);
+          const T inv[9] = {c0 * sc, (J[2] * J[7] - J[1] * J[8]) * sc, (J[1] * J[5] - J[2] * J[4]) * sc,
+                            c3 * sc, (J[0] * J[8] - J[2] * J[6]) * sc, (J[2] * J[3] - J[0] * J[5]) * sc,
+                            c6 * sc, (J[1] * J[6] - J[0] * J[7]) * sc, (J[0] * J[4] - J[1] * J[3]) * sc};
+          const T a0 = flip_if(T(0.5) * (fy * fz), !(ta & 1)), a1 = flip_if(T(0.5) * (fx * fz), !(ta & 2)),
+                  a2 = flip_if(T(0.5) * (fx * fy), !(ta & 4));
+          T ga[3];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) ga[i] = inv[3 * i] * a0 + inv[3 * i + 1] * a1 + inv[3 * i + 2] * a2;
+#pragma unroll
+          for (int b = 0; b < 8; ++b) {
+            const T bx = ((b & 1) == ix) ? hp : hm, by = (((b >> 1) & 1) == iy) ? hp : hm,
+                    bz = ((b >> 2) == iz) ? hp : hm;
+            const T b0 = flip_if(pyz[b >> 1], !(b & 1)), b1 = flip_if(T(0.5) * (bx * bz), !(b & 2)),
+                    b2 = flip_if(T(0.5) * (bx * by), !(b & 4));
+            T gb[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) gb[i] = inv[3 * i] * b0 + inv[3 * i + 1] * b1 + inv[3 * i + 2] * b2;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+              for (int jj = 0; jj < 3; ++jj) G[b][3 * i + jj] += ga[i] * gb[jj];
+          }
+        }
+      }
+      if (iz == 0) {  // the next element's coordinates
+        if (more) load_x(n0, n1, r + 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      }
+    }
+    k += kIsoWarps;
+    el = el_next;
+    el_next = k + kIsoWarps < ke ? nelem[k + kIsoWarps] : 0;
+    T lam = T(0), mu = T(0);
+    int4 s0 = make_int4(0, 0, 0, 0), s1 = s0;
+    if (on) {
+      const int4* sl = reinterpret_cast<const int4*>(slot + e * 64 + a * 8);
+      s0 = sl[0];
+      s1 = sl[1];
+      lam = (T)lame[2 * e];
+      mu = (T)lame[2 * e + 1];
+    }
+    // the turn of this warp: after warp w - 1 in this round (warp 3 of the round before)
+    if (r > 0 || w > 0) bar_sync(1 + w, 64);
+    if (on) {
+      const int32_t ps[8] = {s0.x, s0.y, s0.w, s0.z, s1.x, s1.y, s1.w, s1.z};
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        T* d = acc + lane * stride + 9 * (int)((ps[b] - base) >> 5);
+        const T tr = mu * (G[b][0] + G[b][4] + G[b][8]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int jj = 0; jj < 3; ++jj) {
+            T v = lam * G[b][3 * i + jj] + mu * G[b][3 * jj + i];
+            if (i == jj) v += tr;
+            d[3 * i + jj] += v;
+          }
+      }
+    }
+    if (r + 1 < rounds || w + 1 < kIsoWarps) {
+      __threadfence_block();
+      bar_arrive(1 + (w + 1) % kIsoWarps, 64);
+    }
+  }
+  if (bad) atomicOr(err, (int)kDevBadJacobian);
+  __syncthreads();
+  out.write(len, scol, fixed, acc, stride, val, dinv, val_r, dinv_r);
+}
+
+// Lame constants of every element, [E][2].
+__global__ void k_lame(int32_t E, const double* __restrict__ props, int nprops, double* __restrict__ out) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= E) return;
+  double lam, mu;
+  lame<double>(props[e * nprops], props[e * nprops + 1], lam, mu);
+  out[2 * e] = lam;
+  out[2 * e + 1] = mu;
 }
 
 // Difference form: the diagonal slot of each block row holds the FP64 block
@@ -170,34 +544,6 @@ __global__ void k_diag_rowsum(int32_t N, const int64_t* __restrict__ sptr, const
   const int64_t d = dpos[i];
 #pragma unroll
   for (int c = 0; c < 9; ++c) v32[vpos(d, c)] = (float)S[c];
-}
-
-// Jacobi diagonal in FP32 from the FP64 diagonal.
-__global__ void k_dinv_from64(int32_t N, const int32_t* __restrict__ dpos, const double* __restrict__ val,
-                              float* __restrict__ dinv) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 3 * (int64_t)N) return;
-  const double d = val[vpos(dpos[i / 3], (int)(i % 3) * 4)];
-  dinv[i] = fabs(d) > 1e-30 ? (float)(1.0 / d) : 1.0f;
-}
-
-template <typename T>
-__global__ void k_fix_diag(int32_t nfix, const int32_t* __restrict__ dofs, const int32_t* __restrict__ dpos,
-                           T* __restrict__ val) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nfix) return;
-  const int32_t d = dofs[i];
-  val[vpos(dpos[d / 3], (d % 3) * 4)] = T(1);
-}
-
-// Jacobi diag_inv = 1/K_ii, or 1 when |K_ii| <= 1e-30 (NM_LinSolv_Prec_Jacobi_Build,
-// ufc_core/L2_NM/Solver/LinSolv/NM_Solv_LinPrec.f90:328-353; NM_Solver_PCG uses 1e-30).
-template <typename T>
-__global__ void k_dinv(int32_t N, const int32_t* __restrict__ dpos, const T* __restrict__ val, T* __restrict__ dinv) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 3 * (int64_t)N) return;
-  const T d = val[vpos(dpos[i / 3], (int)(i % 3) * 4)];
-  dinv[i] = fabs((double)d) > 1e-30 ? T(1) / d : T(1);
 }
 
 // Matrix-free FP64 operator, one thread per element of one colour:
@@ -276,12 +622,15 @@ __global__ void __launch_bounds__(128)
     double inv[9], eps[6], s[6];
     const double det = jacobian_inv<double>(X, ip, inv);
     strain_at<double>(inv, ip, xe, eps);
-    const double* D = Dt + (e * 8 + ip) * 36;
+    const double* D = Dt + e * 168 + ip;  // [21][8 Gauss points]
+    double d[21];
+#pragma unroll
+    for (int k = 0; k < 21; ++k) d[k] = D[8 * k];
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
       double t = 0.0;
 #pragma unroll
-      for (int j = 0; j < 6; ++j) t += D[i * 6 + j] * eps[j];
+      for (int j = 0; j < 6; ++j) t += d[tri6(i, j)] * eps[j];
       s[i] = t;
     }
     add_bt_sigma<double>(inv, ip, det, s, fe);
@@ -328,7 +677,9 @@ __global__ void __launch_bounds__(128)
   }
   epeq_t[g] = epeq;
 #pragma unroll
-  for (int k = 0; k < 36; ++k) Dt[g * 36 + k] = D[k];
+  for (int i = 0; i < 6; ++i)
+#pragma unroll
+    for (int j = i; j < 6; ++j) Dt[e * 168 + 8 * tri6(i, j) + ip] = D[i * 6 + j];
   if (!finite) atomicOr(err, (int)kDevNonFinite);
 }
 
@@ -494,18 +845,38 @@ __global__ void k_set_fixed(int32_t nfix, const int32_t* __restrict__ dofs, cons
   if (i < nfix) y[dofs[i]] = vals ? vals[i] : 0.0;
 }
 
-bool g_pairs_ready = false;
+}  // namespace
 
-int ensure_pairs(Ctx* c) {
-  if (g_pairs_ready) return UFC_STATUS_OK;
-  PairTable t;
-  UFC_CUDA(c, cudaMemcpyToSymbol(c_pair_a, t.a, sizeof(t.a)));
-  UFC_CUDA(c, cudaMemcpyToSymbol(c_pair_b, t.b, sizeof(t.b)));
-  g_pairs_ready = true;
+int element_lame(Ctx* c) {
+  UFC_TRY(dalloc(c, &c->lame, 2 * (int64_t)c->E));
+  k_lame<<<grid_for(c->E, 256), 256, 0, c->stream>>>(c->E, c->props, c->nprops, c->lame);
+  UFC_CUDA(c, cudaGetLastError());
   return UFC_STATUS_OK;
 }
 
-}  // namespace
+template <typename T, bool kTangent>
+static int launch_assemble(Ctx* c, T* val, T* dinv, float* val_r, float* dinv_r) {
+  const int stride = (9 * c->max_row_blocks) | 1;  // odd: the rows of an entry lie in different banks
+  if constexpr (!kTangent) {
+    // while the slice's accumulators fit in shared memory
+    const int bytes = kIsoXBytes + (int)sizeof(T) * kSlice * stride;
+    if (bytes <= kAsmMaxSmem) {
+      UFC_CUDA(c, cudaFuncSetAttribute(k_assemble_iso<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+      k_assemble_iso<T><<<(int)c->nslices, kIsoThreads, bytes, c->stream>>>(
+          c->N, c->nptr, c->nelem, c->coords, c->conn, c->lame, c->slot, c->slice_ptr, c->sell_col, c->dpos, c->fixed,
+          stride, val, dinv, val_r, dinv_r, c->dev_err);
+      UFC_CUDA(c, cudaGetLastError());
+      return UFC_STATUS_OK;
+    }
+  }
+  const int bytes = (int)(sizeof(AsmWarp<T, kTangent>) * kAsmWarps + sizeof(T) * kAsmRows * stride);
+  UFC_CUDA(c, cudaFuncSetAttribute(k_assemble_rows<T, kTangent>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  k_assemble_rows<T, kTangent><<<(int)(2 * c->nslices), kAsmWarps * 32, bytes, c->stream>>>(
+      c->N, c->nptr, c->nelem, c->coords, c->conn, c->lame, c->Dt, c->slot, c->slice_ptr, c->sell_col, c->dpos,
+      c->fixed, stride, val, dinv, val_r, dinv_r, c->dev_err);
+  UFC_CUDA(c, cudaGetLastError());
+  return UFC_STATUS_OK;
+}
 
 int assemble(Ctx* c, int build, double* elapsed_ms) {
   if (!c->has_pattern) return fail(c, UFC_STATUS_INVALID, "ufc_elem_compute_ke: pattern not built");
@@ -514,7 +885,6 @@ int assemble(Ctx* c, int build, double* elapsed_ms) {
   if (tangent && !c->has_trial)
     return fail(c, UFC_STATUS_INVALID,
                 "ufc_elem_compute_ke: J2 tangent needs ufc_elem_compute_fint(update_state=1) first");
-  UFC_TRY(ensure_pairs(c));
   mg_mark_stale(c);  // (cached CG graphs stay: they are keyed by the arrays and the SpMV form they read)
   cudaEvent_t e0, e1;
   UFC_CUDA(c, cudaEventCreate(&e0));
@@ -530,65 +900,33 @@ int assemble(Ctx* c, int build, double* elapsed_ms) {
   if (sym) build |= UFC_BUILD_FP64;
   c->has_sval64 = c->has_sval32 = false;  // values change: symmetric copies are stale
   if (build & UFC_BUILD_FP32) c->val32_diff = false;
-  for (int prec = 0; prec < 2; ++prec) {
-    const bool want = prec == 0 ? (build & UFC_BUILD_FP64) : (build & UFC_BUILD_FP32);
-    if (!want) continue;
-    if (prec == 0) {
-      if (!c->val64) UFC_TRY(dalloc(c, &c->val64, nv));
-      if (!c->dinv64) UFC_TRY(dalloc(c, &c->dinv64, c->n));
-      UFC_CUDA(c, cudaMemsetAsync(c->val64, 0, sizeof(double) * nv, c->stream));
-    } else {
-      if (!c->val32) UFC_TRY(dalloc(c, &c->val32, nv));
-      if (!c->dinv32) UFC_TRY(dalloc(c, &c->dinv32, c->n));
-      UFC_CUDA(c, cudaMemsetAsync(c->val32, 0, sizeof(float) * nv, c->stream));
-    }
-    for (int col = 0; col < c->ncol; ++col) {
-      const int32_t ne = c->col_off[col + 1] - c->col_off[col];
-      if (ne == 0) continue;
-      const int32_t* el = c->col_elems + c->col_off[col];
-      const int grid = (int)((ne + kWarpsPerCta - 1) / kWarpsPerCta);
-      if (prec == 0) {
-        if (tangent)
-          k_assemble<double, true><<<grid, kWarpsPerCta * 32, 0, c->stream>>>(
-              el, ne, c->coords, c->conn, c->props, c->nprops, c->Dt, c->slot, c->fixed, c->val64, c->dev_err);
-        else
-          k_assemble<double, false><<<grid, kWarpsPerCta * 32, 0, c->stream>>>(
-              el, ne, c->coords, c->conn, c->props, c->nprops, nullptr, c->slot, c->fixed, c->val64, c->dev_err);
-      } else {
-        if (tangent)
-          k_assemble<float, true><<<grid, kWarpsPerCta * 32, 0, c->stream>>>(
-              el, ne, c->coords, c->conn, c->props, c->nprops, c->Dt, c->slot, c->fixed, c->val32, c->dev_err);
-        else
-          k_assemble<float, false><<<grid, kWarpsPerCta * 32, 0, c->stream>>>(
-              el, ne, c->coords, c->conn, c->props, c->nprops, nullptr, c->slot, c->fixed, c->val32, c->dev_err);
-      }
-      UFC_CUDA(c, cudaGetLastError());
-    }
-    if (c->nfix > 0) {
-      if (prec == 0)
-        k_fix_diag<double><<<grid_for(c->nfix, 256), 256, 0, c->stream>>>(c->nfix, c->fix_dofs, c->dpos, c->val64);
-      else
-        k_fix_diag<float><<<grid_for(c->nfix, 256), 256, 0, c->stream>>>(c->nfix, c->fix_dofs, c->dpos, c->val32);
-      UFC_CUDA(c, cudaGetLastError());
-    }
-    if (prec == 0) {
-      k_dinv<double><<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->N, c->dpos, c->val64, c->dinv64);
-      c->has_val64 = true;
-    } else {
-      k_dinv<float><<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->N, c->dpos, c->val32, c->dinv32);
-      c->has_val32 = true;
-    }
-    UFC_CUDA(c, cudaGetLastError());
+  if (build & UFC_BUILD_FP64) {
+    if (!c->val64) UFC_TRY(dalloc(c, &c->val64, nv));
+    if (!c->dinv64) UFC_TRY(dalloc(c, &c->dinv64, c->n));
   }
-  if (rounded) {
-    // FP32 values = FP64 values rounded to nearest (Dirichlet rows included)
+  if (rounded || (build & UFC_BUILD_FP32)) {
     if (!c->val32) UFC_TRY(dalloc(c, &c->val32, nv));
     if (!c->dinv32) UFC_TRY(dalloc(c, &c->dinv32, c->n));
-    k_round_values<<<(int)std::min<int64_t>(grid_for(nv, 256), 148 * 16), 256, 0, c->stream>>>(nv, c->val64,
-                                                                                               c->val32);
+  }
+  if (build & UFC_BUILD_FP64) {
+    // with `rounded` the FP32 values are the FP64 values rounded to nearest (Dirichlet rows included)
+    float *vr = rounded ? c->val32 : nullptr, *dr = rounded ? c->dinv32 : nullptr;
+    if (tangent)
+      UFC_TRY((launch_assemble<double, true>(c, c->val64, c->dinv64, vr, dr)));
+    else
+      UFC_TRY((launch_assemble<double, false>(c, c->val64, c->dinv64, vr, dr)));
+    c->has_val64 = true;
+  }
+  if (build & UFC_BUILD_FP32) {
+    if (tangent)
+      UFC_TRY((launch_assemble<float, true>(c, c->val32, c->dinv32, nullptr, nullptr)));
+    else
+      UFC_TRY((launch_assemble<float, false>(c, c->val32, c->dinv32, nullptr, nullptr)));
+    c->has_val32 = true;
+  }
+  if (rounded) {
     if (diff)
       k_diag_rowsum<<<grid_for(c->N, 128), 128, 0, c->stream>>>(c->N, c->slice_ptr, c->dpos, c->val64, c->val32);
-    k_dinv_from64<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->N, c->dpos, c->val64, c->dinv32);
     UFC_CUDA(c, cudaGetLastError());
     c->has_val32 = true;
     c->val32_diff = diff;

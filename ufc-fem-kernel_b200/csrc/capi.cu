@@ -132,7 +132,8 @@ void free_all(Ctx* c) {
   release_graphs(c);
   mg_free(c);
   dfree(&c->z64);
-  dfree(&c->coords); dfree(&c->conn); dfree(&c->props); dfree(&c->col_elems);
+  dfree(&c->coords); dfree(&c->conn); dfree(&c->props); dfree(&c->lame); dfree(&c->col_elems);
+  dfree(&c->nptr); dfree(&c->nelem);
   dfree(&c->brow); dfree(&c->bcol); dfree(&c->slice_ptr); dfree(&c->sell_col); dfree(&c->slot); dfree(&c->dpos);
   dfree(&c->val64); dfree(&c->val32); dfree(&c->dinv64); dfree(&c->dinv32);
   dfree(&c->uptr); dfree(&c->ucol); dfree(&c->lptr); dfree(&c->lpos); dfree(&c->lcol); dfree(&c->s_lcnt);
@@ -157,7 +158,7 @@ int alloc_state(Ctx* c) {
   if (c->mat_model == UFC_MAT_J2_ISO) {
     UFC_TRY(dalloc(c, &c->sig_n, G * 6)); UFC_TRY(dalloc(c, &c->epeq_n, G)); UFC_TRY(dalloc(c, &c->epl_n, G * 6));
     UFC_TRY(dalloc(c, &c->sig_t, G * 6)); UFC_TRY(dalloc(c, &c->epeq_t, G)); UFC_TRY(dalloc(c, &c->epl_t, G * 6));
-    UFC_TRY(dalloc(c, &c->Dt, G * 36));
+    UFC_TRY(dalloc(c, &c->Dt, G * 21));
     UFC_CUDA(c, cudaMemsetAsync(c->sig_n, 0, sizeof(double) * G * 6, c->stream));
     UFC_CUDA(c, cudaMemsetAsync(c->epeq_n, 0, sizeof(double) * G, c->stream));
     UFC_CUDA(c, cudaMemsetAsync(c->epl_n, 0, sizeof(double) * G * 6, c->stream));
@@ -369,6 +370,7 @@ int ufc_material_set(ufc_ctx* c, const ufc_material_desc* m) {
   c->nprops = m->nprops;
   UFC_TRY(dalloc(c, &c->props, (int64_t)full.size()));
   UFC_CUDA(c, cudaMemcpyAsync(c->props, full.data(), sizeof(double) * full.size(), cudaMemcpyHostToDevice, c->stream));
+  UFC_TRY(element_lame(c));
   UFC_TRY(alloc_state(c));
   c->has_material = true;
   c->has_val64 = c->has_val32 = c->has_sval64 = c->has_sval32 = false;  // values depend on the material

@@ -127,7 +127,10 @@ __global__ void __launch_bounds__(64)
     } else {
       if (t < 24) X[t] = coords[(int64_t)conn_f[ef * 8 + t / 3] * 3 + t % 3];
       if (TANGENT)
-        for (int q = t; q < 288; q += 64) (&D[0][0])[q] = Dt[ef * 288 + q];
+        for (int q = t; q < 288; q += 64) {
+          const int gp = q / 36, i = (q % 36) / 6, j = q % 6, lo = min(i, j), hi = max(i, j);
+          D[TANGENT ? gp : 0][q % 36] = Dt[ef * 168 + 8 * (lo * 6 - lo * (lo - 1) / 2 + hi - lo) + gp];
+        }
       __syncthreads();
       if (t < 8) {
         double inv[9];

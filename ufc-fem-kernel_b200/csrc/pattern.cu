@@ -66,6 +66,19 @@ __global__ void k_sort_node_elems(int32_t N, const int32_t* __restrict__ nptr, i
   }
 }
 
+// Node -> element lists with the element's local node packed in: 8 e + a.
+__global__ void k_pack_node_elems(int32_t N, const int32_t* __restrict__ conn, const int32_t* __restrict__ nptr,
+                                  const int32_t* __restrict__ nlst, int32_t* __restrict__ nelem) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  for (int32_t k = nptr[i]; k < nptr[i + 1]; ++k) {
+    const int64_t e = nlst[k];
+    int a = 0;
+    while (a < 7 && conn[e * 8 + a] != i) ++a;
+    nelem[k] = (int32_t)(e * 8 + a);
+  }
+}
+
 // Element colouring on the device.  The sequential greedy colouring (elements
 // in ascending order, each taking the smallest colour that none of its lower
 // neighbours -- elements f < e sharing a node with e -- has) is the unique
@@ -722,31 +735,40 @@ int build_pattern(Ctx* c) {
   const int32_t N = c->N, E = c->E;
 
   // 1. node -> element adjacency on the device
-  int32_t *cnt = nullptr, *nptr = nullptr, *fill = nullptr, *nlst = nullptr;
+  int32_t *cnt = nullptr, *fill = nullptr, *nlst = nullptr;
   UFC_TRY(dalloc(c, &cnt, (int64_t)N + 1));
-  UFC_TRY(dalloc(c, &nptr, (int64_t)N + 1));
+  UFC_TRY(dalloc(c, &c->nptr, (int64_t)N + 1));  // kept, with the packed lists: the assembly runs by rows
+  const int32_t* nptr = c->nptr;
   UFC_TRY(dalloc(c, &fill, N));
   UFC_TRY(dalloc(c, &nlst, 8 * (int64_t)E));
   UFC_CUDA(c, cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)N + 1), c->stream));
   UFC_CUDA(c, cudaMemsetAsync(fill, 0, sizeof(int32_t) * N, c->stream));
   UFC_CUDA(c, cudaMemsetAsync(c->dev_err, 0, sizeof(int32_t), c->stream));
   k_count_node_elems<<<grid_for(8 * (int64_t)E, 256), 256, 0, c->stream>>>(E, c->conn, cnt);
-  UFC_TRY(scan_exclusive(c, cnt, nptr, (int64_t)N + 1));
+  UFC_TRY(scan_exclusive(c, cnt, c->nptr, (int64_t)N + 1));
   k_fill_node_elems<<<grid_for(8 * (int64_t)E, 256), 256, 0, c->stream>>>(E, c->conn, nptr, fill, nlst);
   k_sort_node_elems<<<grid_for(N, 128), 128, 0, c->stream>>>(N, nptr, nlst, c->dev_err);
   UFC_CUDA(c, cudaGetLastError());
   int st = check_dev_err(c, "ufc_pattern_build (node adjacency)");
   if (st != UFC_STATUS_OK) {
-    dfree(&cnt); dfree(&nptr); dfree(&fill); dfree(&nlst);
+    dfree(&cnt); dfree(&fill); dfree(&nlst);
     return st;
   }
+
+  st = dalloc(c, &c->nelem, 8 * (int64_t)E);
+  if (st != UFC_STATUS_OK) {
+    dfree(&cnt); dfree(&fill); dfree(&nlst);
+    return st;
+  }
+  k_pack_node_elems<<<grid_for(N, 256), 256, 0, c->stream>>>(N, c->conn, nptr, nlst, c->nelem);
+  UFC_CUDA(c, cudaGetLastError());
 
   // 2. colouring (device sweeps) and colour-grouped element lists
   {
     std::vector<int32_t> color;
     st = color_elements_device(c, nptr, nlst, color);
     if (st != UFC_STATUS_OK) {
-      dfree(&cnt); dfree(&nptr); dfree(&fill); dfree(&nlst);
+      dfree(&cnt); dfree(&fill); dfree(&nlst);
       return st;
     }
     c->col_off.assign(c->ncol + 1, 0);
@@ -763,7 +785,7 @@ int build_pattern(Ctx* c) {
       if (ce != cudaSuccess) st = cuda_fail(c, ce, "ufc_pattern_build (colour lists)");
     }
     if (st != UFC_STATUS_OK) {
-      dfree(&cnt); dfree(&nptr); dfree(&fill); dfree(&nlst);
+      dfree(&cnt); dfree(&fill); dfree(&nlst);
       return st;
     }
   }
@@ -775,7 +797,7 @@ int build_pattern(Ctx* c) {
   UFC_TRY(scan_exclusive(c, cnt, c->brow, (int64_t)N + 1));
   st = check_dev_err(c, "ufc_pattern_build (row count)");
   if (st != UFC_STATUS_OK) {
-    dfree(&cnt); dfree(&nptr); dfree(&fill); dfree(&nlst);
+    dfree(&cnt); dfree(&fill); dfree(&nlst);
     return st;
   }
   int32_t nnzb = 0;
@@ -817,7 +839,7 @@ int build_pattern(Ctx* c) {
                                                                 c->dev_err);
   UFC_CUDA(c, cudaGetLastError());
   st = check_dev_err(c, "ufc_pattern_build (slots)");
-  dfree(&cnt); dfree(&nptr); dfree(&fill); dfree(&nlst);
+  dfree(&cnt); dfree(&fill); dfree(&nlst);
   if (st != UFC_STATUS_OK) return st;
 
   // grid reductions keep 4 partial sums per block; the SpMV grid has one

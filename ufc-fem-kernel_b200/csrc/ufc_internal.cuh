@@ -116,6 +116,7 @@ struct Ctx {
   // material
   int32_t mat_model = 0, nprops = 0;
   double* props = nullptr;  // [E*nprops]
+  double* lame = nullptr;   // [E*2] Lame constants
   bool has_material = false;
 
   // colouring
@@ -128,6 +129,8 @@ struct Ctx {
   bool has_pattern = false;
   int64_t nnzb = 0;
   int32_t max_row_blocks = 0;
+  int32_t* nptr = nullptr;    // [N+1] node -> element lists: 8 e + local node, ascending
+  int32_t* nelem = nullptr;   // [E*8]
   int32_t* brow = nullptr;    // [N+1]
   int32_t* bcol = nullptr;    // [nnzb]
   int64_t nslices = 0, sell_blocks = 0;
@@ -198,7 +201,7 @@ struct Ctx {
   double* u_n = nullptr;    // [n] committed
   double *sig_n = nullptr, *epeq_n = nullptr, *epl_n = nullptr;  // committed [G*6],[G],[G*6]
   double *sig_t = nullptr, *epeq_t = nullptr, *epl_t = nullptr;  // trial
-  double* Dt = nullptr;     // [G*36] consistent tangent of the trial state
+  double* Dt = nullptr;     // [E][21][8 Gauss points] consistent tangent of the trial state, upper triangle
   bool has_trial = false;
 
   // multigrid preconditioner (ufc_mg_setup), and the preconditioned vector z
@@ -230,6 +233,7 @@ int pack_symmetric(Ctx* c, bool fp64, bool fp32);  // full SELL values -> symmet
 int export_csr(Ctx* c, const ufc_csr_export_arg* a);
 
 // c3d8.cu
+int element_lame(Ctx* c);  // Lame constants of the current material into c->lame
 int assemble(Ctx* c, int build, double* elapsed_ms);
 int apply_fp64(Ctx* c, const double* x, double* y, bool masked);  // y = K x matrix-free, FP64
 int apply_fp64_eliminated(Ctx* c, const double* x, double* y);    // eliminated operator incl. identity rows
