@@ -41,9 +41,9 @@ namespace {
 // about 320 when D is applied at every Gauss point); the J2 block as
 // sum_gp (D B_a)^T B_b with D B_a formed once per (row, element, Gauss point).
 //
-// What bounds it: FP64 issue and the shared-memory pipe, about equally (per row
-// and element 250 FP64 operations a lane and some 150 shared-memory wavefronts a
-// warp).  Recomputing an element's Jacobians for each of its 8 rows costs less
+// What bounds it: the shared-memory pipe (97 % busy, 400 wavefronts per element
+// of 4 rows; FP64 35 %).  It serves the J2 tangents, and linear-elastic rows too
+// long for the shared memory of the one-thread form below.  Recomputing an element's Jacobians for each of its 8 rows costs less
 // than the read-modify-write of the values that an element-wise scatter needs
 // (16.6 GB at 192x96x96, in 8 colour passes).
 constexpr int kAsmRows = 16;                // rows per CTA
@@ -329,7 +329,10 @@ __global__ void __launch_bounds__(kAsmWarps * 32)
 // warps add their blocks in turn (named barriers pass the turn on), so each
 // entry still receives its contributions in ascending element order.  The
 // coordinates of a thread's next element come by cp.async while the current one
-// is worked on.
+// is worked on.  128x64x64, FP64 with FP32 copies: 1.32 ms; 8 lanes per row and
+// element as above 1.57 ms (shared-memory pipe 97 % busy); the colour-ordered
+// element scatter before 5.03 ms.  Here FP64 is 40 % busy, the rest is latency
+// (8 warps per SM; the accumulators take the registers).
 constexpr int kIsoWarps = 4;
 constexpr int kIsoThreads = kIsoWarps * 32;
 constexpr int kIsoXBytes = kIsoWarps * 2 * 24 * 32 * (int)sizeof(double);  // [warp][stage][coordinate][lane]

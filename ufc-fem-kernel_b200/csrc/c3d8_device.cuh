@@ -208,4 +208,13 @@ __host__ __device__ __forceinline__ int64_t vpos(int64_t P, int c) {
   return 9 * (P & ~int64_t(31)) + 32 * c + (P & 31);
 }
 
+// The same for the symmetric storage, whose steps are laid out for 16-byte
+// loads: components 0-7 in groups of 16 / sizeof(T) per lane, then component 8.
+template <typename T>
+__host__ __device__ __forceinline__ int64_t spos(int64_t P, int c) {
+  constexpr int V = 16 / (int)sizeof(T);
+  const int64_t b = 9 * (P & ~int64_t(31)), t = P & 31;
+  return c == 8 ? b + 256 + t : b + 32 * V * (c / V) + V * t + c % V;
+}
+
 }  // namespace ufc

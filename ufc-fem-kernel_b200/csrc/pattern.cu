@@ -464,7 +464,7 @@ __global__ void k_sym_pack(int32_t N, const int64_t* __restrict__ sptr, const in
     const int64_t src = sptr[s] + (int64_t)(nl + j) * kSlice + t;
     const int64_t dst = uptr[s] + (int64_t)j * kSlice + t;
 #pragma unroll
-    for (int c = 0; c < 9; ++c) out[vpos(dst, c)] = (TO)v64[vpos(src, c)];
+    for (int c = 0; c < 9; ++c) out[spos<TO>(dst, c)] = (TO)v64[vpos(src, c)];
   }
 }
 

@@ -3,10 +3,15 @@
 // ufc_core/L2_NM/Solver/LinSolv/NM_Solv_IterSolver.f90:713-846).
 //
 // One CG iteration is three kernels:
-//   k_spmv<.., kCg>   q = K p, fused p.q, alpha = r.z / p.q
-//   k_cg_update       x += alpha p (x in FP64), r -= alpha q, z = D^-1 r fused,
-//                     r.z and r.r, beta, the stop test and the refinement trigger
-//   k_cg_pupdate      p = D^-1 r + beta p
+//   k_spmv<.., kCg>   q = K p, per-block partials of p.q
+//   k_cg_update       alpha = r.z / p.q, x += alpha p (x in FP64), r -= alpha q,
+//                     z = D^-1 r fused, per-block partials of r.z and r.r
+//   k_cg_pupdate      beta, the stop test and the refinement trigger, p = D^-1 r + beta p
+// A reduction ends in the kernel that follows it: every block there sums the
+// partials again, in the same order (k_cg_sum first when there are thousands).
+// No block waits for a fence or an election: with that wait at the end of each
+// of the product's 7094 blocks the FP32 product of 192x96x96 took 230 us in the
+// iteration against 186 us on its own.
 // The scalars live in device memory (CgScalars) and every kernel returns at
 // once when the run has stopped, so batches of iterations are launched as one
 // CUDA graph and the host only looks at the scalars between batches.
@@ -63,12 +68,14 @@ void launch_pdl(void (*kernel)(K...), int grid, int block, cudaStream_t st, A&&.
 }
 
 // The CG variants of the products (MODE kCg) run inside the iteration chain.
+// Returns the grid: the number of partial sums a kCg product leaves.
 template <int MODE, typename... K, typename... A>
-void launch_mode(void (*kernel)(K...), int grid, int block, cudaStream_t st, A&&... args) {
+int launch_mode(void (*kernel)(K...), int grid, int block, cudaStream_t st, A&&... args) {
   if constexpr (MODE == 1)
     launch_pdl(kernel, grid, block, st, std::forward<A>(args)...);
   else
     kernel<<<grid, block, 0, st>>>(std::forward<A>(args)...);
+  return grid;
 }
 
 // Grid of the CG vector kernels: they take 4 entries per thread (16-byte
@@ -98,7 +105,7 @@ __device__ __forceinline__ bool halted(const CgScalars* s) { return (s->stop | s
 template <typename TV, typename TX, typename TA, int MODE, bool DIFF>
 __global__ void __launch_bounds__(kSpmvBlock)
     k_spmv(int32_t N, int64_t nrows_pad, const int64_t* __restrict__ sptr, const int32_t* __restrict__ col,
-           const TV* __restrict__ val, const TX* __restrict__ x, TX* __restrict__ y, CgScalars* __restrict__ scal,
+           const TV* __restrict__ val, const TX* __restrict__ x, TX* __restrict__ y, const CgScalars* __restrict__ scal,
            double* __restrict__ partials) {
   pdl_enter();
   if (MODE == kCg && halted(scal)) return;
@@ -140,17 +147,7 @@ __global__ void __launch_bounds__(kSpmvBlock)
         dot[0] = (double)((TA)x[3 * row] * a0 + (TA)x[3 * row + 1] * a1 + (TA)x[3 * row + 2] * a2);
     }
   }
-  if (MODE == kCg) {
-    double tot[1];
-    if (grid_sum<1>(dot, partials, &scal->ticket[0], tot)) {
-      scal->pq = tot[0];
-      if (!(fabs(tot[0]) > 1e-300) || !isfinite(tot[0])) {
-        scal->stop = 3;
-      } else {
-        scal->alpha = scal->rz / tot[0];
-      }
-    }
-  }
+  if (MODE == kCg) block_partial<1>(dot, partials);
 }
 
 // The same product with SPLIT (2, 4 or 8) warps per slice, for meshes with few
@@ -162,7 +159,7 @@ __global__ void __launch_bounds__(kSpmvBlock)
 template <typename TV, typename TX, typename TA, int MODE, bool DIFF, int SPLIT>
 __global__ void __launch_bounds__(kSpmvBlock)
     k_spmv_split(int32_t N, int64_t nslices, const int64_t* __restrict__ sptr, const int32_t* __restrict__ col,
-           const TV* __restrict__ val, const TX* __restrict__ x, TX* __restrict__ y, CgScalars* __restrict__ scal,
+           const TV* __restrict__ val, const TX* __restrict__ x, TX* __restrict__ y, const CgScalars* __restrict__ scal,
            double* __restrict__ partials) {
   pdl_enter();
   if (MODE == kCg && halted(scal)) return;
@@ -221,17 +218,7 @@ __global__ void __launch_bounds__(kSpmvBlock)
     y[3 * row + 2] = (TX)a2;
     if (MODE == kCg) dot[0] = (double)((TA)x[3 * row] * a0 + (TA)x[3 * row + 1] * a1 + (TA)x[3 * row + 2] * a2);
   }
-  if (MODE == kCg) {
-    double tot[1];
-    if (grid_sum<1>(dot, partials, &scal->ticket[0], tot)) {
-      scal->pq = tot[0];
-      if (!(fabs(tot[0]) > 1e-300) || !isfinite(tot[0])) {
-        scal->stop = 3;
-      } else {
-        scal->alpha = scal->rz / tot[0];
-      }
-    }
-  }
+  if (MODE == kCg) block_partial<1>(dot, partials);
 }
 
 // y = K x on the full SELL storage with coded indices (see build_full_codes):
@@ -303,17 +290,7 @@ __global__ void __launch_bounds__(kSpmvBlock)
     y[3 * row + 2] = (TX)a2;
     if (MODE == kCg) dot[0] = (double)((TA)x[3 * row] * a0 + (TA)x[3 * row + 1] * a1 + (TA)x[3 * row + 2] * a2);
   }
-  if (MODE == kCg) {
-    double tot[1];
-    if (grid_sum<1>(dot, partials, &scal->ticket[0], tot)) {
-      scal->pq = tot[0];
-      if (!(fabs(tot[0]) > 1e-300) || !isfinite(tot[0])) {
-        scal->stop = 3;
-      } else {
-        scal->alpha = scal->rz / tot[0];
-      }
-    }
-  }
+  if (MODE == kCg) block_partial<1>(dot, partials);
 }
 
 int sm_count_solver() {
@@ -336,7 +313,7 @@ int spmv_split(const Ctx* c) {
 }
 
 template <typename TV, typename TX, typename TA, int MODE, bool DIFF, int SPLIT>
-void launch_spmv_split(const Ctx* c, cudaStream_t st, const TV* val, const TX* x, TX* y) {
+int launch_spmv_split(const Ctx* c, cudaStream_t st, const TV* val, const TX* x, TX* y) {
   // coded indices with FP32 values and one warp per slice only (measured on
   // B200: 192x96x96 FP32 product 297 against 325 us, FP64 582 against 568 us;
   // with SPLIT warps per slice each warp loads the row's 32 code bytes, more
@@ -345,43 +322,40 @@ void launch_spmv_split(const Ctx* c, cudaStream_t st, const TV* val, const TX* x
   if (!DIFF && SPLIT == 1 && sizeof(TV) == 4 && c->full_coded) {
     constexpr int per_block = kSpmvBlock / 32 / SPLIT;
     const int grid = (int)((c->nslices + per_block - 1) / per_block);
-    launch_mode<MODE>(k_spmvc<TV, TX, TA, MODE, SPLIT>, grid, kSpmvBlock, st, c->N, c->nslices, c->slice_ptr,
-                      reinterpret_cast<const uint4*>(c->full_code), c->full_tab, val, x, y, c->scal, c->partials);
-    return;
+    return launch_mode<MODE>(k_spmvc<TV, TX, TA, MODE, SPLIT>, grid, kSpmvBlock, st, c->N, c->nslices, c->slice_ptr,
+                             reinterpret_cast<const uint4*>(c->full_code), c->full_tab, val, x, y, c->scal,
+                             c->partials);
   }
   if constexpr (SPLIT == 1) {
     const int grid = (int)((c->nslices * kSlice + kSpmvBlock - 1) / kSpmvBlock);
-    launch_mode<MODE>(k_spmv<TV, TX, TA, MODE, DIFF>, grid, kSpmvBlock, st, c->N, c->nslices * kSlice,
-                      c->slice_ptr, c->sell_col, val, x, y, c->scal, c->partials);
+    return launch_mode<MODE>(k_spmv<TV, TX, TA, MODE, DIFF>, grid, kSpmvBlock, st, c->N, c->nslices * kSlice,
+                             c->slice_ptr, c->sell_col, val, x, y, c->scal, c->partials);
   } else {
     constexpr int per_block = kSpmvBlock / 32 / SPLIT;
     const int grid = (int)((c->nslices + per_block - 1) / per_block);
-    launch_mode<MODE>(k_spmv_split<TV, TX, TA, MODE, DIFF, SPLIT>, grid, kSpmvBlock, st, c->N, c->nslices,
-                      c->slice_ptr, c->sell_col, val, x, y, c->scal, c->partials);
+    return launch_mode<MODE>(k_spmv_split<TV, TX, TA, MODE, DIFF, SPLIT>, grid, kSpmvBlock, st, c->N, c->nslices,
+                             c->slice_ptr, c->sell_col, val, x, y, c->scal, c->partials);
   }
 }
 
 template <typename TV, typename TX, typename TA, int MODE, bool DIFF>
-void launch_spmv_diff(const Ctx* c, cudaStream_t st, const TV* val, const TX* x, TX* y) {
+int launch_spmv_diff(const Ctx* c, cudaStream_t st, const TV* val, const TX* x, TX* y) {
   switch (spmv_split(c)) {
-    case 1: launch_spmv_split<TV, TX, TA, MODE, DIFF, 1>(c, st, val, x, y); break;
-    case 2: launch_spmv_split<TV, TX, TA, MODE, DIFF, 2>(c, st, val, x, y); break;
-    case 4: launch_spmv_split<TV, TX, TA, MODE, DIFF, 4>(c, st, val, x, y); break;
-    default: launch_spmv_split<TV, TX, TA, MODE, DIFF, 8>(c, st, val, x, y); break;
+    case 1: return launch_spmv_split<TV, TX, TA, MODE, DIFF, 1>(c, st, val, x, y);
+    case 2: return launch_spmv_split<TV, TX, TA, MODE, DIFF, 2>(c, st, val, x, y);
+    case 4: return launch_spmv_split<TV, TX, TA, MODE, DIFF, 4>(c, st, val, x, y);
+    default: return launch_spmv_split<TV, TX, TA, MODE, DIFF, 8>(c, st, val, x, y);
   }
 }
 
 // SELL SpMV over the full (non-symmetric) storage; the FP32 difference form
 // when the FP32 values were built that way.
 template <typename TV, typename TX, typename TA, int MODE>
-void launch_spmv(const Ctx* c, cudaStream_t st, const TV* val, const TX* x, TX* y) {
+int launch_spmv(const Ctx* c, cudaStream_t st, const TV* val, const TX* x, TX* y) {
   if constexpr (sizeof(TV) == 4) {
-    if (c->val32_diff) {
-      launch_spmv_diff<TV, TX, TA, MODE, true>(c, st, val, x, y);
-      return;
-    }
+    if (c->val32_diff) return launch_spmv_diff<TV, TX, TA, MODE, true>(c, st, val, x, y);
   }
-  launch_spmv_diff<TV, TX, TA, MODE, false>(c, st, val, x, y);
+  return launch_spmv_diff<TV, TX, TA, MODE, false>(c, st, val, x, y);
 }
 
 // Bulk L2 prefetch (cp.async.bulk.prefetch, the TMA unit) of the first k1
@@ -408,6 +382,28 @@ __device__ __forceinline__ void sym_prefetch(int lane, int k1, int ulen, int lle
   }
 }
 
+// The 9 values of lane t's block of one stored step of the symmetric storage
+// (p: the step's 288 values), by 16-byte loads (see spos): an FP32 block takes 3
+// load instructions instead of 9, an FP64 block 5, and the shifted reads of a
+// lower block (the 32 lanes' blocks begin inside one step and run into the
+// next row group) touch 12 cache lines instead of 18.
+template <typename TV>
+__device__ __forceinline__ void load_block(const TV* __restrict__ p, int t, TV (&v)[9]) {
+  if constexpr (sizeof(TV) == 4) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p) + t), b = __ldg(reinterpret_cast<const float4*>(p + 128) + t);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const double2 a = __ldg(reinterpret_cast<const double2*>(p + 64 * g) + t);
+      v[2 * g] = a.x;
+      v[2 * g + 1] = a.y;
+    }
+  }
+  v[8] = __ldg(p + 256 + t);
+}
+
 // y = K x from the symmetric storage: row i sums its upper blocks K_ij x_j
 // (j >= i, SELL-32, coalesced) and its lower blocks as transposes K_ji^T x_j of
 // the blocks stored by the earlier rows j.  Those transposed reads are from
@@ -432,7 +428,7 @@ __global__ void __launch_bounds__(kSpmvBlock)
     const int ulen = (int)((uptr[s + 1] - ub) >> 5);
     const int llen = (int)((lptr[s + 1] - lb) >> 5);
     const int32_t* ucp = ucol + ub + t;
-    const TV* uvp = val + 9 * ub + t;
+    const TV* uvp = val + 9 * ub;
     const int32_t* lpp = lpos + lb + t;
     const int32_t* lcp = lcol + lb + t;
     // step j handles upper entry j and lower entry j, whose partners are read
@@ -441,20 +437,22 @@ __global__ void __launch_bounds__(kSpmvBlock)
     auto upper = [&](int j) {
       const int64_t cj = __ldcs(ucp + 32 * j);
       const TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
-      const TV* v = uvp + 288 * (int64_t)j;
-      a0 += (TA)v[0] * x0 + (TA)v[32] * x1 + (TA)v[64] * x2;
-      a1 += (TA)v[96] * x0 + (TA)v[128] * x1 + (TA)v[160] * x2;
-      a2 += (TA)v[192] * x0 + (TA)v[224] * x1 + (TA)v[256] * x2;
+      TV v[9];
+      load_block(uvp + 288 * (int64_t)j, t, v);
+      a0 += (TA)v[0] * x0 + (TA)v[1] * x1 + (TA)v[2] * x2;
+      a1 += (TA)v[3] * x0 + (TA)v[4] * x1 + (TA)v[5] * x2;
+      a2 += (TA)v[6] * x0 + (TA)v[7] * x1 + (TA)v[8] * x2;
     };
     auto lower = [&](int j) {
       const int64_t P = __ldcs(lpp + 32 * j);
       const int64_t cj = __ldcs(lcp + 32 * j);
       const TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
-      const TV* v = val + 9 * (P & ~int64_t(31)) + (P & 31);
+      TV v[9];
+      load_block(val + 9 * (P & ~int64_t(31)), (int)(P & 31), v);
       // transposed block: (K_ji^T x)_r = sum_c K_ji[c][r] x_c
-      a0 += (TA)__ldg(v) * x0 + (TA)__ldg(v + 96) * x1 + (TA)__ldg(v + 192) * x2;
-      a1 += (TA)__ldg(v + 32) * x0 + (TA)__ldg(v + 128) * x1 + (TA)__ldg(v + 224) * x2;
-      a2 += (TA)__ldg(v + 64) * x0 + (TA)__ldg(v + 160) * x1 + (TA)__ldg(v + 256) * x2;
+      a0 += (TA)v[0] * x0 + (TA)v[3] * x1 + (TA)v[6] * x2;
+      a1 += (TA)v[1] * x0 + (TA)v[4] * x1 + (TA)v[7] * x2;
+      a2 += (TA)v[2] * x0 + (TA)v[5] * x1 + (TA)v[8] * x2;
     };
     const int mlen = ulen < llen ? ulen : llen;
     int j = 0;
@@ -497,17 +495,7 @@ __global__ void __launch_bounds__(kSpmvBlock)
         dot[0] = (double)((TA)x[3 * row] * a0 + (TA)x[3 * row + 1] * a1 + (TA)x[3 * row + 2] * a2);
     }
   }
-  if (MODE == kCg) {
-    double tot[1];
-    if (grid_sum<1, sizeof(TV) == 4>(dot, partials, &scal->ticket[0], tot)) {
-      scal->pq = tot[0];
-      if (!(fabs(tot[0]) > 1e-300) || !isfinite(tot[0])) {
-        scal->stop = 3;
-      } else {
-        scal->alpha = scal->rz / tot[0];
-      }
-    }
-  }
+  if (MODE == kCg) block_partial<1>(dot, partials);
 }
 
 // The symmetric product with coded indices (stencil-like patterns, see
@@ -546,7 +534,7 @@ __global__ void __launch_bounds__(kSpmvBlock)
     const uint4 uc = __ldcs(ucode + row), lc = __ldcs(lcode + row);
     uint64_t ulo = uc.x | ((uint64_t)uc.y << 32), uhi = uc.z | ((uint64_t)uc.w << 32);
     uint64_t llo = lc.x | ((uint64_t)lc.y << 32), lhi = lc.z | ((uint64_t)lc.w << 32);
-    const TV* uvp = val + 9 * ub + t;
+    const TV* uvp = val + 9 * ub;
     if (t == 0) {
       const int k1 = (sizeof(TV) == 8 ? 4 : 8) < ulen ? (sizeof(TV) == 8 ? 4 : 8) : ulen;
       if (k1 > 0)
@@ -565,10 +553,11 @@ __global__ void __launch_bounds__(kSpmvBlock)
         x1 = (TA)__ldg(x + 3 * cj + 1);
         x2 = (TA)__ldg(x + 3 * cj + 2);
       }
-      const TV* v = uvp + 288 * (int64_t)j;
-      a0 += (TA)v[0] * x0 + (TA)v[32] * x1 + (TA)v[64] * x2;
-      a1 += (TA)v[96] * x0 + (TA)v[128] * x1 + (TA)v[160] * x2;
-      a2 += (TA)v[192] * x0 + (TA)v[224] * x1 + (TA)v[256] * x2;
+      TV v[9];
+      load_block(uvp + 288 * (int64_t)j, t, v);
+      a0 += (TA)v[0] * x0 + (TA)v[1] * x1 + (TA)v[2] * x2;
+      a1 += (TA)v[3] * x0 + (TA)v[4] * x1 + (TA)v[5] * x2;
+      a2 += (TA)v[6] * x0 + (TA)v[7] * x1 + (TA)v[8] * x2;
     };
     auto lower = [&](int) {
       const unsigned b = (unsigned)(llo & 0xFF);
@@ -578,10 +567,11 @@ __global__ void __launch_bounds__(kSpmvBlock)
         const int64_t cj = row - soff[b >> 4];
         const int64_t P = __ldg(uptr + (cj >> 5)) + 32 * (int64_t)(b & 15u) + (cj & 31);
         const TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
-        const TV* v = val + 9 * (P & ~int64_t(31)) + (P & 31);
-        a0 += (TA)__ldg(v) * x0 + (TA)__ldg(v + 96) * x1 + (TA)__ldg(v + 192) * x2;
-        a1 += (TA)__ldg(v + 32) * x0 + (TA)__ldg(v + 128) * x1 + (TA)__ldg(v + 224) * x2;
-        a2 += (TA)__ldg(v + 64) * x0 + (TA)__ldg(v + 160) * x1 + (TA)__ldg(v + 256) * x2;
+        TV v[9];
+        load_block(val + 9 * (P & ~int64_t(31)), (int)(P & 31), v);
+        a0 += (TA)v[0] * x0 + (TA)v[3] * x1 + (TA)v[6] * x2;
+        a1 += (TA)v[1] * x0 + (TA)v[4] * x1 + (TA)v[7] * x2;
+        a2 += (TA)v[2] * x0 + (TA)v[5] * x1 + (TA)v[8] * x2;
       }
     };
     const int mlen = ulen < llen ? ulen : llen;
@@ -607,17 +597,7 @@ __global__ void __launch_bounds__(kSpmvBlock)
         dot[0] += (double)((TA)x[3 * row] * a0 + (TA)x[3 * row + 1] * a1 + (TA)x[3 * row + 2] * a2);
     }
   }
-  if (MODE == kCg) {
-    double tot[1];
-    if (grid_sum<1, sizeof(TV) == 4>(dot, partials, &scal->ticket[0], tot)) {
-      scal->pq = tot[0];
-      if (!(fabs(tot[0]) > 1e-300) || !isfinite(tot[0])) {
-        scal->stop = 3;
-      } else {
-        scal->alpha = scal->rz / tot[0];
-      }
-    }
-  }
+  if (MODE == kCg) block_partial<1>(dot, partials);
 }
 
 // The symmetric product with SPLIT warps per slice for meshes with too few
@@ -643,25 +623,27 @@ __global__ void __launch_bounds__(kSpmvBlock)
     const int ulen = (int)((uptr[s + 1] - ub) >> 5);
     const int llen = (int)((lptr[s + 1] - lb) >> 5);
     const int32_t* ucp = ucol + ub + lane;
-    const TV* uvp = val + 9 * ub + lane;
+    const TV* uvp = val + 9 * ub;
     const int32_t* lpp = lpos + lb + lane;
     const int32_t* lcp = lcol + lb + lane;
     auto upper = [&](int j) {
       const int64_t cj = __ldcs(ucp + 32 * j);
       const TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
-      const TV* v = uvp + 288 * (int64_t)j;
-      a0 += (TA)v[0] * x0 + (TA)v[32] * x1 + (TA)v[64] * x2;
-      a1 += (TA)v[96] * x0 + (TA)v[128] * x1 + (TA)v[160] * x2;
-      a2 += (TA)v[192] * x0 + (TA)v[224] * x1 + (TA)v[256] * x2;
+      TV v[9];
+      load_block(uvp + 288 * (int64_t)j, lane, v);
+      a0 += (TA)v[0] * x0 + (TA)v[1] * x1 + (TA)v[2] * x2;
+      a1 += (TA)v[3] * x0 + (TA)v[4] * x1 + (TA)v[5] * x2;
+      a2 += (TA)v[6] * x0 + (TA)v[7] * x1 + (TA)v[8] * x2;
     };
     auto lower = [&](int j) {
       const int64_t P = __ldcs(lpp + 32 * j);
       const int64_t cj = __ldcs(lcp + 32 * j);
       const TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
-      const TV* v = val + 9 * (P & ~int64_t(31)) + (P & 31);
-      a0 += (TA)__ldg(v) * x0 + (TA)__ldg(v + 96) * x1 + (TA)__ldg(v + 192) * x2;
-      a1 += (TA)__ldg(v + 32) * x0 + (TA)__ldg(v + 128) * x1 + (TA)__ldg(v + 224) * x2;
-      a2 += (TA)__ldg(v + 64) * x0 + (TA)__ldg(v + 160) * x1 + (TA)__ldg(v + 256) * x2;
+      TV v[9];
+      load_block(val + 9 * (P & ~int64_t(31)), (int)(P & 31), v);
+      a0 += (TA)v[0] * x0 + (TA)v[3] * x1 + (TA)v[6] * x2;
+      a1 += (TA)v[1] * x0 + (TA)v[4] * x1 + (TA)v[7] * x2;
+      a2 += (TA)v[2] * x0 + (TA)v[5] * x1 + (TA)v[8] * x2;
     };
     const int mlen = ulen < llen ? ulen : llen;
     int j = part;
@@ -695,17 +677,7 @@ __global__ void __launch_bounds__(kSpmvBlock)
     y[3 * row + 2] = (TX)a2;
     if (MODE == kCg) dot[0] = (double)((TA)x[3 * row] * a0 + (TA)x[3 * row + 1] * a1 + (TA)x[3 * row + 2] * a2);
   }
-  if (MODE == kCg) {
-    double tot[1];
-    if (grid_sum<1>(dot, partials, &scal->ticket[0], tot)) {
-      scal->pq = tot[0];
-      if (!(fabs(tot[0]) > 1e-300) || !isfinite(tot[0])) {
-        scal->stop = 3;
-      } else {
-        scal->alpha = scal->rz / tot[0];
-      }
-    }
-  }
+  if (MODE == kCg) block_partial<1>(dot, partials);
 }
 
 // 4 consecutive entries through 16-byte loads and stores (cudaMalloc bases are
@@ -731,14 +703,42 @@ __device__ __forceinline__ void st4(T* __restrict__ p, const T (&o)[4]) {
   }
 }
 
+// Sum of the nb per-block partials of the product, for grids too large to be
+// summed again by every block of the update: one block, result in out[0].
+__global__ void __launch_bounds__(1024)
+    k_cg_sum(const double* __restrict__ partials, int nb, double* __restrict__ out, const CgScalars* __restrict__ scal) {
+  pdl_enter();
+  if (halted(scal)) return;
+  double tot[1];
+  sum_partials<1>(partials, nb, tot);
+  if (threadIdx.x == 0) out[0] = tot[0];
+}
+
+// x += alpha p, r -= alpha q with alpha = r.z / p.q (p.q from the product's nb
+// partials), and the block's partials of r.z and r.r.  Block 0 moves the
+// scalars on; the other blocks read only scal->rz, which this kernel leaves alone.
 template <typename T>
 __global__ void __launch_bounds__(kVecBlock)
     k_cg_update(int64_t n, const T* __restrict__ p, const T* __restrict__ q, T* __restrict__ r,
                 double* __restrict__ x, const T* __restrict__ dinv, CgScalars* __restrict__ scal,
-                double* __restrict__ partials) {
+                const double* __restrict__ pq_partials, int nb, double* __restrict__ partials) {
   pdl_enter();
   if (halted(scal)) return;
-  const double alpha = scal->alpha;
+  double pq[1];
+  sum_partials<1>(pq_partials, nb, pq);
+  const bool broken = !(fabs(pq[0]) > 1e-300) || !isfinite(pq[0]);
+  const double alpha = scal->rz / pq[0];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    scal->pq = pq[0];
+    if (broken) {
+      scal->stop = 3;
+    } else {
+      scal->alpha = alpha;
+      scal->rz_old = scal->rz;
+      scal->iter += 1;
+    }
+  }
+  if (broken) return;
   const T a = (T)alpha;
   T rz = T(0), rr = T(0);
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
@@ -772,33 +772,49 @@ __global__ void __launch_bounds__(kVecBlock)
     rz += ri * zi;
     rr += ri * ri;
   }
-  double v[2] = {(double)rz, (double)rr}, tot[2];
-  if (grid_sum<2>(v, partials, &scal->ticket[1], tot)) {
-    const double rz_old = scal->rz;
-    scal->rz_old = rz_old;
-    scal->rz = tot[0];
-    scal->rr = tot[1];
-    scal->beta = tot[0] / rz_old;
-    const int it = scal->iter + 1;
-    scal->iter = it;
-    if (scal->hist && it <= scal->hist_cap) scal->hist[it - 1] = tot[1];
-    if (tot[1] <= scal->tol2) scal->stop = 1;
-    else if (!(fabs(rz_old) > 1e-300) || !isfinite(tot[0])) scal->stop = 3;
-    else if (it >= scal->max_iter) scal->stop = 2;
-    if (scal->delta2 > 0.0 && tot[1] < scal->delta2 * scal->rr_ref) scal->want_update = 1;
-  }
+  double v[2] = {(double)rz, (double)rr};
+  block_partial<2>(v, partials);
 }
 
+// p = D^-1 r + beta p.  In the iteration (nb > 0) r.z and r.r come from the
+// update's nb partials, every block takes the same decisions from them (stop
+// test, refinement trigger: then p stays), and block 0 records them; the others
+// read only scalars that this kernel leaves alone.  On its own (nb = 0) it
+// takes scal->beta.
 template <typename T>
 __global__ void __launch_bounds__(kVecBlock)
     k_cg_pupdate(int64_t n, const T* __restrict__ r, const T* __restrict__ dinv, T* __restrict__ p,
-                 const CgScalars* __restrict__ scal) {
+                 CgScalars* __restrict__ scal, const double* __restrict__ partials, int nb) {
   pdl_enter();
   if (halted(scal)) return;
-  const T beta = (T)scal->beta;
+  double b;
+  if (nb > 0) {
+    double tot[2];
+    sum_partials<2>(partials, nb, tot);
+    const double rz_old = scal->rz_old;
+    const int it = scal->iter;
+    int stop = 0, want = 0;
+    if (tot[1] <= scal->tol2) stop = 1;
+    else if (!(fabs(rz_old) > 1e-300) || !isfinite(tot[0])) stop = 3;
+    else if (it >= scal->max_iter) stop = 2;
+    if (scal->delta2 > 0.0 && tot[1] < scal->delta2 * scal->rr_ref) want = 1;
+    b = tot[0] / rz_old;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      scal->rz = tot[0];
+      scal->rr = tot[1];
+      scal->beta = b;
+      if (scal->hist && it <= scal->hist_cap) scal->hist[it - 1] = tot[1];
+      if (stop) scal->stop = stop;
+      if (want) scal->want_update = 1;
+    }
+    if (stop | want) return;
+  } else {
+    b = scal->beta;
+  }
+  const T beta = (T)b;
   // beta = 0 (start, restart after a breakdown): p = z without reading p, whose
   // contents are then undefined (fresh memory, or the NaN of the breakdown)
-  const bool fresh = scal->beta == 0.0;
+  const bool fresh = b == 0.0;
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t n4 = n >> 2;
   for (int64_t k = gid; k < n4; k += stride) {
@@ -902,45 +918,60 @@ Vecs<TV, TX> vecs(Ctx* c, bool precond) {
 }
 
 template <typename TV, typename TX, typename TA, int MODE, int SPLIT>
-void launch_spmv_sym_split(const Ctx* c, cudaStream_t st, const TV* val, const TX* x, TX* y) {
+int launch_spmv_sym_split(const Ctx* c, cudaStream_t st, const TV* val, const TX* x, TX* y) {
   constexpr int per_block = kSpmvBlock / 32 / SPLIT;
   const int grid = (int)((c->nslices + per_block - 1) / per_block);
-  launch_mode<MODE>(k_spmv_sym_split<TV, TX, TA, MODE, SPLIT>, grid, kSpmvBlock, st, c->N, c->nslices, c->uptr,
-                    c->ucol, c->lptr, c->lpos, c->lcol, val, x, y, c->scal, c->partials);
+  return launch_mode<MODE>(k_spmv_sym_split<TV, TX, TA, MODE, SPLIT>, grid, kSpmvBlock, st, c->N, c->nslices, c->uptr,
+                           c->ucol, c->lptr, c->lpos, c->lcol, val, x, y, c->scal, c->partials);
 }
 
 // The symmetric product: one warp per slice (grid = slices / 8 blocks), or
 // SPLIT warps per slice on small meshes (the rule of spmv_split).
 template <typename TV, typename TX, typename TA, int MODE>
-void launch_spmv_sym(const Ctx* c, int grid, cudaStream_t st, const TV* val, const TX* x, TX* y) {
+int launch_spmv_sym(const Ctx* c, int grid, cudaStream_t st, const TV* val, const TX* x, TX* y) {
   switch (spmv_split(c)) {
     case 1:
       if (c->sym_coded)
-        launch_mode<MODE>(k_spmv_symc<TV, TX, TA, MODE>,
-                          sizeof(TV) == 8 ? std::min(grid, 15 * sm_count_solver()) : grid, kSpmvBlock, st, c->N, c->nslices * kSlice, c->uptr,
-                          c->lptr, reinterpret_cast<const uint4*>(c->sym_ucode),
-                          reinterpret_cast<const uint4*>(c->sym_lcode), c->sym_tab, val, x, y, c->scal, c->partials);
-      else
-        launch_mode<MODE>(k_spmv_sym<TV, TX, TA, MODE>, grid, kSpmvBlock, st, c->N, c->nslices * kSlice, c->uptr,
-                          c->ucol, c->lptr, c->lpos, c->lcol, val, x, y, c->scal, c->partials);
-      break;
-    case 2: launch_spmv_sym_split<TV, TX, TA, MODE, 2>(c, st, val, x, y); break;
-    case 4: launch_spmv_sym_split<TV, TX, TA, MODE, 4>(c, st, val, x, y); break;
-    default: launch_spmv_sym_split<TV, TX, TA, MODE, 8>(c, st, val, x, y); break;
+        return launch_mode<MODE>(k_spmv_symc<TV, TX, TA, MODE>,
+                                 sizeof(TV) == 8 ? std::min(grid, 15 * sm_count_solver()) : grid, kSpmvBlock, st, c->N,
+                                 c->nslices * kSlice, c->uptr, c->lptr, reinterpret_cast<const uint4*>(c->sym_ucode),
+                                 reinterpret_cast<const uint4*>(c->sym_lcode), c->sym_tab, val, x, y, c->scal,
+                                 c->partials);
+      return launch_mode<MODE>(k_spmv_sym<TV, TX, TA, MODE>, grid, kSpmvBlock, st, c->N, c->nslices * kSlice, c->uptr,
+                               c->ucol, c->lptr, c->lpos, c->lcol, val, x, y, c->scal, c->partials);
+    case 2: return launch_spmv_sym_split<TV, TX, TA, MODE, 2>(c, st, val, x, y);
+    case 4: return launch_spmv_sym_split<TV, TX, TA, MODE, 4>(c, st, val, x, y);
+    default: return launch_spmv_sym_split<TV, TX, TA, MODE, 8>(c, st, val, x, y);
   }
+}
+
+// The product's partials for the update: as they are, or summed first by one
+// block when every block of the update would have to read more than
+// kMaxPartials of them.
+constexpr int kMaxPartials = 2560;
+struct Partials {
+  const double* p;
+  int nb;
+};
+Partials product_partials(Ctx* c, cudaStream_t st, int nb) {
+  if (nb <= kMaxPartials) return {c->partials, nb};
+  double* out = c->partials + c->partials_cap - 1;
+  launch_pdl(k_cg_sum, 1, 1024, st, (const double*)c->partials, nb, out, (const CgScalars*)c->scal);
+  c->launches += 1;
+  return {out, 1};
 }
 
 template <typename TV, typename TX, typename TA>
 void launch_iteration(const Run& R, const Vecs<TV, TX>& V, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1) {
   Ctx* c = R.c;
   if (ev0) cudaEventRecord(ev0, st);
-  if (V.sym)
-    launch_spmv_sym<TV, TX, TA, kCg>(c, R.sg, st, V.val, V.p, V.q);
-  else
-    launch_spmv<TV, TX, TA, kCg>(c, st, V.val, V.p, V.q);
+  const int nb = V.sym ? launch_spmv_sym<TV, TX, TA, kCg>(c, R.sg, st, V.val, V.p, V.q)
+                       : launch_spmv<TV, TX, TA, kCg>(c, st, V.val, V.p, V.q);
   if (ev1) cudaEventRecord(ev1, st);
-  launch_pdl(k_cg_update<TX>, R.vg, kVecBlock, st, R.n, V.p, V.q, V.r, c->x64, V.dinv, c->scal, c->partials);
-  launch_pdl(k_cg_pupdate<TX>, R.vg, kVecBlock, st, R.n, V.r, V.dinv, V.p, c->scal);
+  const Partials pq = product_partials(c, st, nb);
+  double* rz = c->partials + c->partials_cap / 2;  // the update's partials, behind the product's
+  launch_pdl(k_cg_update<TX>, R.vg, kVecBlock, st, R.n, V.p, V.q, V.r, c->x64, V.dinv, c->scal, pq.p, pq.nb, rz);
+  launch_pdl(k_cg_pupdate<TX>, R.vg, kVecBlock, st, R.n, V.r, V.dinv, V.p, c->scal, (const double*)rz, R.vg);
   c->launches += 3;
 }
 
@@ -973,7 +1004,7 @@ int replace(const Run& R, const Vecs<TV, TX>& V, int mode) {
   UFC_CUDA(c, cudaGetLastError());
   c->launches += 1;
   if (mode != 0) {
-    k_cg_pupdate<TX><<<R.vg, kVecBlock, 0, c->stream>>>(R.n, V.r, V.dinv, V.p, c->scal);
+    k_cg_pupdate<TX><<<R.vg, kVecBlock, 0, c->stream>>>(R.n, V.r, V.dinv, V.p, c->scal, nullptr, 0);
     UFC_CUDA(c, cudaGetLastError());
     c->launches += 1;
   }
@@ -987,7 +1018,7 @@ int read_scalars(Ctx* c) {
 }
 
 template <typename TV, typename TX, typename TA>
-int get_graph(const Run& R, const Vecs<TV, TX>& V, int batch, cudaGraphExec_t* out) {
+int get_graph(const Run& R, const Vecs<TV, TX>& V, int batch, cudaGraphExec_t* out, int64_t* launches) {
   Ctx* c = R.c;
   // one cached graph per (value, vector, accumulator) type combination
   const int slot = sizeof(TV) == 8 ? 0 : sizeof(TX) == 8 ? 3 : sizeof(TA) == 8 ? 2 : 1;
@@ -1004,6 +1035,7 @@ int get_graph(const Run& R, const Vecs<TV, TX>& V, int batch, cudaGraphExec_t* o
       c->cg_graph_val[slot] == val && c->cg_graph_form[slot] == form && c->cg_graph_n[slot] == R.n &&
       c->cg_graph_slices[slot] == c->nslices) {
     *out = c->cg_graph[slot];
+    *launches = c->cg_graph_launches[slot];
     return UFC_STATUS_OK;
   }
   if (c->cg_graph[slot]) cudaGraphExecDestroy(c->cg_graph[slot]);
@@ -1013,6 +1045,7 @@ int get_graph(const Run& R, const Vecs<TV, TX>& V, int batch, cudaGraphExec_t* o
   UFC_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   for (int k = 0; k < batch; ++k) launch_iteration<TV, TX, TA>(R, V, c->stream, nullptr, nullptr);
   cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+  *launches = c->cg_graph_launches[slot] = c->launches - counted;
   c->launches = counted;
   if (e != cudaSuccess) return cuda_fail(c, e, "cudaStreamEndCapture");
   e = cudaGraphInstantiate(&c->cg_graph[slot], g, 0);
@@ -1107,7 +1140,8 @@ int pcg_run(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
     UFC_CUDA(c, cudaMemcpyAsync(&c->scal->tol2, &tol2, sizeof(double), cudaMemcpyHostToDevice, c->stream));
     UFC_TRY(replace(R, V, 2));
     cudaGraphExec_t graph = nullptr;
-    if (!c->instrument) UFC_TRY((get_graph<TV, TX, TA>(R, V, batch, &graph)));
+    int64_t graph_launches = 0;
+    if (!c->instrument) UFC_TRY((get_graph<TV, TX, TA>(R, V, batch, &graph, &graph_launches)));
     std::vector<cudaEvent_t> evs;
     if (c->instrument) {
       evs.resize(2 * batch);
@@ -1134,7 +1168,7 @@ int pcg_run(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
           status = cuda_fail(c, e, "cudaGraphLaunch");
           break;
         }
-        c->launches += 3 * (int64_t)batch;
+        c->launches += graph_launches;
       } else {
         for (int k = 0; k < batch; ++k)
           launch_iteration<TV, TX, TA>(R, V, c->stream, evs[2 * k], evs[2 * k + 1]);
@@ -1314,11 +1348,27 @@ void spmv32_on(const Ctx* lvl, cudaStream_t st, const float* val, const float* x
     launch_spmv_diff<float, float, float, kPlain, false>(lvl, st, val, x, y);
 }
 
-void cg_spmv64(Ctx* c, const double* p, double* q) {
-  if (c->has_sval64)
-    launch_spmv_sym<double, double, double, kCg>(c, sym_grid(c), c->stream, c->sval64, p, q);
+// alpha = r.z / p.q from the product's partials (the multigrid PCG).
+__global__ void __launch_bounds__(1024)
+    k_cg_alpha(const double* __restrict__ partials, int nb, CgScalars* __restrict__ scal) {
+  pdl_enter();
+  if (halted(scal)) return;
+  double tot[1];
+  sum_partials<1>(partials, nb, tot);
+  if (threadIdx.x != 0) return;
+  scal->pq = tot[0];
+  if (!(fabs(tot[0]) > 1e-300) || !isfinite(tot[0]))
+    scal->stop = 3;
   else
-    launch_spmv<double, double, double, kCg>(c, c->stream, c->val64, p, q);
+    scal->alpha = scal->rz / tot[0];
+}
+
+void cg_spmv64(Ctx* c, const double* p, double* q) {
+  const int nb = c->has_sval64
+                     ? launch_spmv_sym<double, double, double, kCg>(c, sym_grid(c), c->stream, c->sval64, p, q)
+                     : launch_spmv<double, double, double, kCg>(c, c->stream, c->val64, p, q);
+  launch_pdl(k_cg_alpha, 1, 1024, c->stream, (const double*)c->partials, nb, c->scal);
+  c->launches += 1;
 }
 
 int true_residual_fp64(Ctx* c, bool want_bb) {

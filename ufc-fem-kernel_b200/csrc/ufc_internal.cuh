@@ -211,6 +211,7 @@ struct Ctx {
   // cached CUDA graphs of CG batches
   cudaGraphExec_t cg_graph[kGraphSlots] = {};
   int cg_graph_batch[kGraphSlots] = {};
+  int64_t cg_graph_launches[kGraphSlots] = {};  // kernels in one graph
   // what a cached graph baked in: value and diagonal arrays, storage and SpMV form
   const void* cg_graph_val[kGraphSlots] = {};
   const void* cg_graph_key[kGraphSlots] = {};
