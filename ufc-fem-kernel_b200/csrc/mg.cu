@@ -38,28 +38,37 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <cstddef>
 #include <vector>
 
 #include "c3d8_device.cuh"
 #include "reduce.cuh"
+#include "rows.cuh"
+#include "spmv.cuh"
 #include "ufc_internal.cuh"
 
 namespace ufc {
+
+template <typename T>
+struct MgVecs {
+  T *x = nullptr, *b = nullptr, *r = nullptr, *d = nullptr, *e = nullptr, *w = nullptr;
+};
 
 struct MgLevel {
   Ctx* c = nullptr;          // the level's context (level 0: the owner)
   ufc_ctx* own = nullptr;    // levels >= 1: a context holding the coarse box
   int32_t nx = 0, ny = 0, nz = 0;
-  double* ke = nullptr;      // levels >= 1: Galerkin element matrices [E][24][24]
-  // FP64 cycle: level vectors (level 0: x and b are the PCG's z and r)
-  double *x = nullptr, *b = nullptr, *r = nullptr, *d = nullptr, *w = nullptr;
-  // FP32 cycle: level vectors, and the level's values and diagonal rounded to FP32
-  float *x32 = nullptr, *b32 = nullptr, *r32 = nullptr, *d32 = nullptr, *w32 = nullptr;
-  float *val32 = nullptr, *dinv32 = nullptr;
-  bool own_xb = false;       // x and b allocated here
-  double lmax = 0.0;
-  double* inv = nullptr;     // coarsest level: dense inverse [n][n]
+  double* ke = nullptr;      // levels >= 1: Galerkin element matrices [E][9][64], node pairs by sign bits
+  // vectors of the cycle, in its precision (FP64, level 0: x and b are the PCG's z and r)
+  MgVecs<double> v64;
+  MgVecs<float> v32;
+  // FP32 cycle: the level's values and diagonal rounded to FP32, and the
+  // symmetric storage rounded where the level holds it in FP64 only
+  float *val32 = nullptr, *sval32 = nullptr, *dinv32 = nullptr;
+  double* coef = nullptr;    // smoother: lambda_max, 1/theta, then c1, c2 of every further step
+  double* inv = nullptr;     // coarsest level: dense inverse [ld][ld], ld = n rounded up to 32
   float* inv32 = nullptr;
+  double* gj = nullptr;      // its elimination's column panel and pivot block
   double *pv = nullptr, *pw = nullptr;  // power-iteration vectors (lambda_max), kept across refreshes
 };
 
@@ -70,7 +79,14 @@ struct Mg {
   bool stale = false;
   bool fp32 = false;         // the cycle runs in FP32 (values, vectors); the PCG around it in FP64
   int cheb_coarse = 0;       // degree of the coarsest Chebyshev solve (0: dense inverse)
+  double lmax_scale = 1.0;   // raised when the smoother's interval proved too short
   double* dnorm = nullptr;   // ||v||^2 of the power iteration, on the device
+  int32_t* gj_flag = nullptr;  // set when the coarsest elimination met a pivot that is not positive
+  // the PCG iteration as a graph, and what it baked in
+  cudaGraphExec_t graph = nullptr;
+  int batch = 0;
+  int64_t graph_launches = 0;
+  const void* key[9] = {};
 };
 
 namespace {
@@ -96,304 +112,445 @@ __device__ __forceinline__ double hat(int A, int x0, int x1, int x2) {
   return w;
 }
 
-// Galerkin element matrices of one coarse level, one CTA of 64 threads per
-// coarse element.  FROM_KE: the child matrices are read from the finer level's
-// element matrices; otherwise they are computed from the fine elements (the
-// linear-elastic D, or the J2 tangent per Gauss point when Dt is given).
+// Galerkin element matrices of one coarse level: one CTA per coarse element, one
+// warp per child.  A lane holds the blocks (p, q) and (p + 4, q) of the child's
+// 8x8 block grid, p = lane / 8, q = lane % 8 in sign-bit numbering; FROM_KE
+// reads them from the finer level's element matrices, otherwise they are formed
+// from the fine element (linear-elastic D, or the J2 tangent per Gauss point)
+// as in the stiffness assembly.  The restriction W of P to the child is a
+// tensor product of 2x2 matrices, so W^T K W is three exchanges with the lane
+// whose q differs in one bit and three for p (two by shuffles, the last between
+// the lane's own two blocks); rows and columns of fixed DOFs are zeroed before
+// (fine) and after (coarse).  The 8 children are added in order.
+// 64x32x32, level 1 from the elements: 1298 us with one 64-thread CTA walking
+// through the children and the dense W, now 132 us.
+constexpr int kGalThreads = 256;
+
+template <bool TANGENT>
+struct GalWarp {
+  double X[24];
+  double g[8][8][3];                       // [gp][node][dir], scaled by sqrt(det J)
+  double M[TANGENT ? 8 : 1][8][18];        // [node][gp]: D B_a (J2)
+};
+
 template <bool FROM_KE, bool TANGENT>
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(kGalThreads)
     k_mg_galerkin(int32_t nxc, int32_t nyc, int32_t nzc, const double* __restrict__ coords,
-                  const int32_t* __restrict__ conn_f, const double* __restrict__ props, int nprops,
+                  const int32_t* __restrict__ conn_f, const double* __restrict__ lame,
                   const double* __restrict__ Dt, const double* __restrict__ ke_f, const uint8_t* __restrict__ fixed_f,
                   const int32_t* __restrict__ conn_c, const uint8_t* __restrict__ fixed_c, double* __restrict__ ke_c,
                   int32_t* __restrict__ err) {
-  __shared__ double Kc[576], Kf[576];
-  __shared__ double X[24], g[8][8][3], wdet[8];
-  __shared__ double D[TANGENT ? 8 : 1][36];
-  __shared__ uint8_t ff[24], fc[24];
-  const int t = threadIdx.x;
+  extern __shared__ __align__(16) unsigned char gal_smem[];
+  double* out = reinterpret_cast<double*>(gal_smem);  // [child][9][64], over the warps' areas
+  const int ch = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t ec = blockIdx.x;
   const int nxf = 2 * nxc, nyf = 2 * nyc;
   const int64_t I = ec % nxc, J = (ec / nxc) % nyc, K = ec / ((int64_t)nxc * nyc);
-  for (int q = t; q < 576; q += 64) Kc[q] = 0.0;
-  if (t < 24) fc[t] = fixed_c[3 * (int64_t)conn_c[ec * 8 + t / 3] + t % 3];
-  for (int ch = 0; ch < 8; ++ch) {
-    const int ca = ch & 1, cb = (ch >> 1) & 1, cc = ch >> 2;
-    const int64_t ef = (2 * I + ca) + (int64_t)nxf * ((2 * J + cb) + (int64_t)nyf * (2 * K + cc));
-    __syncthreads();  // Kf and the gradients of the previous child are consumed
-    if (t < 24) ff[t] = fixed_f[3 * (int64_t)conn_f[ef * 8 + t / 3] + t % 3];
-    if (FROM_KE) {
-      for (int q = t; q < 576; q += 64) Kf[q] = ke_f[ef * 576 + q];
-    } else {
-      if (t < 24) X[t] = coords[(int64_t)conn_f[ef * 8 + t / 3] * 3 + t % 3];
-      if (TANGENT)
-        for (int q = t; q < 288; q += 64) {
-          const int gp = q / 36, i = (q % 36) / 6, j = q % 6, lo = min(i, j), hi = max(i, j);
-          D[TANGENT ? gp : 0][q % 36] = Dt[ef * 168 + 8 * (lo * 6 - lo * (lo - 1) / 2 + hi - lo) + gp];
+  const int cb[3] = {ch & 1, (ch >> 1) & 1, ch >> 2};
+  const int64_t ef = (2 * I + cb[0]) + (int64_t)nxf * ((2 * J + cb[1]) + (int64_t)nyf * (2 * K + cb[2]));
+  const int p = lane >> 3, q = lane & 7;
+  double B[2][9];
+  if constexpr (FROM_KE) {
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+      B[0][c] = ke_f[ef * 576 + 64 * c + lane];
+      B[1][c] = ke_f[ef * 576 + 64 * c + 32 + lane];
+    }
+  } else {
+    GalWarp<TANGENT>& sm = reinterpret_cast<GalWarp<TANGENT>*>(gal_smem)[ch];
+    if (lane < 24) sm.X[lane] = coords[(int64_t)conn_f[ef * 8 + lane / 3] * 3 + lane % 3];
+    __syncwarp();
+    {
+      // Gauss point lane / 4, gradients of the two nodes 2 (lane % 4) and the next
+      const int gp = lane >> 2;
+      double J9[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) J9[k] = 0.0;
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        double d0, d1, d2;
+        dN_dxi<double>(gp, a, d0, d1, d2);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          J9[i] += d0 * sm.X[3 * a + i];
+          J9[3 + i] += d1 * sm.X[3 * a + i];
+          J9[6 + i] += d2 * sm.X[3 * a + i];
         }
-      __syncthreads();
-      if (t < 8) {
-        double inv[9];
-        const double det = jacobian_inv<double>(X, t, inv);
-        if (!(det > 0.0)) atomicOr(err, (int)kDevBadJacobian);
-        wdet[t] = det;
-#pragma unroll
-        for (int a = 0; a < 8; ++a) grad_x<double>(inv, t, a, g[t][a]);
       }
-      __syncthreads();
-      // thread t: block (p, q) of the 8x8 block grid of the child's Ke
-      const int p = t >> 3, q = t & 7;
-      double lam = 0.0, mu = 0.0;
-      if (!TANGENT) lame<double>(props[ef * nprops], props[ef * nprops + 1], lam, mu);
-      double Kb[9];
+      const double c0 = J9[4] * J9[8] - J9[5] * J9[7], c3 = J9[5] * J9[6] - J9[3] * J9[8],
+                   c6 = J9[3] * J9[7] - J9[4] * J9[6];
+      const double det = J9[0] * c0 + J9[1] * c3 + J9[2] * c6;
+      if (!(det > 0.0)) atomicOr(err, (int)kDevBadJacobian);
+      const double sc = rsqrt(det);
+      const double inv[9] = {c0 * sc, (J9[2] * J9[7] - J9[1] * J9[8]) * sc, (J9[1] * J9[5] - J9[2] * J9[4]) * sc,
+                             c3 * sc, (J9[0] * J9[8] - J9[2] * J9[6]) * sc, (J9[2] * J9[3] - J9[0] * J9[5]) * sc,
+                             c6 * sc, (J9[1] * J9[6] - J9[0] * J9[7]) * sc, (J9[0] * J9[4] - J9[1] * J9[3]) * sc};
 #pragma unroll
-      for (int k = 0; k < 9; ++k) Kb[k] = 0.0;
+      for (int h = 0; h < 2; ++h) {
+        const int t = 2 * (lane & 3) + h;
+        double g3[3];
+        grad_x<double>(inv, gp, bits_node(t), g3);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) sm.g[gp][t][i] = g3[i];
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) B[h][c] = 0.0;
+    if constexpr (TANGENT) {
+      // D B_a for node p (+ 4) at Gauss point q of this lane
+      constexpr int kIdx[3][3] = {{0, 3, 5}, {1, 3, 4}, {2, 4, 5}};
+      constexpr int kCmp[3][3] = {{0, 1, 2}, {1, 0, 2}, {2, 1, 0}};
+      double D[21];
+#pragma unroll
+      for (int k = 0; k < 21; ++k) D[k] = Dt[(ef * 21 + k) * 8 + q];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double* ga = sm.g[q][p + 4 * h];
+        double* M = sm.M[p + 4 * h][q];
+#pragma unroll
+        for (int v = 0; v < 6; ++v)
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+            M[v * 3 + i] = D[tri6(v, kIdx[i][0])] * ga[kCmp[i][0]] + D[tri6(v, kIdx[i][1])] * ga[kCmp[i][1]] +
+                           D[tri6(v, kIdx[i][2])] * ga[kCmp[i][2]];
+      }
+      __syncwarp();
 #pragma unroll 1
       for (int gp = 0; gp < 8; ++gp) {
-        const double* ga = g[gp][p];
-        const double* gb = g[gp][q];
-        if (TANGENT) {
-          constexpr int kIdx[3][3] = {{0, 3, 5}, {1, 3, 4}, {2, 4, 5}};
-          constexpr int kCmp[3][3] = {{0, 1, 2}, {1, 0, 2}, {2, 1, 0}};
-          const double* Dg = D[TANGENT ? gp : 0];
-          double DB[6][3];
+        const double* gb = sm.g[gp][q];
 #pragma unroll
-          for (int k = 0; k < 6; ++k)
-#pragma unroll
-            for (int j = 0; j < 3; ++j)
-              DB[k][j] = Dg[k * 6 + kIdx[j][0]] * gb[kCmp[j][0]] + Dg[k * 6 + kIdx[j][1]] * gb[kCmp[j][1]] +
-                         Dg[k * 6 + kIdx[j][2]] * gb[kCmp[j][2]];
+        for (int h = 0; h < 2; ++h) {
+          const double* M = sm.M[p + 4 * h][gp];
 #pragma unroll
           for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = 0; j < 3; ++j)
-              Kb[i * 3 + j] += wdet[gp] * (ga[kCmp[i][0]] * DB[kIdx[i][0]][j] + ga[kCmp[i][1]] * DB[kIdx[i][1]][j] +
-                                           ga[kCmp[i][2]] * DB[kIdx[i][2]][j]);
-        } else {
-          const double dot = ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2];
-#pragma unroll
-          for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-              double v = lam * ga[i] * gb[j] + mu * ga[j] * gb[i];
-              if (i == j) v += mu * dot;
-              Kb[i * 3 + j] += wdet[gp] * v;
-            }
+              B[h][3 * i + j] += M[kIdx[j][0] * 3 + i] * gb[kCmp[j][0]] + M[kIdx[j][1] * 3 + i] * gb[kCmp[j][1]] +
+                                 M[kIdx[j][2] * 3 + i] * gb[kCmp[j][2]];
         }
       }
+    } else {
+#pragma unroll 2
+      for (int gp = 0; gp < 8; ++gp) {
+        const double* gb = sm.g[gp][q];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
+        for (int h = 0; h < 2; ++h) {
+          const double* ga = sm.g[gp][p + 4 * h];
 #pragma unroll
-        for (int j = 0; j < 3; ++j) Kf[(3 * p + i) * 24 + 3 * q + j] = Kb[i * 3 + j];
-    }
-    __syncthreads();
-    // thread t: coarse block (A, B) += sum_pq W(p, A) Kf[p][q] W(q, B), masked
-    const int A = t >> 3, B = t & 7;
-    double wA[8], wB[8];
+          for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
-      const int o0 = ca + ((node_sign(p, 0) + 1) >> 1) - 1, o1 = cb + ((node_sign(p, 1) + 1) >> 1) - 1,
-                o2 = cc + ((node_sign(p, 2) + 1) >> 1) - 1;
-      wA[p] = hat(A, o0, o1, o2);
-      wB[p] = hat(B, o0, o1, o2);
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        if (fc[3 * A + i] || fc[3 * B + j]) continue;
-        double acc = 0.0;
-#pragma unroll
-        for (int p = 0; p < 8; ++p) {
-          if (wA[p] == 0.0 || ff[3 * p + i]) continue;
-          double row = 0.0;
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            if (wB[q] != 0.0 && !ff[3 * q + j]) row += Kf[(3 * p + i) * 24 + 3 * q + j] * wB[q];
-          acc += wA[p] * row;
+            for (int j = 0; j < 3; ++j) B[h][3 * i + j] += ga[i] * gb[j];
         }
-        Kc[(3 * A + i) * 24 + 3 * B + j] += acc;
+      }
+      const double lam = lame[2 * ef], mu = lame[2 * ef + 1];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double tr = mu * (B[h][0] + B[h][4] + B[h][8]);
+        double k9[9];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            k9[3 * i + j] = lam * B[h][3 * i + j] + mu * B[h][3 * j + i];
+            if (i == j) k9[3 * i + j] += tr;
+          }
+#pragma unroll
+        for (int c = 0; c < 9; ++c) B[h][c] = k9[c];
+      }
+    }
+  }
+  // zero rows and columns of P at fixed fine DOFs
+  {
+    const int64_t nq = conn_f[ef * 8 + bits_node(q)];
+    bool fq[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) fq[j] = fixed_f[3 * nq + j] != 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int64_t np = conn_f[ef * 8 + bits_node(p + 4 * h)];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const bool fp = fixed_f[3 * np + i] != 0;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          if (fp || fq[j]) B[h][3 * i + j] = 0.0;
+      }
+    }
+  }
+  // W^T K W, one direction at a time: a lane's block with node bit b takes the
+  // weight of its own block and of the one with the other bit (a coarse node on
+  // the child's side of the box, b == cb: 1 and 1/2; across it: 1/2 and 0)
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+    const int dir = s < 3 ? s : s - 3, bit = (lane >> s) & 1;
+    const double wo = bit == cb[dir] ? 1.0 : 0.5, wx = bit == cb[dir] ? 0.5 : 0.0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) {
+        const double other = __shfl_xor_sync(0xffffffffu, B[h][c], 1 << s);
+        B[h][c] = wo * B[h][c] + wx * other;
       }
   }
+#pragma unroll
+  for (int c = 0; c < 9; ++c) {
+    const double lo = B[0][c], hi = B[1][c];
+    B[0][c] = cb[2] == 0 ? lo + 0.5 * hi : 0.5 * lo;
+    B[1][c] = cb[2] == 0 ? 0.5 * hi : hi + 0.5 * lo;
+  }
+  __syncthreads();  // the warps' areas are consumed
+#pragma unroll
+  for (int c = 0; c < 9; ++c) {
+    out[ch * 576 + 64 * c + lane] = B[0][c];
+    out[ch * 576 + 64 * c + 32 + lane] = B[1][c];
+  }
   __syncthreads();
-  for (int q = t; q < 576; q += 64) ke_c[ec * 576 + q] = Kc[q];
-}
-
-// Scatter of given element matrices into the SELL values, one thread per
-// (element, node pair) of one colour; rows and columns of fixed DOFs skipped.
-__global__ void k_mg_scatter(const int32_t* __restrict__ elems, int32_t ne, const int32_t* __restrict__ conn,
-                             const double* __restrict__ ke, const int32_t* __restrict__ slot,
-                             const uint8_t* __restrict__ fixed, double* __restrict__ val) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)ne * 64) return;
-  const int64_t e = elems[t >> 6];
-  const int a = (int)(t & 63) >> 3, b = (int)(t & 7);
-  const int64_t na = conn[e * 8 + a], nb = conn[e * 8 + b];
-  const int64_t P = slot[e * 64 + a * 8 + b];
+  for (int k = threadIdx.x; k < 576; k += kGalThreads) {
+    const int c = k >> 6, P = (k >> 3) & 7, Q = k & 7;
+    const int64_t nP = conn_c[ec * 8 + bits_node(P)], nQ = conn_c[ec * 8 + bits_node(Q)];
+    double v = 0.0;
 #pragma unroll
-  for (int r = 0; r < 3; ++r)
+    for (int h = 0; h < 8; ++h) v += out[h * 576 + k];
+    ke_c[ec * 576 + k] = (fixed_c[3 * nP + c / 3] || fixed_c[3 * nQ + c % 3]) ? 0.0 : v;
+  }
+}
+
+// Block rows of a coarse level from its element matrices, 16 rows per CTA and 8
+// lanes per row, each entry summed in ascending element order and written once
+// (see k_assemble_rows).
+constexpr int kMgRows = 16;
+constexpr int kMgRowThreads = 128;
+
+__global__ void __launch_bounds__(kMgRowThreads)
+    k_mg_rows(int32_t N, const int32_t* __restrict__ nptr, const int32_t* __restrict__ nelem,
+              const double* __restrict__ ke, const int32_t* __restrict__ slot, const int64_t* __restrict__ sptr,
+              const int32_t* __restrict__ scol, const int32_t* __restrict__ dpos, const uint8_t* __restrict__ fixed,
+              int stride, double* __restrict__ val, double* __restrict__ dinv, float* __restrict__ val_r,
+              float* __restrict__ dinv_r) {
+  extern __shared__ double mg_acc[];  // [row][stride]
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 7;
+  const int64_t s = blockIdx.x >> 1;
+  const int half = (blockIdx.x & 1) * kMgRows;
+  const int64_t base = sptr[s];
+  const int len = (int)((sptr[s + 1] - base) >> 5);
+  RowWriter<double, kMgRows, kMgRowThreads> out;
+  out.init(N, s, half, base, len, scol, dpos, fixed);
+  for (int k = threadIdx.x; k < kMgRows * stride; k += kMgRowThreads) mg_acc[k] = 0.0;
+  __syncthreads();
+  const int r = 4 * w + (lane >> 3);
+  const int64_t row = s * kSlice + half + r;
+  const int32_t kb = row < N ? nptr[row] : 0, ke_end = row < N ? nptr[row + 1] : 0;
+  const int kmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)(ke_end - kb));
+#pragma unroll 2
+  for (int k = 0; k < kmax; ++k) {
+    if (kb + k < ke_end) {
+      const int32_t el = nelem[kb + k];
+      const int64_t e = el >> 3;
+      const int a = el & 7;
+      const int j = (int)((slot[e * 64 + a * 8 + bits_node(t)] - base) >> 5);
+      const double* src = ke + e * 576 + bits_node(a) * 8 + t;
+      double* d = mg_acc + r * stride + 9 * j;
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-      if (!fixed[3 * na + r] && !fixed[3 * nb + c]) val[vpos(P, r * 3 + c)] += ke[e * 576 + (3 * a + r) * 24 + 3 * b + c];
+      for (int c = 0; c < 9; ++c) d[c] += src[64 * c];
+    }
+    __syncwarp();  // the lanes of a row meet again at the same entries
+  }
+  __syncthreads();
+  out.write(len, scol, fixed, mg_acc, stride, val, dinv, val_r, dinv_r);
 }
 
-__global__ void k_mg_fix_diag(int32_t nfix, const int32_t* __restrict__ dofs, const int32_t* __restrict__ dpos,
-                              double* __restrict__ val) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nfix) val[vpos(dpos[dofs[i] / 3], (dofs[i] % 3) * 4)] = 1.0;
-}
-
-__global__ void k_mg_dinv(int32_t N, const int32_t* __restrict__ dpos, const double* __restrict__ val,
-                          double* __restrict__ dinv) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 3 * (int64_t)N) return;
-  const double d = val[vpos(dpos[i / 3], (int)(i % 3) * 4)];
-  dinv[i] = fabs(d) > 1e-30 ? 1.0 / d : 1.0;
-}
-
-// r_c = P^T r_f: one thread per coarse node gathers the fine nodes within one
-// fine spacing of it, weight prod_d (1 or 1/2).
+// b = P^T r_f and d = D^-1 b / theta (the coarse smoother's first step): one
+// thread per coarse node gathers the fine nodes within one fine spacing of it,
+// weight prod_d (1 or 1/2).  dinv null: no smoother on the coarse level.
 template <typename T>
 __global__ void k_mg_restrict(int32_t nxc, int32_t nyc, int32_t nzc, const T* __restrict__ rf,
                               const uint8_t* __restrict__ fixed_f, const uint8_t* __restrict__ fixed_c,
-                              T* __restrict__ rc, const CgScalars* __restrict__ scal) {
-  if (scal && scal->stop) return;
+                              const T* __restrict__ dinv, const double* __restrict__ coef, T* __restrict__ bc,
+                              T* __restrict__ dc, const CgScalars* __restrict__ scal) {
   const int64_t nc = (int64_t)(nxc + 1) * (nyc + 1) * (nzc + 1);
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nc) return;
   const int nxf = 2 * nxc, nyf = 2 * nyc, nzf = 2 * nzc;
-  const int64_t I = v % (nxc + 1), J = (v / (nxc + 1)) % (nyc + 1), K = v / ((int64_t)(nxc + 1) * (nyc + 1));
+  const int32_t I = (int32_t)(v % (nxc + 1)), J = (int32_t)((v / (nxc + 1)) % (nyc + 1)),
+                K = (int32_t)(v / ((int64_t)(nxc + 1) * (nyc + 1)));
+  pdl_enter();
+  if (v >= nc || (scal && scal->stop)) return;
   T s[3] = {T(0), T(0), T(0)};
-  for (int dk = -1; dk <= 1; ++dk) {
-    const int64_t k = 2 * K + dk;
-    if (k < 0 || k > nzf) continue;
-    for (int dj = -1; dj <= 1; ++dj) {
-      const int64_t j = 2 * J + dj;
-      if (j < 0 || j > nyf) continue;
+#pragma unroll
+  for (int dk = -1; dk <= 1; ++dk)
+#pragma unroll
+    for (int dj = -1; dj <= 1; ++dj)
+#pragma unroll
       for (int di = -1; di <= 1; ++di) {
-        const int64_t i = 2 * I + di;
-        if (i < 0 || i > nxf) continue;
+        const int k = 2 * K + dk, j = 2 * J + dj, i = 2 * I + di;
+        if (k < 0 || k > nzf || j < 0 || j > nyf || i < 0 || i > nxf) continue;
         const T w = T((di ? 0.5 : 1.0) * (dj ? 0.5 : 1.0) * (dk ? 0.5 : 1.0));
         const int64_t f = box_node(i, j, k, nxf, nyf);
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
-          if (!fixed_f[3 * f + d]) s[d] += w * rf[3 * f + d];
+        for (int d = 0; d < 3; ++d) s[d] += fixed_f[3 * f + d] ? T(0) : w * rf[3 * f + d];
       }
-    }
-  }
+  const T it = dinv ? (T)coef[1] : T(0);
 #pragma unroll
-  for (int d = 0; d < 3; ++d) rc[3 * v + d] = fixed_c[3 * v + d] ? T(0) : s[d];
+  for (int d = 0; d < 3; ++d) {
+    const T b = fixed_c[3 * v + d] ? T(0) : s[d];
+    bc[3 * v + d] = b;
+    if (dinv) dc[3 * v + d] = dinv[3 * v + d] * b * it;
+  }
 }
 
-// x_f += P x_c: one thread per fine node gathers its 1, 2, 4 or 8 coarse parents.
+// v = P x_c: one thread per fine node gathers its 1, 2, 4 or 8 coarse parents.
 template <typename T>
-__global__ void k_mg_prolong_add(int32_t nxc, int32_t nyc, int32_t nzc, const T* __restrict__ xc,
-                                 const uint8_t* __restrict__ fixed_f, const uint8_t* __restrict__ fixed_c,
-                                 T* __restrict__ xf, const CgScalars* __restrict__ scal) {
-  if (scal && scal->stop) return;
+__global__ void k_mg_prolong(int32_t nxc, int32_t nyc, int32_t nzc, const T* __restrict__ xc,
+                             const uint8_t* __restrict__ fixed_f, const uint8_t* __restrict__ fixed_c,
+                             T* __restrict__ vf, const CgScalars* __restrict__ scal) {
   const int nxf = 2 * nxc, nyf = 2 * nyc, nzf = 2 * nzc;
   const int64_t nf = (int64_t)(nxf + 1) * (nyf + 1) * (nzf + 1);
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nf) return;
-  const int64_t i = v % (nxf + 1), j = (v / (nxf + 1)) % (nyf + 1), k = v / ((int64_t)(nxf + 1) * (nyf + 1));
-  const int64_t i0 = i >> 1, j0 = j >> 1, k0 = k >> 1;
-  const int ni = (i & 1) ? 2 : 1, nj = (j & 1) ? 2 : 1, nk = (k & 1) ? 2 : 1;
-  const T w = T((ni == 2 ? 0.5 : 1.0) * (nj == 2 ? 0.5 : 1.0) * (nk == 2 ? 0.5 : 1.0));
+  const int32_t i = (int32_t)(v % (nxf + 1)), j = (int32_t)((v / (nxf + 1)) % (nyf + 1)),
+                k = (int32_t)(v / ((int64_t)(nxf + 1) * (nyf + 1)));
+  pdl_enter();
+  if (v >= nf || (scal && scal->stop)) return;
+  const T w = T(((i & 1) ? 0.5 : 1.0) * ((j & 1) ? 0.5 : 1.0) * ((k & 1) ? 0.5 : 1.0));
   T s[3] = {T(0), T(0), T(0)};
-  for (int c = 0; c < nk; ++c)
-    for (int b = 0; b < nj; ++b)
-      for (int a = 0; a < ni; ++a) {
-        const int64_t cn = box_node(i0 + a, j0 + b, k0 + c, nxc, nyc);
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
-          if (!fixed_c[3 * cn + d]) s[d] += w * xc[3 * cn + d];
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        if ((c && !(k & 1)) || (b && !(j & 1)) || (a && !(i & 1))) continue;
+        const int64_t cn = box_node((i >> 1) + a, (j >> 1) + b, (k >> 1) + c, nxc, nyc);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) s[d] += fixed_c[3 * cn + d] ? T(0) : w * xc[3 * cn + d];
       }
 #pragma unroll
-  for (int d = 0; d < 3; ++d)
-    if (!fixed_f[3 * v + d]) xf[3 * v + d] += s[d];
+  for (int d = 0; d < 3; ++d) vf[3 * v + d] = fixed_f[3 * v + d] ? T(0) : s[d];
 }
 
-// Chebyshev smoother (three-term recurrence of Saad, Iterative Methods for
-// Sparse Linear Systems, Alg. 12.1, with the Jacobi preconditioner).
-// Start: r = b - w (w = A x, or zero when x starts at zero), d = D^-1 r / theta,
-// x (+)= d.
+// The Chebyshev smoother (three-term recurrence of Saad, Iterative Methods for
+// Sparse Linear Systems, Alg. 12.1, with the Jacobi preconditioner) as the
+// epilogue of the products it is made of: with w = (A v)_row for the gathered
+// vector v,
+//   kStep   v = d: r = rin - w, d' = c1 d + c2 D^-1 r, x = xin + d'
+//   kResid  v = d: r = rin - w (the residual after the last step)
+//   kStart  v = the prolonged coarse correction: r = rin - w,
+//           d' = D^-1 r / theta, x = xin + v + d'
+//   kPower  d' = D^-1 w and ||d'||^2 (the power iteration of set-up)
+// One launch then does a product and its vector updates, and the vectors of a
+// step are read once.  d' goes to another buffer than d, which other rows still
+// gather.  The last step of a cycle writes z in FP64 and the row's part of r.z.
+enum MgMode { kStep, kResid, kStart, kPower };
+
 template <typename T>
-__global__ void k_cheb_start(int64_t n, const T* __restrict__ b, const T* __restrict__ w,
-                             const T* __restrict__ dinv, T inv_theta, int x_zero, T* __restrict__ x,
-                             T* __restrict__ r, T* __restrict__ d, const CgScalars* __restrict__ scal) {
-  if (scal && scal->stop) return;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const T ri = b[i] - (x_zero ? T(0) : w[i]);
-    const T di = dinv[i] * ri * inv_theta;
-    r[i] = ri;
-    d[i] = di;
-    x[i] = x_zero ? di : x[i] + di;
+struct MgEpi {
+  static constexpr bool kDot = true, kPdl = true;
+  int mode = kStep, step = 0;
+  bool dot = false;
+  const CgScalars* scal = nullptr;
+  const double* coef = nullptr;
+  const T *rin = nullptr, *dinv = nullptr, *xin = nullptr;
+  T *rout = nullptr, *dout = nullptr, *xout = nullptr;
+  double* z = nullptr;
+  const double* r64 = nullptr;
+  __device__ __forceinline__ bool halt() const { return scal && scal->stop; }
+  __device__ __forceinline__ bool want_dot() const { return dot; }
+  __device__ __forceinline__ double operator()(int64_t row, T a0, T a1, T a2, const T* __restrict__ v) const {
+    const T w[3] = {a0, a1, a2};
+    double part = 0.0;
+    const T c1 = mode == kStep ? (T)coef[2 * step] : mode == kStart ? (T)coef[1] : T(0);
+    const T c2 = mode == kStep ? (T)coef[2 * step + 1] : T(0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int64_t i = 3 * row + c;
+      if (mode == kPower) {
+        const T dn = dinv[i] * w[c];
+        dout[i] = dn;
+        part += (double)dn * (double)dn;
+        continue;
+      }
+      const T ri = rin[i] - w[c];
+      if (rout) rout[i] = ri;
+      if (mode == kResid) continue;
+      const T vi = v[i];
+      const T dn = mode == kStep ? c1 * vi + c2 * dinv[i] * ri : dinv[i] * ri * c1;
+      const T xn = (mode == kStep ? xin[i] : xin[i] + vi) + dn;
+      if (dout) dout[i] = dn;
+      if (xout) xout[i] = xn;
+      if (z) z[i] = (double)xn;
+      if (dot) part += r64[i] * (double)xn;
+    }
+    return part;
   }
-}
+};
 
-// Step: r -= w (w = A d), d = c1 d + c2 D^-1 r, x += d.
+// x = Inv b (dense, coarsest level, leading dimension ld), one warp per row.
 template <typename T>
-__global__ void k_cheb_step(int64_t n, const T* __restrict__ w, const T* __restrict__ dinv, T c1, T c2,
-                            T* __restrict__ x, T* __restrict__ r, T* __restrict__ d,
-                            const CgScalars* __restrict__ scal) {
-  if (scal && scal->stop) return;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const T ri = r[i] - w[i];
-    const T di = c1 * d[i] + c2 * dinv[i] * ri;
-    r[i] = ri;
-    d[i] = di;
-    x[i] += di;
-  }
-}
-
-// out = b - w
-template <typename T>
-__global__ void k_mg_sub(int64_t n, const T* __restrict__ b, const T* __restrict__ w, T* __restrict__ out,
-                         const CgScalars* __restrict__ scal) {
-  if (scal && scal->stop) return;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = b[i] - w[i];
-}
-
-// x = Inv b (dense, coarsest level), one warp per row.
-template <typename T>
-__global__ void k_mg_dense(int64_t n, const T* __restrict__ inv, const T* __restrict__ b, T* __restrict__ x,
-                           const CgScalars* __restrict__ scal) {
+__global__ void k_mg_dense(int64_t n, int64_t ld, const T* __restrict__ inv, const T* __restrict__ b,
+                           T* __restrict__ x, const CgScalars* __restrict__ scal) {
+  pdl_enter();
   if (scal && scal->stop) return;
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= n) return;
   T s = T(0);
-  for (int64_t j = lane; j < n; j += 32) s += inv[row * n + j] * b[j];
+#pragma unroll 4
+  for (int64_t j = lane; j < n; j += 32) s += inv[row * ld + j] * b[j];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if (lane == 0) x[row] = s;
 }
 
-template <typename A, typename B>
-__global__ void k_mg_convert(int64_t n, const A* __restrict__ a, B* __restrict__ b, const CgScalars* __restrict__ scal) {
-  if (scal && scal->stop) return;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    b[i] = (B)a[i];
+// The first smoothing step of the finest level, from the PCG's residual:
+// b = r in the cycle's precision (when it is not r itself), d = D^-1 b / theta.
+template <typename T>
+__device__ __forceinline__ void mg_begin(int64_t i, double r, T* __restrict__ b, T* __restrict__ d,
+                                         const T* __restrict__ dinv, T it) {
+  const T bi = (T)r;
+  if (sizeof(T) == 4) b[i] = bi;
+  d[i] = dinv[i] * bi * it;
 }
 
-// ||v||^2 into *out (power iteration at set-up).
-__global__ void k_mg_norm2(int64_t n, const double* __restrict__ v, double* __restrict__ partials,
-                           uint32_t* ticket, double* __restrict__ out) {
-  double a[1] = {0.0};
+template <typename T>
+__global__ void __launch_bounds__(kBlk)
+    k_mg_begin(int64_t n, const double* __restrict__ r, T* __restrict__ b, T* __restrict__ d,
+               const T* __restrict__ dinv, const double* __restrict__ coef) {
+  const T it = (T)coef[1];
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    a[0] += v[i] * v[i];
+    mg_begin<T>(i, r[i], b, d, dinv, it);
+}
+
+// Sum of the power iteration's partials.
+__global__ void __launch_bounds__(kBlk) k_mg_sum(const double* __restrict__ partials, int nb, double* __restrict__ out) {
   double tot[1];
-  if (grid_sum<1>(a, partials, ticket, tot)) *out = tot[0];
+  sum_partials<1>(partials, nb, tot);
+  if (threadIdx.x == 0) *out = tot[0];
 }
 
-// v = D^-1 w / ||v_prev|| with ||v_prev||^2 read from the device (0: v = 0)
-__global__ void k_mg_scale_dinv(int64_t n, const double* __restrict__ w, const double* __restrict__ dinv,
-                                const double* __restrict__ nrm2, double* __restrict__ v) {
-  const double q = *nrm2;
-  const double s = q > 0.0 ? 1.0 / sqrt(q) : 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    v[i] = dinv[i] * w[i] * s;
+// The smoother's interval [1.1 lambda_max / ratio, 1.1 lambda_max] and the
+// coefficients of m steps.  nb > 0: lambda_max = ||v_k|| / ||v_{k-1}|| of the
+// power iteration (partials of ||v_k||^2 and *prev = ||v_{k-1}||^2); nb = 0: the
+// stored one, times scale.
+__global__ void __launch_bounds__(kBlk)
+    k_mg_coef(const double* __restrict__ partials, int nb, const double* __restrict__ prev, double scale, double ratio,
+              int m, double* __restrict__ coef) {
+  double tot[1] = {0.0};
+  if (nb > 0) sum_partials<1>(partials, nb, tot);
+  if (threadIdx.x != 0) return;
+  const double lambda = nb > 0 ? (*prev > 0.0 ? sqrt(tot[0] / *prev) : 0.0) : coef[0] * scale;
+  coef[0] = lambda;
+  const double lmax = 1.1 * lambda, lmin = lmax / ratio;
+  const double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin);
+  const double sigma = theta / delta;
+  coef[1] = 1.0 / theta;
+  double rho = 1.0 / sigma;
+  for (int k = 1; k < m; ++k) {
+    const double rho_new = 1.0 / (2.0 * sigma - rho);
+    coef[2 * k] = rho_new * rho;
+    coef[2 * k + 1] = 2.0 * rho_new / delta;
+    rho = rho_new;
+  }
 }
 
 __global__ void k_mg_start_vector(int64_t n, const uint8_t* __restrict__ fixed, double* __restrict__ v) {
@@ -403,21 +560,38 @@ __global__ void k_mg_start_vector(int64_t n, const uint8_t* __restrict__ fixed, 
 
 // ---- the PCG around the V-cycle: the Jacobi kernels' recurrence with z = M r
 
-// x += alpha p, r -= alpha q, ||r||^2, the stop tests.
+// alpha = r.z / p.q (from the product's partials), x += alpha p, r -= alpha q,
+// the next cycle's first smoothing step, ||r||^2 and the stop tests.
+template <typename T>
 __global__ void __launch_bounds__(kBlk)
     k_mgcg_update(int64_t n, const double* __restrict__ p, const double* __restrict__ q, double* __restrict__ r,
-                  double* __restrict__ x, CgScalars* __restrict__ scal, double* __restrict__ partials) {
+                  double* __restrict__ x, T* __restrict__ b, T* __restrict__ d, const T* __restrict__ dinv,
+                  const double* __restrict__ coef, CgScalars* __restrict__ scal,
+                  const double* __restrict__ pq_partials, int nb, double* __restrict__ partials) {
+  pdl_enter();
   if (scal->stop) return;
-  const double a = scal->alpha;
+  double pq[1];
+  sum_partials<1>(pq_partials, nb, pq);
+  if (!(fabs(pq[0]) > 1e-300) || !isfinite(pq[0])) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) scal->stop = 3;
+    return;
+  }
+  const double a = scal->rz / pq[0];
+  const T it0 = (T)coef[1];
   double v[1] = {0.0};
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     x[i] += a * p[i];
     const double ri = r[i] - a * q[i];
     r[i] = ri;
+    mg_begin<T>(i, ri, b, d, dinv, it0);
     v[0] += ri * ri;
   }
   double tot[1];
   if (grid_sum<1>(v, partials, &scal->ticket[1], tot)) {
+    scal->pq = pq[0];
+    scal->alpha = a;
+    scal->rz_old = scal->rz;
+    scal->fresh = 0;
     scal->rr = tot[0];
     const int it = scal->iter + 1;
     scal->iter = it;
@@ -428,32 +602,104 @@ __global__ void __launch_bounds__(kBlk)
   }
 }
 
-// r.z, beta = r.z / r.z_old (first call: beta = 0).
+// r.z from the cycle's partials, beta = r.z / r.z_old, p = z + beta p (beta = 0
+// after a (re)start: p = z without reading p, which may hold anything).  Every
+// block takes the same sum; block 0 records it.
 __global__ void __launch_bounds__(kBlk)
-    k_mgcg_rz(int64_t n, const double* __restrict__ r, const double* __restrict__ z, CgScalars* __restrict__ scal,
-              double* __restrict__ partials, int first) {
+    k_mgcg_pupdate(int64_t n, const double* __restrict__ z, double* __restrict__ p, CgScalars* __restrict__ scal,
+                   const double* __restrict__ partials, int nb) {
+  pdl_enter();
   if (scal->stop) return;
-  double v[1] = {0.0};
+  double rz[1];
+  sum_partials<1>(partials, nb, rz);
+  const bool fresh = scal->fresh != 0, bad = !isfinite(rz[0]) || !(rz[0] > 0.0);  // M must stay positive definite
+  const double b = fresh ? 0.0 : rz[0] / scal->rz_old;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    scal->beta = b;
+    scal->rz = rz[0];
+    if (bad) scal->stop = 3;
+  }
+  if (bad) return;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    v[0] += r[i] * z[i];
-  double tot[1];
-  if (grid_sum<1>(v, partials, &scal->ticket[2], tot)) {
-    const double old = scal->rz;
-    scal->beta = first ? 0.0 : tot[0] / old;
-    scal->rz_old = old;
-    scal->rz = tot[0];
-    if (!isfinite(tot[0]) || !(tot[0] > 0.0)) scal->stop = 3;  // M must stay positive definite
+    p[i] = fresh ? z[i] : z[i] + b * p[i];
+}
+
+// ---- coarsest inverse: block Gauss-Jordan in place, blocks of 32, without
+// pivoting (the matrix is symmetric positive definite); a pivot that is not
+// positive sets *flag, and the host elimination with pivoting takes over.
+constexpr int kGj = 32;
+
+// The matrix of a level as a dense array, padded with the identity.
+__global__ void k_gj_fill(int32_t N, int64_t n, int64_t ld, const int32_t* __restrict__ brow,
+                          const int32_t* __restrict__ bcol, const int64_t* __restrict__ sptr,
+                          const double* __restrict__ val, double* __restrict__ M) {
+  const int64_t row = blockIdx.x;
+  for (int64_t j = threadIdx.x; j < ld; j += blockDim.x) M[row * ld + j] = (row >= n && j == row) ? 1.0 : 0.0;
+  __syncthreads();
+  if (row >= n) return;
+  const int64_t i = row / 3;
+  const int r = (int)(row % 3);
+  const int64_t s = i >> 5, b = brow[i], m = brow[i + 1] - b;
+  for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
+    const int64_t P = sptr[s] + k * kSlice + (i & 31), col = bcol[b + k];
+    for (int c = 0; c < 3; ++c) M[row * ld + 3 * col + c] = val[vpos(P, 3 * r + c)];
   }
 }
 
-// p = z + beta p
-__global__ void k_mgcg_pupdate(int64_t n, const double* __restrict__ z, double* __restrict__ p,
-                               const CgScalars* __restrict__ scal) {
-  if (scal->stop) return;
-  const double b = scal->beta;
-  // beta = 0 (start, restart): p = z without reading p, which may hold anything
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = b == 0.0 ? z[i] : z[i] + b * p[i];
+// Step k, first half: the inverse of the pivot block (every CTA forms it), block
+// column j of the pivot row multiplied by it, and the old pivot column block of
+// row j kept in C.
+__global__ void __launch_bounds__(kGj* kGj)
+    k_gj_panel(int64_t ld, int k, double* __restrict__ M, double* __restrict__ C, double* __restrict__ Pinv,
+               int32_t* __restrict__ flag) {
+  __shared__ double D[kGj][kGj + 1], A[kGj][kGj + 1];
+  const int r = threadIdx.x / kGj, c = threadIdx.x % kGj, j = blockIdx.x;
+  const int64_t k0 = (int64_t)k * kGj, j0 = (int64_t)j * kGj;
+  D[r][c] = M[(k0 + r) * ld + k0 + c];
+  A[r][c] = M[(k0 + r) * ld + j0 + c];
+  C[(j0 + r) * kGj + c] = M[(j0 + r) * ld + k0 + c];
+  __syncthreads();
+  for (int s = 0; s < kGj; ++s) {
+    const double piv = D[s][s];
+    if (!(piv > 0.0) && threadIdx.x == 0) *flag = 1;
+    const double ip = 1.0 / piv, row = D[s][c], col = D[r][s], own = D[r][c];
+    __syncthreads();
+    if (r == s)
+      D[r][c] = c == s ? ip : row * ip;
+    else
+      D[r][c] = c == s ? -col * ip : own - col * (row * ip);
+    __syncthreads();
+  }
+  if (j == k) {
+    Pinv[r * kGj + c] = D[r][c];
+    return;
+  }
+  double v = 0.0;
+#pragma unroll
+  for (int s = 0; s < kGj; ++s) v += D[r][s] * A[s][c];
+  M[(k0 + r) * ld + j0 + c] = v;
+}
+
+// Second half: every block of the other rows, minus the old pivot column times
+// the new pivot row; the pivot column becomes -C Pinv, the pivot block Pinv.
+__global__ void __launch_bounds__(kGj* kGj)
+    k_gj_update(int64_t ld, int k, double* __restrict__ M, const double* __restrict__ C,
+                const double* __restrict__ Pinv) {
+  __shared__ double A[kGj][kGj + 1], B[kGj][kGj + 1];
+  const int r = threadIdx.x / kGj, c = threadIdx.x % kGj, i = blockIdx.y, j = blockIdx.x;
+  const int64_t k0 = (int64_t)k * kGj, i0 = (int64_t)i * kGj, j0 = (int64_t)j * kGj;
+  if (i == k) {
+    if (j == k) M[(k0 + r) * ld + k0 + c] = Pinv[r * kGj + c];
+    return;
+  }
+  A[r][c] = C[(i0 + r) * kGj + c];
+  B[r][c] = j == k ? Pinv[r * kGj + c] : M[(k0 + r) * ld + j0 + c];
+  __syncthreads();
+  double v = 0.0;
+#pragma unroll
+  for (int s = 0; s < kGj; ++s) v += A[r][s] * B[s][c];
+  const int64_t at = (i0 + r) * ld + j0 + c;
+  M[at] = j == k ? -v : M[at] - v;
 }
 
 // ---------------------------------------------------------------- host side
@@ -468,34 +714,92 @@ __global__ void k_mg_round(int64_t n, const double* __restrict__ a, float* __res
     b[i] = (float)a[i];
 }
 
-// lambda_max of D^-1 A on level L by power iteration (deterministic start), in
-// FP64: v <- D^-1 A v / ||v||, lambda = ||v|| after the last step.  The norms
-// stay on the device, so the iterations run without a host round trip; the
-// vectors are kept for the next refresh.
-int estimate_lmax(Ctx* owner, Mg& mg, MgLevel& L, int iters) {
+// The symmetric storage rounded to FP32, step by step (the layouts differ).
+__global__ void k_mg_round_sym(int64_t nblocks, const double* __restrict__ a, float* __restrict__ b) {
+  for (int64_t P = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; P < nblocks; P += (int64_t)gridDim.x * blockDim.x)
+#pragma unroll
+    for (int c = 0; c < 9; ++c) b[spos<float>(P, c)] = (float)a[spos<double>(P, c)];
+}
+
+// A level's product in the cycle's precision: the symmetric storage where the
+// level holds it (the finest level of a model assembled with
+// UFC_BUILD_SYMMETRIC), else the full SELL storage.  Returns the number of
+// partial sums.
+int lv_product(const MgLevel& L, cudaStream_t st, const double* x, const MgEpi<double>& epi) {
+  const Ctx* lc = L.c;
+  if (lc->has_sval64) return launch_spmv_sym<double, double, double>(lc, st, lc->sval64, x, epi);
+  return launch_spmv_diff<double, double, double, false>(lc, st, lc->val64, x, epi);
+}
+int lv_product(const MgLevel& L, cudaStream_t st, const float* x, const MgEpi<float>& epi) {
+  const Ctx* lc = L.c;
+  if (L.sval32) return launch_spmv_sym<float, float, float>(lc, st, L.sval32, x, epi);
+  return launch_spmv_diff<float, float, float, false>(lc, st, L.val32, x, epi);
+}
+
+// Degree of the smoother (or of the Chebyshev solve) on level l.
+int lv_degree(const Mg& mg, size_t l) { return l + 1 == mg.lv.size() ? mg.cheb_coarse : mg.degree; }
+double lv_ratio(const Mg& mg, size_t l) { return l + 1 == mg.lv.size() ? 1000.0 : mg.ratio; }
+
+// lambda_max of D^-1 A on level L by 15 steps of the power iteration v <- D^-1 A v
+// (deterministic start, FP64), lambda = ||v_15|| / ||v_14||, and the smoother's
+// coefficients from it; everything stays on the device.
+int estimate_lmax(Ctx* owner, Mg& mg, size_t l) {
+  constexpr int kIters = 15;
+  MgLevel& L = mg.lv[l];
   Ctx* lc = L.c;
   const int64_t n = lc->n;
-  const int g = grid_n(n);
+  const int m = lv_degree(mg, l);
   if (!L.pv) UFC_TRY(dalloc(owner, &L.pv, n));
   if (!L.pw) UFC_TRY(dalloc(owner, &L.pw, n));
+  if (!L.coef) UFC_TRY(dalloc(owner, &L.coef, 2 * (int64_t)std::max(m, 1) + 2));
   if (!mg.dnorm) UFC_TRY(dalloc(owner, &mg.dnorm, 1));
-  k_mg_start_vector<<<g, kBlk, 0, owner->stream>>>(n, lc->fixed, L.pv);
-  k_mg_norm2<<<g, kBlk, 0, owner->stream>>>(n, L.pv, owner->partials, &owner->scal->ticket[6], mg.dnorm);
-  for (int it = 0; it < iters; ++it) {
-    spmv64_on(lc, owner->stream, L.pv, L.pw);
-    k_mg_scale_dinv<<<g, kBlk, 0, owner->stream>>>(n, L.pw, lc->dinv64, mg.dnorm, L.pv);
-    k_mg_norm2<<<g, kBlk, 0, owner->stream>>>(n, L.pv, owner->partials, &owner->scal->ticket[6], mg.dnorm);
+  k_mg_start_vector<<<grid_n(n), kBlk, 0, owner->stream>>>(n, lc->fixed, L.pv);
+  double *v = L.pv, *w = L.pw;
+  int nb = 0;
+  for (int it = 1; it <= kIters; ++it) {
+    MgEpi<double> epi;
+    epi.mode = kPower;
+    epi.dinv = lc->dinv64;
+    epi.dout = w;
+    epi.dot = it + 1 >= kIters;
+    nb = lv_product(L, owner->stream, v, epi);
+    if (it + 1 == kIters) k_mg_sum<<<1, kBlk, 0, owner->stream>>>(lc->partials, nb, mg.dnorm);
+    std::swap(v, w);
   }
+  k_mg_coef<<<1, kBlk, 0, owner->stream>>>(lc->partials, nb, mg.dnorm, 1.0, lv_ratio(mg, l), m, L.coef);
   UFC_CUDA(owner, cudaGetLastError());
-  double q = 0.0;
-  UFC_CUDA(owner, cudaMemcpyAsync(&q, mg.dnorm, sizeof(double), cudaMemcpyDeviceToHost, owner->stream));
-  UFC_CUDA(owner, cudaStreamSynchronize(owner->stream));
-  L.lmax = iters > 0 ? std::sqrt(q) : 0.0;
   return UFC_STATUS_OK;
 }
 
-// Dense inverse of the coarsest matrix (Gauss-Jordan with partial pivoting).
-int dense_inverse(Ctx* owner, MgLevel& L, bool fp32) {
+int64_t dense_ld(int64_t n) { return (n + kGj - 1) / kGj * kGj; }
+
+// The coarsest inverse on the device: enqueued only, *mg.gj_flag says whether it holds.
+int dense_inverse_device(Ctx* owner, Mg& mg, MgLevel& L) {
+  Ctx* lc = L.c;
+  const int64_t n = lc->n, ld = dense_ld(n);
+  const int nb = (int)(ld / kGj);
+  if (!L.inv) UFC_TRY(dalloc(owner, &L.inv, ld * ld));
+  if (!L.gj) UFC_TRY(dalloc(owner, &L.gj, ld * kGj + kGj * kGj));
+  if (!mg.gj_flag) UFC_TRY(dalloc(owner, &mg.gj_flag, 1));
+  double *C = L.gj, *Pinv = L.gj + ld * kGj;
+  UFC_CUDA(owner, cudaMemsetAsync(mg.gj_flag, 0, sizeof(int32_t), owner->stream));
+  k_gj_fill<<<(int)ld, 128, 0, owner->stream>>>(lc->N, n, ld, lc->brow, lc->bcol, lc->slice_ptr, lc->val64, L.inv);
+  for (int k = 0; k < nb; ++k) {
+    k_gj_panel<<<nb, kGj * kGj, 0, owner->stream>>>(ld, k, L.inv, C, Pinv, mg.gj_flag);
+    k_gj_update<<<dim3(nb, nb), kGj * kGj, 0, owner->stream>>>(ld, k, L.inv, C, Pinv);
+  }
+  if (mg.fp32) {
+    if (!L.inv32) UFC_TRY(dalloc(owner, &L.inv32, ld * ld));
+    k_mg_round<<<grid_n(ld * ld), kBlk, 0, owner->stream>>>(ld * ld, L.inv, L.inv32);
+  }
+  UFC_CUDA(owner, cudaGetLastError());
+  return UFC_STATUS_OK;
+}
+
+// Dense inverse of the coarsest matrix on the host (Gauss-Jordan with partial
+// pivoting), for matrices whose elimination on the device met a pivot that is
+// not positive.
+int dense_inverse_host(Ctx* owner, MgLevel& L, bool fp32) {
   Ctx* lc = L.c;
   const int64_t n = lc->n, nnz = 9 * lc->nnzb;
   std::vector<int64_t> rp(n + 1);
@@ -539,128 +843,163 @@ int dense_inverse(Ctx* owner, MgLevel& L, bool fp32) {
       }
     }
   }
-  if (fp32) {
-    std::vector<float> f(Inv.begin(), Inv.end());
-    if (!L.inv32) UFC_TRY(dalloc(owner, &L.inv32, n * n));  // same size at every refresh
-    UFC_CUDA(owner, cudaMemcpyAsync(L.inv32, f.data(), sizeof(float) * n * n, cudaMemcpyHostToDevice, owner->stream));
-    UFC_CUDA(owner, cudaStreamSynchronize(owner->stream));
-  } else {
-    if (!L.inv) UFC_TRY(dalloc(owner, &L.inv, n * n));
-    UFC_CUDA(owner, cudaMemcpyAsync(L.inv, Inv.data(), sizeof(double) * n * n, cudaMemcpyHostToDevice, owner->stream));
-    UFC_CUDA(owner, cudaStreamSynchronize(owner->stream));
-  }
+  const int64_t ld = dense_ld(n);
+  std::vector<double> out((size_t)ld * ld, 0.0);
+  for (int64_t i = 0; i < n; ++i) std::copy(Inv.begin() + i * n, Inv.begin() + (i + 1) * n, out.begin() + i * ld);
+  UFC_CUDA(owner, cudaMemcpyAsync(L.inv, out.data(), sizeof(double) * ld * ld, cudaMemcpyHostToDevice, owner->stream));
+  if (fp32) k_mg_round<<<grid_n(ld * ld), kBlk, 0, owner->stream>>>(ld * ld, L.inv, L.inv32);
+  UFC_CUDA(owner, cudaStreamSynchronize(owner->stream));
   return UFC_STATUS_OK;
 }
 
+template <typename T>
+void free_vecs(MgVecs<T>& v, bool own_xb) {
+  if (own_xb) {
+    dfree(&v.x);
+    dfree(&v.b);
+  }
+  dfree(&v.r);
+  dfree(&v.d);
+  dfree(&v.e);
+  dfree(&v.w);
+}
+
 void free_level(MgLevel& L) {
+  free_vecs(L.v64, L.own != nullptr);  // level 0: x and b are the caller's
+  free_vecs(L.v32, true);
   dfree(&L.ke);
-  dfree(&L.r);
-  dfree(&L.d);
-  dfree(&L.w);
-  dfree(&L.r32);
-  dfree(&L.d32);
-  dfree(&L.w32);
-  dfree(&L.x32);
-  dfree(&L.b32);
   dfree(&L.val32);
+  dfree(&L.sval32);
   dfree(&L.dinv32);
+  dfree(&L.coef);
   dfree(&L.inv);
   dfree(&L.inv32);
+  dfree(&L.gj);
   dfree(&L.pv);
   dfree(&L.pw);
-  if (L.own_xb) {
-    dfree(&L.x);
-    dfree(&L.b);
-  }
   if (L.own) ufc_ctx_destroy(L.own);
   L.own = nullptr;
 }
 
-// The vectors, values and diagonal of a level in the cycle's precision.
+// The vectors, diagonal and coarsest inverse of a level in the cycle's precision.
+MgVecs<double>& vecs_of(MgLevel& L, double*) { return L.v64; }
+MgVecs<float>& vecs_of(MgLevel& L, float*) { return L.v32; }
+const double* dinv_of(const MgLevel& L, double*) { return L.c->dinv64; }
+const float* dinv_of(const MgLevel& L, float*) { return L.dinv32; }
+const double* inv_of(const MgLevel& L, double*) { return L.inv; }
+const float* inv_of(const MgLevel& L, float*) { return L.inv32; }
+
+// One V-cycle from level l, whose b and first step d = D^-1 b / theta are in
+// place.  The result goes to x; on the finest level to z (FP64) with the
+// partials of r.z left for the caller: returns their number.
 template <typename T>
-struct View {
-  T *x, *b, *r, *d, *w;
-  const T *val, *dinv, *inv;
-};
-
-View<double> view(MgLevel& L, double*) { return {L.x, L.b, L.r, L.d, L.w, L.c->val64, L.c->dinv64, L.inv}; }
-View<float> view(MgLevel& L, float*) { return {L.x32, L.b32, L.r32, L.d32, L.w32, L.val32, L.dinv32, L.inv32}; }
-
-void spmv_lv(const Ctx* lc, cudaStream_t st, const double* val, const double* x, double* y) {
-  (void)val;
-  spmv64_on(lc, st, x, y);
-}
-void spmv_lv(const Ctx* lc, cudaStream_t st, const float* val, const float* x, float* y) {
-  spmv32_on(lc, st, val, x, y);
-}
-
-// Chebyshev smoothing of A x = b on level L (m steps).
-template <typename T>
-void cheb(Ctx* owner, MgLevel& L, int m, double ratio, bool x_zero, const CgScalars* scal) {
-  Ctx* lc = L.c;
-  const View<T> V = view(L, (T*)nullptr);
-  const int64_t n = lc->n;
-  const int g = grid_n(n);
-  const double lmax = 1.1 * L.lmax, lmin = lmax / ratio;
-  const double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin);
-  const double sigma = theta / delta;
-  if (!x_zero) spmv_lv(lc, owner->stream, V.val, V.x, V.w);
-  k_cheb_start<T><<<g, kBlk, 0, owner->stream>>>(n, V.b, V.w, V.dinv, (T)(1.0 / theta), x_zero ? 1 : 0, V.x, V.r,
-                                                 V.d, scal);
-  double rho = 1.0 / sigma;
-  for (int k = 1; k < m; ++k) {
-    spmv_lv(lc, owner->stream, V.val, V.d, V.w);
-    const double rho_new = 1.0 / (2.0 * sigma - rho);
-    k_cheb_step<T><<<g, kBlk, 0, owner->stream>>>(n, V.w, V.dinv, (T)(rho_new * rho), (T)(2.0 * rho_new / delta),
-                                                  V.x, V.r, V.d, scal);
-    rho = rho_new;
-  }
-  owner->launches += 2 * m - (x_zero ? 1 : 0);
-}
-
-// One V-cycle from level l: x ~ A_l^-1 b.
-template <typename T>
-void vcycle(Ctx* owner, Mg& mg, size_t l, const CgScalars* scal) {
+int vcycle(Ctx* owner, Mg& mg, size_t l, const CgScalars* scal, double* z, const double* r64) {
   MgLevel& L = mg.lv[l];
   Ctx* lc = L.c;
-  const View<T> V = view(L, (T*)nullptr);
-  if (l + 1 == mg.lv.size()) {
-    if (V.inv) {
-      k_mg_dense<T><<<(int)((lc->n * 32 + kBlk - 1) / kBlk), kBlk, 0, owner->stream>>>(lc->n, V.inv, V.b, V.x, scal);
-      owner->launches += 1;
-    } else {
-      cheb<T>(owner, L, mg.cheb_coarse, 1000.0, true, scal);
+  cudaStream_t st = owner->stream;
+  MgVecs<T>& V = vecs_of(L, (T*)nullptr);
+  const T* dinv = dinv_of(L, (T*)nullptr);
+  const bool last = l + 1 == mg.lv.size();
+  if (last && !mg.cheb_coarse) {
+    const int grid = (int)((lc->n * 32 + kBlk - 1) / kBlk);
+    launch_pdl(k_mg_dense<T>, grid, kBlk, st, lc->n, dense_ld(lc->n), inv_of(L, (T*)nullptr), (const T*)V.b, V.x, scal);
+    owner->launches += 1;
+    return 0;
+  }
+  const int m = lv_degree(mg, l);
+  MgEpi<T> e0;
+  e0.scal = scal;
+  e0.coef = L.coef;
+  e0.dinv = dinv;
+  // x = d, then m - 1 steps; `d` is gathered, the new one goes to the other buffer
+  const T *rc = V.b, *xc = V.d;
+  T *d = V.d, *dn = V.e;
+  auto step = [&](int k, bool final_step) {
+    MgEpi<T> e = e0;
+    e.mode = kStep;
+    e.step = k;
+    e.rin = rc;
+    e.xin = xc;
+    e.rout = final_step ? nullptr : V.r;
+    e.dout = final_step ? nullptr : dn;
+    e.xout = V.x;
+    if (final_step && l == 0) {
+      e.xout = nullptr;
+      e.z = z;
+      e.r64 = r64;
+      e.dot = r64 != nullptr;
     }
-    return;
+    const int nb = lv_product(L, st, (const T*)d, e);
+    rc = V.r;
+    xc = V.x;
+    std::swap(d, dn);
+    owner->launches += 1;
+    return nb;
+  };
+  if (last) {  // Chebyshev solve from zero
+    for (int k = 1; k < m; ++k) step(k, k + 1 == m);
+    return 0;
+  }
+  for (int k = 1; k < m; ++k) step(k, false);
+  {
+    MgEpi<T> e = e0;
+    e.mode = kResid;
+    e.rin = rc;
+    e.rout = V.r;
+    lv_product(L, st, (const T*)d, e);
   }
   MgLevel& C = mg.lv[l + 1];
-  const View<T> W = view(C, (T*)nullptr);
-  cheb<T>(owner, L, mg.degree, mg.ratio, true, scal);
-  spmv_lv(lc, owner->stream, V.val, V.x, V.w);
-  k_mg_sub<T><<<grid_n(lc->n), kBlk, 0, owner->stream>>>(lc->n, V.b, V.w, V.r, scal);
-  k_mg_restrict<T><<<grid_for(C.c->N, kBlk), kBlk, 0, owner->stream>>>(C.nx, C.ny, C.nz, V.r, lc->fixed, C.c->fixed,
-                                                                      W.b, scal);
-  vcycle<T>(owner, mg, l + 1, scal);
-  k_mg_prolong_add<T><<<grid_for(lc->N, kBlk), kBlk, 0, owner->stream>>>(C.nx, C.ny, C.nz, W.x, lc->fixed,
-                                                                        C.c->fixed, V.x, scal);
-  cheb<T>(owner, L, mg.degree, mg.ratio, false, scal);
-  owner->launches += 5;
+  MgVecs<T>& W = vecs_of(C, (T*)nullptr);
+  const bool cs = l + 2 < mg.lv.size() || mg.cheb_coarse;  // the coarse level smooths
+  launch_pdl(k_mg_restrict<T>, grid_for(C.c->N, 128), 128, st, C.nx, C.ny, C.nz, (const T*)V.r,
+             (const uint8_t*)lc->fixed, (const uint8_t*)C.c->fixed, cs ? dinv_of(C, (T*)nullptr) : (const T*)nullptr,
+             (const double*)C.coef, W.b, W.d, scal);
+  vcycle<T>(owner, mg, l + 1, scal, nullptr, nullptr);
+  launch_pdl(k_mg_prolong<T>, grid_for(lc->N, 128), 128, st, C.nx, C.ny, C.nz, (const T*)W.x,
+             (const uint8_t*)lc->fixed, (const uint8_t*)C.c->fixed, V.w, scal);
+  owner->launches += 3;
+  MgEpi<T> e = e0;
+  e.mode = kStart;
+  e.rin = V.r;
+  e.xin = xc;
+  e.rout = m > 1 ? V.r : nullptr;
+  e.dout = m > 1 ? dn : nullptr;
+  e.xout = V.x;
+  if (m == 1 && l == 0) {
+    e.xout = nullptr;
+    e.z = z;
+    e.r64 = r64;
+    e.dot = r64 != nullptr;
+  }
+  int nb = lv_product(L, st, (const T*)V.w, e);
+  owner->launches += 1;
+  std::swap(d, dn);
+  rc = V.r;
+  xc = V.x;
+  for (int k = 1; k < m; ++k) nb = step(k, k + 1 == m);
+  return nb;
 }
 
-// z = M r on the owner's stream (r, z: FP64 vectors of level 0).
-void run_cycle(Ctx* c, Mg& mg, const double* r, double* z, const CgScalars* scal) {
+// z = M r on the owner's stream from b and d of level 0 (mg_begin); r64, when
+// given, takes part in r.z.  Returns the number of its partials.
+int run_cycle(Ctx* c, Mg& mg, const double* r, double* z, const CgScalars* scal, bool dot) {
   MgLevel& L0 = mg.lv[0];
-  const int64_t n = c->n;
-  if (mg.fp32) {
-    k_mg_convert<double, float><<<grid_n(n), kBlk, 0, c->stream>>>(n, r, L0.b32, scal);
-    vcycle<float>(c, mg, 0, scal);
-    k_mg_convert<float, double><<<grid_n(n), kBlk, 0, c->stream>>>(n, L0.x32, z, scal);
-    c->launches += 2;
-  } else {
-    L0.b = const_cast<double*>(r);
-    L0.x = z;
-    vcycle<double>(c, mg, 0, scal);
-  }
+  if (mg.fp32) return vcycle<float>(c, mg, 0, scal, z, dot ? r : nullptr);
+  L0.v64.b = const_cast<double*>(r);
+  L0.v64.x = z;  // the smoother's running x
+  return vcycle<double>(c, mg, 0, scal, z, dot ? r : nullptr);
+}
+
+// b and d of level 0 from r.
+int begin_cycle(Ctx* c, Mg& mg, const double* r) {
+  MgLevel& L0 = mg.lv[0];
+  if (mg.fp32)
+    k_mg_begin<float><<<grid_n(c->n), kBlk, 0, c->stream>>>(c->n, r, L0.v32.b, L0.v32.d, L0.dinv32, L0.coef);
+  else
+    k_mg_begin<double><<<grid_n(c->n), kBlk, 0, c->stream>>>(c->n, r, nullptr, L0.v64.d, c->dinv64, L0.coef);
+  UFC_CUDA(c, cudaGetLastError());
+  c->launches += 1;
+  return UFC_STATUS_OK;
 }
 
 }  // namespace
@@ -669,10 +1008,18 @@ void mg_mark_stale(Ctx* c) {
   if (c->mg) c->mg->stale = true;
 }
 
+void mg_release_graph(Ctx* c) {
+  if (!c->mg || !c->mg->graph) return;
+  cudaGraphExecDestroy(c->mg->graph);
+  c->mg->graph = nullptr;
+}
+
 void mg_free(Ctx* c) {
   if (!c->mg) return;
   for (auto& L : c->mg->lv) free_level(L);
   dfree(&c->mg->dnorm);
+  dfree(&c->mg->gj_flag);
+  if (c->mg->graph) cudaGraphExecDestroy(c->mg->graph);
   delete c->mg;
   c->mg = nullptr;
 }
@@ -683,6 +1030,18 @@ void mg_free(Ctx* c) {
 // again, on the same boxes and patterns, whenever the owner reassembles.
 static int mg_alloc(Ctx* c, double** p, int64_t n) { return *p ? UFC_STATUS_OK : dalloc(c, p, n); }
 static int mg_alloc(Ctx* c, float** p, int64_t n) { return *p ? UFC_STATUS_OK : dalloc(c, p, n); }
+
+template <typename T>
+static int alloc_vecs(Ctx* c, MgVecs<T>& v, int64_t n, bool xb) {
+  if (xb) {
+    UFC_TRY(mg_alloc(c, &v.x, n));
+    UFC_TRY(mg_alloc(c, &v.b, n));
+  }
+  UFC_TRY(mg_alloc(c, &v.r, n));
+  UFC_TRY(mg_alloc(c, &v.d, n));
+  UFC_TRY(mg_alloc(c, &v.e, n));
+  return mg_alloc(c, &v.w, n);
+}
 
 int mg_refresh(Ctx* c);
 
@@ -696,72 +1055,77 @@ int mg_numeric(Ctx* c) {
     MgLevel& L = mg.lv[l];
     Ctx* lc = L.c;
     UFC_TRY(mg_alloc(c, &L.ke, (int64_t)lc->E * 576));
-    const int grid = lc->E;
-    if (l == 1) {
-      if (tangent)
-        k_mg_galerkin<false, true><<<grid, 64, 0, c->stream>>>(L.nx, L.ny, L.nz, c->coords, c->conn, c->props,
-                                                               c->nprops, c->Dt, nullptr, c->fixed, lc->conn,
-                                                               lc->fixed, L.ke, c->dev_err);
-      else
-        k_mg_galerkin<false, false><<<grid, 64, 0, c->stream>>>(L.nx, L.ny, L.nz, c->coords, c->conn, c->props,
-                                                                c->nprops, nullptr, nullptr, c->fixed, lc->conn,
-                                                                lc->fixed, L.ke, c->dev_err);
+    constexpr int out_bytes = 8 * 576 * (int)sizeof(double);
+    if (l > 1) {
+      k_mg_galerkin<true, false><<<lc->E, kGalThreads, out_bytes, c->stream>>>(
+          L.nx, L.ny, L.nz, nullptr, F.c->conn, nullptr, nullptr, F.ke, F.c->fixed, lc->conn, lc->fixed, L.ke,
+          c->dev_err);
+    } else if (tangent) {
+      constexpr int bytes = std::max(out_bytes, 8 * (int)sizeof(GalWarp<true>));
+      UFC_CUDA(c, cudaFuncSetAttribute(k_mg_galerkin<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+      k_mg_galerkin<false, true><<<lc->E, kGalThreads, bytes, c->stream>>>(
+          L.nx, L.ny, L.nz, c->coords, c->conn, nullptr, c->Dt, nullptr, c->fixed, lc->conn, lc->fixed, L.ke,
+          c->dev_err);
     } else {
-      k_mg_galerkin<true, false><<<grid, 64, 0, c->stream>>>(L.nx, L.ny, L.nz, nullptr, F.c->conn, nullptr, 0,
-                                                             nullptr, F.ke, F.c->fixed, lc->conn, lc->fixed, L.ke,
-                                                             c->dev_err);
+      constexpr int bytes = std::max(out_bytes, 8 * (int)sizeof(GalWarp<false>));
+      UFC_CUDA(c, cudaFuncSetAttribute(k_mg_galerkin<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+      k_mg_galerkin<false, false><<<lc->E, kGalThreads, bytes, c->stream>>>(
+          L.nx, L.ny, L.nz, c->coords, c->conn, c->lame, nullptr, nullptr, c->fixed, lc->conn, lc->fixed, L.ke,
+          c->dev_err);
     }
     UFC_CUDA(c, cudaGetLastError());
     const int64_t nv = lc->sell_blocks * 9;
     UFC_TRY(mg_alloc(c, &lc->val64, nv));
     UFC_TRY(dinv_of(lc));
-    UFC_CUDA(c, cudaMemsetAsync(lc->val64, 0, sizeof(double) * nv, c->stream));
-    for (int col = 0; col < lc->ncol; ++col) {
-      const int32_t ne = lc->col_off[col + 1] - lc->col_off[col];
-      if (ne == 0) continue;
-      k_mg_scatter<<<(int)(((int64_t)ne * 64 + kBlk - 1) / kBlk), kBlk, 0, c->stream>>>(
-          lc->col_elems + lc->col_off[col], ne, lc->conn, L.ke, lc->slot, lc->fixed, lc->val64);
+    if (mg.fp32) {
+      UFC_TRY(mg_alloc(c, &L.val32, nv));
+      UFC_TRY(mg_alloc(c, &L.dinv32, lc->n));
     }
-    if (lc->nfix > 0)
-      k_mg_fix_diag<<<grid_for(lc->nfix, kBlk), kBlk, 0, c->stream>>>(lc->nfix, lc->fix_dofs, lc->dpos, lc->val64);
-    k_mg_dinv<<<grid_for(lc->n, kBlk), kBlk, 0, c->stream>>>(lc->N, lc->dpos, lc->val64, lc->dinv64);
+    const int stride = (9 * lc->max_row_blocks) | 1;
+    const int bytes = (int)sizeof(double) * kMgRows * stride;
+    UFC_CUDA(c, cudaFuncSetAttribute(k_mg_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    k_mg_rows<<<(int)(2 * lc->nslices), kMgRowThreads, bytes, c->stream>>>(
+        lc->N, lc->nptr, lc->nelem, L.ke, lc->slot, lc->slice_ptr, lc->sell_col, lc->dpos, lc->fixed, stride,
+        lc->val64, lc->dinv64, L.val32, L.dinv32);
     UFC_CUDA(c, cudaGetLastError());
     lc->has_val64 = true;
   }
-  UFC_TRY(check_dev_err(c, "ufc_mg_setup"));
-  // level vectors (and FP32 values) in the cycle's precision, smoother bounds, coarsest solve
+  mg.lmax_scale = 1.0;
+  mg.cheb_coarse = mg.lv.back().c->n <= kDenseMax ? 0 : 24;
+  // level vectors in the cycle's precision (level 0: FP32 values too), smoother, coarsest solve
   for (size_t l = 0; l < mg.lv.size(); ++l) {
     MgLevel& L = mg.lv[l];
     const int64_t n = L.c->n;
     if (mg.fp32) {
-      const int64_t nv = L.c->sell_blocks * 9;
-      UFC_TRY(mg_alloc(c, &L.r32, n));
-      UFC_TRY(mg_alloc(c, &L.d32, n));
-      UFC_TRY(mg_alloc(c, &L.w32, n));
-      UFC_TRY(mg_alloc(c, &L.x32, n));
-      UFC_TRY(mg_alloc(c, &L.b32, n));
-      UFC_TRY(mg_alloc(c, &L.val32, nv));
-      UFC_TRY(mg_alloc(c, &L.dinv32, n));
-      k_mg_round<<<grid_n(nv), kBlk, 0, c->stream>>>(nv, L.c->val64, L.val32);
-      k_mg_round<<<grid_n(n), kBlk, 0, c->stream>>>(n, L.c->dinv64, L.dinv32);
-    } else {
-      UFC_TRY(mg_alloc(c, &L.r, n));
-      UFC_TRY(mg_alloc(c, &L.d, n));
-      UFC_TRY(mg_alloc(c, &L.w, n));
-      if (l > 0) {
-        L.own_xb = true;
-        UFC_TRY(mg_alloc(c, &L.x, n));
-        UFC_TRY(mg_alloc(c, &L.b, n));
+      UFC_TRY(alloc_vecs(c, L.v32, n, true));
+      if (l == 0) {
+        UFC_TRY(mg_alloc(c, &L.dinv32, n));
+        k_mg_round<<<grid_n(n), kBlk, 0, c->stream>>>(n, c->dinv64, L.dinv32);
+        if (c->has_sval64 && c->sym_coded && spmv_split(c) == 1) {
+          // the coded symmetric product reads half the bytes (128x64x64: 62 against 89 us)
+          const int64_t nb = c->s_ublocks + kSlice;
+          UFC_TRY(mg_alloc(c, &L.sval32, nb * 9));
+          k_mg_round_sym<<<grid_n(nb), kBlk, 0, c->stream>>>(nb, c->sval64, L.sval32);
+        } else {
+          const int64_t nv = c->sell_blocks * 9;
+          dfree(&L.sval32);
+          UFC_TRY(mg_alloc(c, &L.val32, nv));
+          k_mg_round<<<grid_n(nv), kBlk, 0, c->stream>>>(nv, c->val64, L.val32);
+        }
       }
+    } else {
+      UFC_TRY(alloc_vecs(c, L.v64, n, l > 0));
     }
-    if (l + 1 < mg.lv.size() || n > kDenseMax) UFC_TRY(estimate_lmax(c, mg, L, 15));
+    if (l + 1 < mg.lv.size() || mg.cheb_coarse) UFC_TRY(estimate_lmax(c, mg, l));
   }
   MgLevel& Cst = mg.lv.back();
-  if (Cst.c->n <= kDenseMax) {
-    UFC_TRY(dense_inverse(c, Cst, mg.fp32));
-    mg.cheb_coarse = 0;
-  } else {
-    mg.cheb_coarse = 24;
+  if (!mg.cheb_coarse) UFC_TRY(dense_inverse_device(c, mg, Cst));
+  UFC_TRY(check_dev_err(c, "ufc_mg_setup"));
+  if (!mg.cheb_coarse) {
+    int32_t flag = 0;
+    UFC_CUDA(c, cudaMemcpyAsync(&flag, mg.gj_flag, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+    UFC_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (flag) UFC_TRY(dense_inverse_host(c, Cst, mg.fp32));
   }
   mg.stale = false;
   return UFC_STATUS_OK;
@@ -884,7 +1248,8 @@ int mg_setup(Ctx* c, ufc_mg_arg* a) {
 int mg_apply(Ctx* c, const double* r, double* z) {
   if (!c->mg) return fail(c, UFC_STATUS_INVALID, "ufc_mg_apply: multigrid not set up (ufc_mg_setup)");
   if (c->mg->stale) UFC_TRY(mg_refresh(c));
-  run_cycle(c, *c->mg, r, z, nullptr);
+  UFC_TRY(begin_cycle(c, *c->mg, r));
+  run_cycle(c, *c->mg, r, z, nullptr, false);
   UFC_CUDA(c, cudaGetLastError());
   return UFC_STATUS_OK;
 }
@@ -900,8 +1265,54 @@ int mg_refresh(Ctx* c) {
   if (!c->has_val64) return fail(c, UFC_STATUS_INVALID, "multigrid: the FP64 values are not assembled");
   if (c->mat_model == UFC_MAT_J2_ISO && !c->has_trial)
     return fail(c, UFC_STATUS_INVALID, "multigrid: J2 tangent needs ufc_elem_compute_fint(update_state=1) first");
-  release_graphs(c);
   return mg_numeric(c);
+}
+
+// The PCG iteration as a graph: the V-cycle from b and d of level 0 (z and the
+// partials of r.z), the direction, the product, the update with the next b and
+// d and the stop test.  Kept with the hierarchy (the smoothers' coefficients
+// are read from memory, so a refresh keeps it); rebuilt when one of the vectors
+// or values it reads has moved.  What else it bakes in (pattern, partial sums)
+// is released with the CG graphs (release_graphs) when it is rebuilt.
+static int pcg_mg_graph(Ctx* c, Mg& mg, int batch) {
+  const void* key[9] = {c->r64, c->p64, c->q64, c->z64, c->x64, c->has_sval64 ? c->sval64 : nullptr, c->val64,
+                        mg.lv[0].sval32, mg.lv[0].val32};
+  if (mg.graph && mg.batch == batch && std::equal(key, key + 9, mg.key)) return UFC_STATUS_OK;
+  if (mg.graph) cudaGraphExecDestroy(mg.graph);
+  mg.graph = nullptr;
+  MgLevel& L0 = mg.lv[0];
+  const int64_t n = c->n, counted = c->launches;
+  const int vg = grid_n(n);
+  double* upd = c->partials + c->partials_cap / 2;  // the update's partials, behind the products'
+  cudaGraph_t g;
+  UFC_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+  for (int b = 0; b < batch; ++b) {
+    const Partials rz = product_partials(c, c->stream, run_cycle(c, mg, c->r64, c->z64, c->scal, true));
+    launch_pdl(k_mgcg_pupdate, vg, kBlk, c->stream, n, (const double*)c->z64, c->p64, c->scal, rz.p, rz.nb);
+    const EpiCg<double> epi{c->q64, c->scal};
+    const int nb = c->has_sval64 ? launch_spmv_sym<double, double, double>(c, c->stream, c->sval64, c->p64, epi)
+                                 : launch_spmv<double, double, double>(c, c->stream, c->val64, c->p64, epi);
+    const Partials pq = product_partials(c, c->stream, nb);
+    if (mg.fp32)
+      launch_pdl(k_mgcg_update<float>, vg, kBlk, c->stream, n, (const double*)c->p64, (const double*)c->q64, c->r64,
+                 c->x64, L0.v32.b, L0.v32.d, (const float*)L0.dinv32, (const double*)L0.coef, c->scal, pq.p, pq.nb,
+                 upd);
+    else
+      launch_pdl(k_mgcg_update<double>, vg, kBlk, c->stream, n, (const double*)c->p64, (const double*)c->q64, c->r64,
+                 c->x64, (double*)nullptr, L0.v64.d, (const double*)c->dinv64, (const double*)L0.coef, c->scal, pq.p,
+                 pq.nb, upd);
+    c->launches += 3;
+  }
+  cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+  mg.graph_launches = c->launches - counted;  // captured launches run when the graph does
+  c->launches = counted;
+  if (e != cudaSuccess) return cuda_fail(c, e, "cudaStreamEndCapture");
+  e = cudaGraphInstantiate(&mg.graph, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) return cuda_fail(c, e, "cudaGraphInstantiate");
+  mg.batch = batch;
+  std::copy(key, key + 9, mg.key);
+  return UFC_STATUS_OK;
 }
 
 int pcg_mg(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
@@ -944,53 +1355,48 @@ int pcg_mg(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
   double true_rr = c->h_scal->true_rr;
   bool converged = std::sqrt(true_rr) <= tol;
   int flag = 0, restarts = 0;
-  const int batch = algo->check_every > 0 ? algo->check_every : 4;
-  cudaGraphExec_t ge = nullptr;
-  int64_t graph_launches = 0;
+  const int batch = algo->check_every > 0 ? algo->check_every : 2;
   int status = UFC_STATUS_OK;
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  if (!converged) {
+    UFC_TRY(pcg_mg_graph(c, mg, batch));
+    for (auto& e : done) UFC_CUDA(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
+  CgScalars* hs[2] = {c->h_scal + 1, c->h_scal + 2};
   while (!converged && status == UFC_STATUS_OK) {
-    // (re)start: r = the FP64 residual, z = M r, p = z
+    // (re)start: r = the FP64 residual, b and d of the cycle; the first iteration takes p = z = M r
+    struct {
+      int32_t stop, want, fresh;
+    } restart{0, 0, 1};
+    static_assert(offsetof(CgScalars, want_update) == offsetof(CgScalars, stop) + 4 &&
+                      offsetof(CgScalars, fresh) == offsetof(CgScalars, stop) + 8,
+                  "restart writes stop, want_update and fresh in one copy");
     double tol2 = tol * tol;
     UFC_CUDA(c, cudaMemcpyAsync(&c->scal->tol2, &tol2, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    UFC_CUDA(c, cudaMemsetAsync(&c->scal->stop, 0, sizeof(int32_t), c->stream));
+    UFC_CUDA(c, cudaMemcpyAsync(&c->scal->stop, &restart, sizeof(restart), cudaMemcpyHostToDevice, c->stream));
     UFC_CUDA(c, cudaMemcpyAsync(c->r64, c->y64, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
-    run_cycle(c, mg, c->r64, c->z64, c->scal);
-    k_mgcg_rz<<<vg, kBlk, 0, c->stream>>>(n, c->r64, c->z64, c->scal, c->partials, 1);
-    c->launches += 1;
-    UFC_CUDA(c, cudaMemcpyAsync(c->p64, c->z64, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
-    if (!ge) {
-      cudaGraph_t g;
-      const int64_t counted = c->launches;
-      UFC_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-      for (int b = 0; b < batch; ++b) {
-        cg_spmv64(c, c->p64, c->q64);
-        k_mgcg_update<<<vg, kBlk, 0, c->stream>>>(n, c->p64, c->q64, c->r64, c->x64, c->scal, c->partials);
-        run_cycle(c, mg, c->r64, c->z64, c->scal);
-        k_mgcg_rz<<<vg, kBlk, 0, c->stream>>>(n, c->r64, c->z64, c->scal, c->partials, 0);
-        k_mgcg_pupdate<<<vg, kBlk, 0, c->stream>>>(n, c->z64, c->p64, c->scal);
-        c->launches += 4;
-      }
-      cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-      if (e != cudaSuccess) return cuda_fail(c, e, "cudaStreamEndCapture");
-      e = cudaGraphInstantiate(&ge, g, 0);
-      cudaGraphDestroy(g);
-      if (e != cudaSuccess) return cuda_fail(c, e, "cudaGraphInstantiate");
-      graph_launches = c->launches - counted;  // captured launches run when the graph does
-      c->launches = counted;
-    }
+    UFC_TRY(begin_cycle(c, mg, c->r64));
+    // one batch stays in flight while the one before it is looked at
+    int slot = 0, in_flight = 0;
     for (;;) {
-      cudaError_t e = cudaGraphLaunch(ge, c->stream);
+      cudaError_t e = cudaGraphLaunch(mg.graph, c->stream);
       if (e != cudaSuccess) {
         status = cuda_fail(c, e, "cudaGraphLaunch");
         break;
       }
-      c->launches += graph_launches;
-      UFC_CUDA(c, cudaMemcpyAsync(c->h_scal, c->scal, sizeof(CgScalars), cudaMemcpyDeviceToHost, c->stream));
-      UFC_CUDA(c, cudaStreamSynchronize(c->stream));
-      if (c->h_scal->stop) break;
+      c->launches += mg.graph_launches;
+      UFC_CUDA(c, cudaMemcpyAsync(hs[slot], c->scal, sizeof(CgScalars), cudaMemcpyDeviceToHost, c->stream));
+      UFC_CUDA(c, cudaEventRecord(done[slot], c->stream));
+      slot ^= 1;
+      if (in_flight == 0) {
+        in_flight = 1;
+        continue;
+      }
+      UFC_CUDA(c, cudaEventSynchronize(done[slot]));
+      if (hs[slot]->stop) break;
     }
     if (status != UFC_STATUS_OK) break;
-    const int stop = c->h_scal->stop;
+    const int stop = hs[slot]->stop;
     UFC_TRY(true_residual_fp64(c, false));
     UFC_CUDA(c, cudaMemcpyAsync(c->h_scal, c->scal, sizeof(CgScalars), cudaMemcpyDeviceToHost, c->stream));
     UFC_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1007,8 +1413,20 @@ int pcg_mg(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
       flag = 3;
       break;
     }
+    if (stop == 3) {
+      // the cycle was not positive definite: lambda_max was underestimated, so
+      // the smoothers' intervals are widened before the restart
+      constexpr double kWiden = 1.3;
+      mg.lmax_scale *= kWiden;
+      for (size_t l = 0; l < mg.lv.size(); ++l)
+        if (mg.lv[l].coef && lv_degree(mg, l) > 0)
+          k_mg_coef<<<1, kBlk, 0, c->stream>>>(nullptr, 0, nullptr, kWiden, lv_ratio(mg, l), lv_degree(mg, l),
+                                               mg.lv[l].coef);
+      UFC_CUDA(c, cudaGetLastError());
+    }
   }
-  if (ge) cudaGraphExecDestroy(ge);
+  for (auto& e : done)
+    if (e) cudaEventDestroy(e);
   if (status != UFC_STATUS_OK) return status;
   UFC_CUDA(c, cudaEventRecord(t1, c->stream));
   UFC_CUDA(c, cudaEventSynchronize(t1));

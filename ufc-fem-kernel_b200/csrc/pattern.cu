@@ -956,10 +956,12 @@ int build_sym_pattern(Ctx* c) {
 
 int pack_symmetric(Ctx* c, bool fp64, bool fp32) {
   if (!c->has_val64) return fail(c, UFC_STATUS_INVALID, "symmetric storage: FP64 values not assembled");
+  bool moved = !c->has_sym_pattern;  // arrays that captured graphs read
   UFC_TRY(build_sym_pattern(c));
   // stored blocks plus one zero slice that padded lower references point at
   const int64_t nv = (c->s_ublocks + kSlice) * 9;
   if (fp64) {
+    moved |= !c->sval64;
     if (!c->sval64) UFC_TRY(dalloc(c, &c->sval64, nv));
     UFC_CUDA(c, cudaMemsetAsync(c->sval64, 0, sizeof(double) * nv, c->stream));
     k_sym_pack<double><<<grid_for(c->N, 128), 128, 0, c->stream>>>(c->N, c->slice_ptr, c->uptr, c->brow, c->s_lcnt,
@@ -968,6 +970,7 @@ int pack_symmetric(Ctx* c, bool fp64, bool fp32) {
     c->has_sval64 = true;
   }
   if (fp32) {
+    moved |= !c->sval32;
     if (!c->sval32) UFC_TRY(dalloc(c, &c->sval32, nv));
     UFC_CUDA(c, cudaMemsetAsync(c->sval32, 0, sizeof(float) * nv, c->stream));
     k_sym_pack<float><<<grid_for(c->N, 128), 128, 0, c->stream>>>(c->N, c->slice_ptr, c->uptr, c->brow, c->s_lcnt,
@@ -975,7 +978,7 @@ int pack_symmetric(Ctx* c, bool fp64, bool fp32) {
     UFC_CUDA(c, cudaGetLastError());
     c->has_sval32 = true;
   }
-  release_graphs(c);
+  if (moved) release_graphs(c);
   return UFC_STATUS_OK;
 }
 

@@ -42,6 +42,7 @@ struct CgScalars {
   int32_t max_iter;
   int32_t stop;     // 1 converged (recursive), 2 max-iter, 3 breakdown
   int32_t want_update;
+  int32_t fresh;    // multigrid PCG: the next direction starts anew (p = z)
   double nr_rr, nr_ff, nr_ee;  // Newton: ||R_free||^2, ||F_int||^2, ||F_ext||^2
   double* hist;        // ||r||^2 of the recursive residual per iteration (or null)
   int32_t hist_cap;
@@ -250,15 +251,13 @@ int adjoint_sens(Ctx* c, int nrhs, const double* U, const double* L, double* g);
 // mg.cu
 int mg_setup(Ctx* c, ufc_mg_arg* a);
 void mg_free(Ctx* c);
+void mg_release_graph(Ctx* c);
 void mg_mark_stale(Ctx* c);  // the matrix changed: the hierarchy must be set up again
 int mg_apply(Ctx* c, const double* r, double* z);
 int mg_level_ctx(Ctx* c, int32_t level, Ctx** out);
 int pcg_mg(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st);
 // FP64 SELL SpMV (full storage) of any context's values, on the given stream (solver.cu)
 void spmv64_on(const Ctx* lvl, cudaStream_t st, const double* x, double* y);
-// FP32 SELL SpMV of the given values (standard form) on any context's pattern
-void spmv32_on(const Ctx* lvl, cudaStream_t st, const float* val, const float* x, float* y);
-void cg_spmv64(Ctx* c, const double* p, double* q);  // q = K p, p.q and alpha = r.z / p.q into the scalars
 int true_residual_fp64(Ctx* c, bool want_bb);  // y64 = b64 - K x64, scal->true_rr (and bb)
 
 // output.cu
