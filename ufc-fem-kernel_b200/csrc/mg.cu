@@ -123,7 +123,7 @@ __device__ __forceinline__ double hat(int A, int x0, int x1, int x2) {
 // the lane's own two blocks); rows and columns of fixed DOFs are zeroed before
 // (fine) and after (coarse).  The 8 children are added in order.
 // 64x32x32, level 1 from the elements: 1298 us with one 64-thread CTA walking
-// through the children and the dense W, now 132 us.
+// through the children and the dense W, now 153 us.
 constexpr int kGalThreads = 256;
 
 template <bool TANGENT>
@@ -375,28 +375,44 @@ __global__ void k_mg_restrict(int32_t nxc, int32_t nyc, int32_t nzc, const T* __
   const int nxf = 2 * nxc, nyf = 2 * nyc, nzf = 2 * nzc;
   const int32_t I = (int32_t)(v % (nxc + 1)), J = (int32_t)((v / (nxc + 1)) % (nyc + 1)),
                 K = (int32_t)(v / ((int64_t)(nxc + 1) * (nyc + 1)));
+  // which of the 27 x 3 entries count (Dirichlet flags, box edges): read before
+  // the wait for the kernel in front
+  uint32_t use[3] = {0, 0, 0};
+  if (v < nc) {
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+      const int k = 2 * K + q / 9 - 1, j = 2 * J + (q / 3) % 3 - 1, i = 2 * I + q % 3 - 1;
+      if (k < 0 || k > nzf || j < 0 || j > nyf || i < 0 || i > nxf) continue;
+      const int64_t f = box_node(i, j, k, nxf, nyf);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) use[d] |= fixed_f[3 * f + d] ? 0u : 1u << q;
+    }
+  }
+  T di[3] = {T(0), T(0), T(0)};
+  bool fc[3] = {true, true, true};
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    if (v < nc) {
+      fc[d] = fixed_c[3 * v + d] != 0;
+      if (dinv) di[d] = dinv[3 * v + d];
+    }
   pdl_enter();
   if (v >= nc || (scal && scal->stop)) return;
   T s[3] = {T(0), T(0), T(0)};
 #pragma unroll
-  for (int dk = -1; dk <= 1; ++dk)
+  for (int q = 0; q < 27; ++q) {
+    const int k = q / 9 - 1, j = (q / 3) % 3 - 1, i = q % 3 - 1;
+    const T w = T((i ? 0.5 : 1.0) * (j ? 0.5 : 1.0) * (k ? 0.5 : 1.0));
+    const int64_t f = box_node(2 * I + i, 2 * J + j, 2 * K + k, nxf, nyf);
 #pragma unroll
-    for (int dj = -1; dj <= 1; ++dj)
-#pragma unroll
-      for (int di = -1; di <= 1; ++di) {
-        const int k = 2 * K + dk, j = 2 * J + dj, i = 2 * I + di;
-        if (k < 0 || k > nzf || j < 0 || j > nyf || i < 0 || i > nxf) continue;
-        const T w = T((di ? 0.5 : 1.0) * (dj ? 0.5 : 1.0) * (dk ? 0.5 : 1.0));
-        const int64_t f = box_node(i, j, k, nxf, nyf);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) s[d] += fixed_f[3 * f + d] ? T(0) : w * rf[3 * f + d];
-      }
+    for (int d = 0; d < 3; ++d) s[d] += (use[d] >> q) & 1u ? w * rf[3 * f + d] : T(0);
+  }
   const T it = dinv ? (T)coef[1] : T(0);
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const T b = fixed_c[3 * v + d] ? T(0) : s[d];
+    const T b = fc[d] ? T(0) : s[d];
     bc[3 * v + d] = b;
-    if (dinv) dc[3 * v + d] = dinv[3 * v + d] * b * it;
+    if (dinv) dc[3 * v + d] = di[d] * b * it;
   }
 }
 
@@ -410,23 +426,32 @@ __global__ void k_mg_prolong(int32_t nxc, int32_t nyc, int32_t nzc, const T* __r
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int32_t i = (int32_t)(v % (nxf + 1)), j = (int32_t)((v / (nxf + 1)) % (nyf + 1)),
                 k = (int32_t)(v / ((int64_t)(nxf + 1) * (nyf + 1)));
+  const T w = T(((i & 1) ? 0.5 : 1.0) * ((j & 1) ? 0.5 : 1.0) * ((k & 1) ? 0.5 : 1.0));
+  uint32_t use[3] = {0, 0, 0};  // as in k_mg_restrict
+  bool ff[3] = {true, true, true};
+  if (v < nf) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int a = q & 1, b = (q >> 1) & 1, c = q >> 2;
+      if ((c && !(k & 1)) || (b && !(j & 1)) || (a && !(i & 1))) continue;
+      const int64_t cn = box_node((i >> 1) + a, (j >> 1) + b, (k >> 1) + c, nxc, nyc);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) use[d] |= fixed_c[3 * cn + d] ? 0u : 1u << q;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) ff[d] = fixed_f[3 * v + d] != 0;
+  }
   pdl_enter();
   if (v >= nf || (scal && scal->stop)) return;
-  const T w = T(((i & 1) ? 0.5 : 1.0) * ((j & 1) ? 0.5 : 1.0) * ((k & 1) ? 0.5 : 1.0));
   T s[3] = {T(0), T(0), T(0)};
 #pragma unroll
-  for (int c = 0; c < 2; ++c)
+  for (int q = 0; q < 8; ++q) {
+    const int64_t cn = box_node((i >> 1) + (q & 1), (j >> 1) + ((q >> 1) & 1), (k >> 1) + (q >> 2), nxc, nyc);
 #pragma unroll
-    for (int b = 0; b < 2; ++b)
+    for (int d = 0; d < 3; ++d) s[d] += (use[d] >> q) & 1u ? w * xc[3 * cn + d] : T(0);
+  }
 #pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        if ((c && !(k & 1)) || (b && !(j & 1)) || (a && !(i & 1))) continue;
-        const int64_t cn = box_node((i >> 1) + a, (j >> 1) + b, (k >> 1) + c, nxc, nyc);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) s[d] += fixed_c[3 * cn + d] ? T(0) : w * xc[3 * cn + d];
-      }
-#pragma unroll
-  for (int d = 0; d < 3; ++d) vf[3 * v + d] = fixed_f[3 * v + d] ? T(0) : s[d];
+  for (int d = 0; d < 3; ++d) vf[3 * v + d] = ff[d] ? T(0) : s[d];
 }
 
 // The Chebyshev smoother (three-term recurrence of Saad, Iterative Methods for

@@ -67,6 +67,18 @@ __device__ __forceinline__ void ld4(const T* __restrict__ p, T (&o)[4]) {
   }
 }
 
+// The same past L1, for loads before griddepcontrol.wait.
+template <typename T>
+__device__ __forceinline__ void ld4_cg(const T* __restrict__ p, T (&o)[4]) {
+  if constexpr (sizeof(T) == 4) {
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
+    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+  } else {
+    const double2 a = __ldcg(reinterpret_cast<const double2*>(p)), b = __ldcg(reinterpret_cast<const double2*>(p + 2));
+    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
+  }
+}
+
 template <typename T>
 __device__ __forceinline__ void st4(T* __restrict__ p, const T (&o)[4]) {
   if constexpr (sizeof(T) == 4) {
@@ -80,13 +92,28 @@ __device__ __forceinline__ void st4(T* __restrict__ p, const T (&o)[4]) {
 // x += alpha p, r -= alpha q with alpha = r.z / p.q (p.q from the product's nb
 // partials), and the block's partials of r.z and r.r.  Block 0 moves the
 // scalars on; the other blocks read only scal->rz, which this kernel leaves alone.
+// A thread's first entries of p, r, x and D^-1 are read before the wait for the
+// product, which writes only q and its partials (the kernels that wrote p, r and
+// x were complete before the product began).
 template <typename T>
 __global__ void __launch_bounds__(kVecBlock)
     k_cg_update(int64_t n, const T* __restrict__ p, const T* __restrict__ q, T* __restrict__ r,
                 double* __restrict__ x, const T* __restrict__ dinv, CgScalars* __restrict__ scal,
                 const double* __restrict__ pq_partials, int nb, double* __restrict__ partials) {
+  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t n4 = n >> 2;
+  T pv[4], qv[4], rv[4], dv[4];
+  double xv[4];
+  auto load = [&](int64_t i) {
+    ld4_cg(p + i, pv);
+    ld4_cg(r + i, rv);
+    ld4_cg(x + i, xv);
+    if (dinv) ld4_cg(dinv + i, dv);
+  };
+  if (gid < n4) load(gid << 2);
   pdl_enter();
   if (halted(scal)) return;
+  if (gid < n4) ld4_cg(q + (gid << 2), qv);
   double pq[1];
   sum_partials<1>(pq_partials, nb, pq);
   const bool broken = !(fabs(pq[0]) > 1e-300) || !isfinite(pq[0]);
@@ -104,17 +131,12 @@ __global__ void __launch_bounds__(kVecBlock)
   if (broken) return;
   const T a = (T)alpha;
   T rz = T(0), rr = T(0);
-  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t n4 = n >> 2;
   for (int64_t k = gid; k < n4; k += stride) {
     const int64_t i = k << 2;
-    T pv[4], qv[4], rv[4], dv[4];
-    double xv[4];
-    ld4(p + i, pv);
-    ld4(q + i, qv);
-    ld4(r + i, rv);
-    ld4(x + i, xv);
-    if (dinv) ld4(dinv + i, dv);
+    if (k != gid) {
+      load(i);
+      ld4_cg(q + i, qv);
+    }
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       xv[c] += alpha * (double)pv[c];
@@ -148,8 +170,18 @@ template <typename T>
 __global__ void __launch_bounds__(kVecBlock)
     k_cg_pupdate(int64_t n, const T* __restrict__ r, const T* __restrict__ dinv, T* __restrict__ p,
                  CgScalars* __restrict__ scal, const double* __restrict__ partials, int nb) {
+  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t n4 = n >> 2;
+  T rv[4], pv[4], dv[4];
+  // the update in front writes r, not p and D^-1
+  auto load = [&](int64_t i) {
+    ld4_cg(p + i, pv);
+    if (dinv) ld4_cg(dinv + i, dv);
+  };
+  if (gid < n4) load(gid << 2);
   pdl_enter();
   if (halted(scal)) return;
+  if (gid < n4) ld4_cg(r + (gid << 2), rv);
   double b;
   if (nb > 0) {
     double tot[2];
@@ -175,19 +207,17 @@ __global__ void __launch_bounds__(kVecBlock)
     b = scal->beta;
   }
   const T beta = (T)b;
-  // beta = 0 (start, restart after a breakdown): p = z without reading p, whose
-  // contents are then undefined (fresh memory, or the NaN of the breakdown)
+  // beta = 0 (start, restart after a breakdown): p = z whatever p holds (fresh
+  // memory, or the NaN of the breakdown)
   const bool fresh = b == 0.0;
-  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t n4 = n >> 2;
   for (int64_t k = gid; k < n4; k += stride) {
     const int64_t i = k << 2;
-    T rv[4], pv[4] = {T(0), T(0), T(0), T(0)}, dv[4];
-    ld4(r + i, rv);
-    if (!fresh) ld4(p + i, pv);
-    if (dinv) ld4(dinv + i, dv);
+    if (k != gid) {
+      load(i);
+      ld4_cg(r + i, rv);
+    }
 #pragma unroll
-    for (int c = 0; c < 4; ++c) pv[c] = (dinv ? dv[c] * rv[c] : rv[c]) + beta * pv[c];
+    for (int c = 0; c < 4; ++c) pv[c] = (dinv ? dv[c] * rv[c] : rv[c]) + (fresh ? T(0) : beta * pv[c]);
     st4(p + i, pv);
   }
   for (int64_t i = (n4 << 2) + gid; i < n; i += stride) {

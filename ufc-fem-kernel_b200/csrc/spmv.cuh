@@ -28,6 +28,16 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" :::);
 }
 
+// Stored steps that a warp of a split product loads (columns and values) before
+// it waits for the kernel in front: the matrix is not written inside a chain,
+// so these loads pass behind that kernel's end, and what follows the wait is
+// one gather.  All steps of a warp on the small meshes that take 8 warps per
+// slice, where a product's time is latency.
+template <typename TV, int SPLIT>
+constexpr int split_ahead() {
+  return SPLIT == 8 ? 4 : sizeof(TV) == 4 ? 4 : 2;
+}
+
 template <typename... K, typename... A>
 void launch_pdl(void (*kernel)(K...), int grid, int block, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -151,42 +161,57 @@ __global__ void __launch_bounds__(kSpmvBlock)
 template <typename TV, typename TX, typename TA, class EPI, bool DIFF, int SPLIT>
 __global__ void __launch_bounds__(kSpmvBlock)
     k_spmv_split(int32_t N, int64_t nslices, const int64_t* __restrict__ sptr, const int32_t* __restrict__ col,
-           const TV* __restrict__ val, const TX* __restrict__ x, EPI epi,
-           double* __restrict__ partials) {
-  pdl_enter();
-  if (epi.halt()) return;
-  constexpr int kWarps = kSpmvBlock / 32;
+                 const TV* __restrict__ val, const TX* __restrict__ x, EPI epi, double* __restrict__ partials) {
+  constexpr int kWarps = kSpmvBlock / 32, kAhead = split_ahead<TV, SPLIT>();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int part = warp % SPLIT;
   const int64_t s = (int64_t)blockIdx.x * (kWarps / SPLIT) + warp / SPLIT;
   const int64_t row = s * kSlice + lane;
+  const int64_t base = s < nslices ? sptr[s] : 0;
+  const int len = s < nslices ? (int)((sptr[s + 1] - base) >> 5) : 0;
+  const int32_t* cp = col + base + lane;
+  const TV* vp = val + 9 * base + lane;
+  int32_t ca[kAhead];
+  TV va[kAhead][9];
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) {
+    const int j = part + u * SPLIT;
+    ca[u] = j < len ? __ldcs(cp + 32 * j) : 0;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) va[u][c] = j < len ? __ldcs(vp + 288 * (int64_t)j + 32 * c) : TV(0);
+  }
+  pdl_enter();
+  if (epi.halt()) return;
   TA a0 = TA(0), a1 = TA(0), a2 = TA(0);
   if (s < nslices) {
-    const int64_t base = sptr[s];
-    const int len = (int)((sptr[s + 1] - base) >> 5);
-    const int32_t* cp = col + base + lane;
-    const TV* vp = val + 9 * base + lane;
     TA xi0 = TA(0), xi1 = TA(0), xi2 = TA(0);
     if (DIFF && row < N) {
       xi0 = (TA)x[3 * row];
       xi1 = (TA)x[3 * row + 1];
       xi2 = (TA)x[3 * row + 2];
     }
-    auto block = [&](int j) {
-      const int64_t cj = __ldcs(cp + 32 * j);
+    auto block = [&](int64_t cj, const TV(&v)[9]) {
       TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
       if (DIFF && cj != row) {
         x0 -= xi0;
         x1 -= xi1;
         x2 -= xi2;
       }
-      const TV* v = vp + 288 * (int64_t)j;
-      a0 += (TA)__ldcs(v) * x0 + (TA)__ldcs(v + 32) * x1 + (TA)__ldcs(v + 64) * x2;
-      a1 += (TA)__ldcs(v + 96) * x0 + (TA)__ldcs(v + 128) * x1 + (TA)__ldcs(v + 160) * x2;
-      a2 += (TA)__ldcs(v + 192) * x0 + (TA)__ldcs(v + 224) * x1 + (TA)__ldcs(v + 256) * x2;
+      a0 += (TA)v[0] * x0 + (TA)v[1] * x1 + (TA)v[2] * x2;
+      a1 += (TA)v[3] * x0 + (TA)v[4] * x1 + (TA)v[5] * x2;
+      a2 += (TA)v[6] * x0 + (TA)v[7] * x1 + (TA)v[8] * x2;
     };
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (part + u * SPLIT < len) block(ca[u], va[u]);
 #pragma unroll 2
-    for (int j = part; j < len; j += SPLIT) block(j);
+    for (int j = part + kAhead * SPLIT; j < len; j += SPLIT) {
+      const int64_t cj = __ldcs(cp + 32 * j);
+      TV v[9];
+#pragma unroll
+      for (int c = 0; c < 9; ++c) v[c] = __ldcs(vp + 288 * (int64_t)j + 32 * c);
+      block(cj, v);
+    }
   }
   {
     __shared__ TA sh[kWarps][3][32];
@@ -521,53 +546,71 @@ template <typename TV, typename TX, typename TA, class EPI, int SPLIT>
 __global__ void __launch_bounds__(kSpmvBlock)
     k_spmv_sym_split(int32_t N, int64_t nslices, const int64_t* __restrict__ uptr, const int32_t* __restrict__ ucol,
                      const int64_t* __restrict__ lptr, const int32_t* __restrict__ lpos,
-                     const int32_t* __restrict__ lcol, const TV* __restrict__ val, const TX* __restrict__ x,
-                     EPI epi,
-           double* __restrict__ partials) {
-  pdl_enter();
-  if (epi.halt()) return;
-  constexpr int kWarps = kSpmvBlock / 32;
+                     const int32_t* __restrict__ lcol, const TV* __restrict__ val, const TX* __restrict__ x, EPI epi,
+                     double* __restrict__ partials) {
+  // a warp's steps hold an upper and a lower block each: half as many ahead
+  constexpr int kWarps = kSpmvBlock / 32, kAhead = split_ahead<TV, SPLIT>() / 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int part = warp % SPLIT;
   const int64_t s = (int64_t)blockIdx.x * (kWarps / SPLIT) + warp / SPLIT;
   const int64_t row = s * kSlice + lane;
+  const bool real = s < nslices;
+  const int64_t ub = real ? uptr[s] : 0, lb = real ? lptr[s] : 0;
+  const int ulen = real ? (int)((uptr[s + 1] - ub) >> 5) : 0;
+  const int llen = real ? (int)((lptr[s + 1] - lb) >> 5) : 0;
+  const int32_t* ucp = ucol + ub + lane;
+  const TV* uvp = val + 9 * ub;
+  const int32_t* lpp = lpos + lb + lane;
+  const int32_t* lcp = lcol + lb + lane;
+  auto load_lower = [&](int j, TV(&v)[9]) {
+    const int64_t P = __ldcs(lpp + 32 * j);
+    load_block(val + 9 * (P & ~int64_t(31)), (int)(P & 31), v);
+  };
+  int32_t cu[kAhead], cl[kAhead];
+  TV vu[kAhead][9], vl[kAhead][9];
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) {
+    const int j = part + u * SPLIT;
+    cu[u] = j < ulen ? __ldcs(ucp + 32 * j) : 0;
+    cl[u] = j < llen ? __ldcs(lcp + 32 * j) : 0;
+    if (j < ulen) load_block(uvp + 288 * (int64_t)j, lane, vu[u]);
+    if (j < llen) load_lower(j, vl[u]);
+  }
+  pdl_enter();
+  if (epi.halt()) return;
   TA a0 = TA(0), a1 = TA(0), a2 = TA(0);
-  if (s < nslices) {
-    const int64_t ub = uptr[s], lb = lptr[s];
-    const int ulen = (int)((uptr[s + 1] - ub) >> 5);
-    const int llen = (int)((lptr[s + 1] - lb) >> 5);
-    const int32_t* ucp = ucol + ub + lane;
-    const TV* uvp = val + 9 * ub;
-    const int32_t* lpp = lpos + lb + lane;
-    const int32_t* lcp = lcol + lb + lane;
-    auto upper = [&](int j) {
-      const int64_t cj = __ldcs(ucp + 32 * j);
-      const TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
-      TV v[9];
-      load_block(uvp + 288 * (int64_t)j, lane, v);
-      a0 += (TA)v[0] * x0 + (TA)v[1] * x1 + (TA)v[2] * x2;
-      a1 += (TA)v[3] * x0 + (TA)v[4] * x1 + (TA)v[5] * x2;
-      a2 += (TA)v[6] * x0 + (TA)v[7] * x1 + (TA)v[8] * x2;
-    };
-    auto lower = [&](int j) {
-      const int64_t P = __ldcs(lpp + 32 * j);
-      const int64_t cj = __ldcs(lcp + 32 * j);
-      const TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
-      TV v[9];
-      load_block(val + 9 * (P & ~int64_t(31)), (int)(P & 31), v);
-      a0 += (TA)v[0] * x0 + (TA)v[3] * x1 + (TA)v[6] * x2;
-      a1 += (TA)v[1] * x0 + (TA)v[4] * x1 + (TA)v[7] * x2;
-      a2 += (TA)v[2] * x0 + (TA)v[5] * x1 + (TA)v[8] * x2;
-    };
-    const int mlen = ulen < llen ? ulen : llen;
-    int j = part;
+  auto upper = [&](int64_t cj, const TV(&v)[9]) {
+    const TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
+    a0 += (TA)v[0] * x0 + (TA)v[1] * x1 + (TA)v[2] * x2;
+    a1 += (TA)v[3] * x0 + (TA)v[4] * x1 + (TA)v[5] * x2;
+    a2 += (TA)v[6] * x0 + (TA)v[7] * x1 + (TA)v[8] * x2;
+  };
+  // transposed block: (K_ji^T x)_r = sum_c K_ji[c][r] x_c
+  auto lower = [&](int64_t cj, const TV(&v)[9]) {
+    const TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
+    a0 += (TA)v[0] * x0 + (TA)v[3] * x1 + (TA)v[6] * x2;
+    a1 += (TA)v[1] * x0 + (TA)v[4] * x1 + (TA)v[7] * x2;
+    a2 += (TA)v[2] * x0 + (TA)v[5] * x1 + (TA)v[8] * x2;
+  };
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) {
+    if (part + u * SPLIT < ulen) upper(cu[u], vu[u]);
+    if (part + u * SPLIT < llen) lower(cl[u], vl[u]);
+  }
+  const int mlen = ulen > llen ? ulen : llen;
 #pragma unroll 1
-    for (; j < mlen; j += SPLIT) {
-      upper(j);
-      lower(j);
+  for (int j = part + kAhead * SPLIT; j < mlen; j += SPLIT) {
+    TV v[9];
+    if (j < ulen) {
+      const int64_t cj = __ldcs(ucp + 32 * j);
+      load_block(uvp + 288 * (int64_t)j, lane, v);
+      upper(cj, v);
     }
-    for (int k = j; k < ulen; k += SPLIT) upper(k);
-    for (int k = j; k < llen; k += SPLIT) lower(k);
+    if (j < llen) {
+      const int64_t cj = __ldcs(lcp + 32 * j);
+      load_lower(j, v);
+      lower(cj, v);
+    }
   }
   {
     __shared__ TA sh[kWarps][3][32];
