@@ -435,6 +435,8 @@ int ensure_vectors(Ctx* c, int prec) {
   return UFC_STATUS_OK;
 }
 
+constexpr int kResidentChunk = 1024;  // iterations of one resident launch between host checks
+
 template <typename TV, typename TX, typename TA>
 int pcg_run(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
   const int prec = algo->precision_mode;
@@ -490,7 +492,10 @@ int pcg_run(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
     UFC_TRY(replace(R, V, 2));
     cudaGraphExec_t graph = nullptr;
     int64_t graph_launches = 0;
-    if (!c->instrument) UFC_TRY((get_graph<TV, TX, TA>(R, V, batch, &graph, &graph_launches)));
+    // small FP64 systems: all iterations in one kernel (resident.cu)
+    bool resident = false;
+    if constexpr (sizeof(TV) == 8) resident = !c->instrument && cg_resident_fits(c);
+    if (!c->instrument && !resident) UFC_TRY((get_graph<TV, TX, TA>(R, V, batch, &graph, &graph_launches)));
     std::vector<cudaEvent_t> evs;
     if (c->instrument) {
       evs.resize(2 * batch);
@@ -511,52 +516,61 @@ int pcg_run(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
     bool finished = false;
     int status = UFC_STATUS_OK;
     while (!finished) {
-      if (graph) {
-        cudaError_t e = cudaGraphLaunch(graph, c->stream);
-        if (e != cudaSuccess) {
-          status = cuda_fail(c, e, "cudaGraphLaunch");
-          break;
-        }
-        c->launches += graph_launches;
+      CgScalars cur;
+      if (resident) {
+        if constexpr (sizeof(TV) == 8)
+          status = cg_resident(c, V.dinv, algo->check_every > 0 ? algo->check_every : kResidentChunk);
+        if (status == UFC_STATUS_OK) status = read_scalars(c);
+        if (status != UFC_STATUS_OK) break;
+        cur = *c->h_scal;
       } else {
-        for (int k = 0; k < batch; ++k)
-          launch_iteration<TV, TX, TA>(R, V, c->stream, evs[2 * k], evs[2 * k + 1]);
-      }
-      cudaMemcpyAsync(hs[slot], c->scal, sizeof(CgScalars), cudaMemcpyDeviceToHost, c->stream);
-      cudaEventRecord(done[slot], c->stream);
-      if (c->instrument) {
-        // one batch in flight at a time: the events are reused; only the
-        // launches that did an iteration (not the no-op tail) are counted
-        cudaEventSynchronize(done[slot]);
-        const int did = std::min(batch, hs[slot]->iter - iter_seen);
-        iter_seen = hs[slot]->iter;
-        for (int k = 0; k < did; ++k) {
-          float ms = 0.f;
-          if (cudaEventElapsedTime(&ms, evs[2 * k], evs[2 * k + 1]) == cudaSuccess) {
-            c->timing.spmv_ms += ms;
-            c->timing.spmv_launches += 1;
+        if (graph) {
+          cudaError_t e = cudaGraphLaunch(graph, c->stream);
+          if (e != cudaSuccess) {
+            status = cuda_fail(c, e, "cudaGraphLaunch");
+            break;
           }
+          c->launches += graph_launches;
+        } else {
+          for (int k = 0; k < batch; ++k)
+            launch_iteration<TV, TX, TA>(R, V, c->stream, evs[2 * k], evs[2 * k + 1]);
         }
-        in_flight = 1;
-        slot ^= 1;
+        cudaMemcpyAsync(hs[slot], c->scal, sizeof(CgScalars), cudaMemcpyDeviceToHost, c->stream);
+        cudaEventRecord(done[slot], c->stream);
+        if (c->instrument) {
+          // one batch in flight at a time: the events are reused; only the
+          // launches that did an iteration (not the no-op tail) are counted
+          cudaEventSynchronize(done[slot]);
+          const int did = std::min(batch, hs[slot]->iter - iter_seen);
+          iter_seen = hs[slot]->iter;
+          for (int k = 0; k < did; ++k) {
+            float ms = 0.f;
+            if (cudaEventElapsedTime(&ms, evs[2 * k], evs[2 * k + 1]) == cudaSuccess) {
+              c->timing.spmv_ms += ms;
+              c->timing.spmv_launches += 1;
+            }
+          }
+          in_flight = 1;
+          slot ^= 1;
+        }
+        if (in_flight == 0) {
+          in_flight = 1;
+          slot ^= 1;
+          continue;
+        }
+        const int prev = slot ^ 1;
+        cudaEventSynchronize(done[prev]);
+        const CgScalars* s = hs[prev];
+        if (!(s->stop || s->want_update)) {
+          slot ^= 1;
+          continue;
+        }
+        // act on the latest state
+        cudaEventSynchronize(done[slot]);
+        in_flight = 0;
+        cur = *hs[c->instrument ? prev : slot];
+        slot = 0;
       }
-      if (in_flight == 0) {
-        in_flight = 1;
-        slot ^= 1;
-        continue;
-      }
-      const int prev = slot ^ 1;
-      cudaEventSynchronize(done[prev]);
-      const CgScalars* s = hs[prev];
-      if (!(s->stop || s->want_update)) {
-        slot ^= 1;
-        continue;
-      }
-      // act on the latest state
-      cudaEventSynchronize(done[slot]);
-      in_flight = 0;
-      const CgScalars cur = *hs[c->instrument ? prev : slot];
-      slot = 0;
       if (cur.stop == 0 && !cur.want_update) continue;
       status = true_residual(R, false);
       if (status != UFC_STATUS_OK) break;

@@ -209,6 +209,8 @@ struct Ctx {
   Mg* mg = nullptr;
   double* z64 = nullptr;
 
+  double* res_zp = nullptr;  // [N][6] z and p records of the resident CG
+
   // cached CUDA graphs of CG batches
   cudaGraphExec_t cg_graph[kGraphSlots] = {};
   int cg_graph_batch[kGraphSlots] = {};
@@ -276,6 +278,10 @@ int pcg_solve(Ctx* c, const double* b, double* x, const ufc_solver_algo* algo, u
 int pcg_solve_block(Ctx* c, int nrhs, const double* B, double* X, const ufc_solver_algo* algo,
                     ufc_solver_state* st);
 void release_graphs(Ctx* c);
+
+// resident.cu
+bool cg_resident_fits(const Ctx* c);  // small enough for all iterations in one kernel
+int cg_resident(Ctx* c, const double* dinv, int chunk);
 
 // device memory helper
 template <class T>
