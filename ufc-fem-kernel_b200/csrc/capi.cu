@@ -148,6 +148,7 @@ void free_all(Ctx* c) {
   dfree(&c->sig_n); dfree(&c->epeq_n); dfree(&c->epl_n); dfree(&c->sig_t); dfree(&c->epeq_t); dfree(&c->epl_t);
   dfree(&c->Dt);
   dfree(&c->res_zp);
+  dfree(&c->fe);
 }
 
 int alloc_state(Ctx* c) {

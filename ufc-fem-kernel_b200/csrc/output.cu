@@ -8,9 +8,9 @@
 //                     PH_Elem_C3D8_EvalVonMises (:2768-2780)
 //   reactions         constrained rows of R = F_ext - F_int, RT_Asm_ComputeResidual (RT_Asm_Solv.f90:1311-1426)
 //
-// Both scatters (face loads into nodal forces, element extrapolations into
-// nodal sums) run per element colour, so no two threads of a launch touch the
-// same node and the sums are deterministic without atomics.
+// The scatter of face loads into nodal forces runs per element colour, so no two
+// threads of a launch touch the same node and the sums are deterministic without
+// atomics; nodal stresses are summed node by node.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -111,68 +111,6 @@ __global__ void k_face_load(int32_t nf, const int32_t* __restrict__ idx, const i
     for (int i = 0; i < 3; ++i) f[(int64_t)nd[a] * 3 + i] += F[a][i];
 }
 
-// Extrapolation from the 2x2x2 Gauss points to node a: the inverse of the
-// interpolation matrix A(ip, a) = N_a(gauss point ip), which factors into 1-D
-// inverses: E(a, ip) = prod_d (1 + sqrt(3) s_a,d s_ip,d) / 2.
-__device__ __forceinline__ double extrap(int a, int ip) {
-  const double r3 = 1.7320508075688772935;
-  double v = 1.0;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const double sip = ((ip >> d) & 1) ? 1.0 : -1.0;
-    v *= 0.5 * (1.0 + r3 * (double)node_sign(a, d) * sip);
-  }
-  return v;
-}
-
-// One thread per element of this colour: nodal values of the element's
-// Gauss-point stress added to the node sums.
-__global__ void k_extrap_scatter(const int32_t* __restrict__ el, int32_t ne, const int32_t* __restrict__ conn,
-                                 const double* __restrict__ sig_gp, double* __restrict__ sum,
-                                 int32_t* __restrict__ cnt) {
-  const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ne) return;
-  const int64_t e = el[t];
-  double s[8][6];
-#pragma unroll
-  for (int ip = 0; ip < 8; ++ip)
-#pragma unroll
-    for (int c = 0; c < 6; ++c) s[ip][c] = sig_gp[(e * 8 + ip) * 6 + c];
-#pragma unroll 1
-  for (int a = 0; a < 8; ++a) {
-    const int64_t nd = conn[e * 8 + a];
-    double v[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll
-    for (int ip = 0; ip < 8; ++ip) {
-      const double w = extrap(a, ip);
-#pragma unroll
-      for (int c = 0; c < 6; ++c) v[c] += w * s[ip][c];
-    }
-#pragma unroll
-    for (int c = 0; c < 6; ++c) sum[nd * 6 + c] += v[c];
-    cnt[nd] += 1;
-  }
-}
-
-__global__ void k_nodal_finish(int32_t N, const double* __restrict__ sum, const int32_t* __restrict__ cnt,
-                               double* __restrict__ sig, double* __restrict__ vm) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const double w = cnt[i] > 0 ? 1.0 / (double)cnt[i] : 0.0;
-  double s[6];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) s[c] = sum[i * 6 + c] * w;
-  if (sig)
-#pragma unroll
-    for (int c = 0; c < 6; ++c) sig[i * 6 + c] = s[c];
-  if (vm) {
-    const double p = (s[0] + s[1] + s[2]) / 3.0;
-    const double j2 = 0.5 * ((s[0] - p) * (s[0] - p) + (s[1] - p) * (s[1] - p) + (s[2] - p) * (s[2] - p)) +
-                      s[3] * s[3] + s[4] * s[4] + s[5] * s[5];
-    vm[i] = sqrt(3.0 * fmax(j2, 0.0));
-  }
-}
-
 __global__ void k_gather_rf(int32_t nfix, const int32_t* __restrict__ dofs, const double* __restrict__ fint,
                             const double* __restrict__ fext, double* __restrict__ rf) {
   const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -256,25 +194,9 @@ int face_loads(Ctx* c, int32_t n_faces, const int32_t* h_elem, const int32_t* h_
 }
 
 int stress_nodal(Ctx* c, const double* u, double* sig_node, double* vm_node) {
-  const int64_t G = (int64_t)c->E * 8;
-  AsyncBuf<double> sgp, sum;
-  AsyncBuf<int32_t> cnt;
-  UFC_TRY(async_alloc(c, sgp, G * 6));
-  UFC_TRY(async_alloc(c, sum, (int64_t)c->N * 6));
-  UFC_TRY(async_alloc(c, cnt, c->N));
-  UFC_TRY(stress_eval(c, u, sgp.p, nullptr));
-  UFC_CUDA(c, cudaMemsetAsync(sum.p, 0, sizeof(double) * c->N * 6, c->stream));
-  UFC_CUDA(c, cudaMemsetAsync(cnt.p, 0, sizeof(int32_t) * c->N, c->stream));
-  for (int col = 0; col < c->ncol; ++col) {
-    const int32_t ne = c->col_off[col + 1] - c->col_off[col];
-    if (ne == 0) continue;
-    k_extrap_scatter<<<grid_for(ne, 128), 128, 0, c->stream>>>(c->col_elems + c->col_off[col], ne, c->conn, sgp.p,
-                                                               sum.p, cnt.p);
-    UFC_CUDA(c, cudaGetLastError());
-  }
-  k_nodal_finish<<<grid_for(c->N, 256), 256, 0, c->stream>>>(c->N, sum.p, cnt.p, sig_node, vm_node);
-  UFC_CUDA(c, cudaGetLastError());
-  return UFC_STATUS_OK;
+  AsyncBuf<double> fs;
+  UFC_TRY(async_alloc(c, fs, (int64_t)c->E * 48));
+  return stress_at_nodes(c, u, fs.p, sig_node, vm_node);
 }
 
 int reactions(Ctx* c, const double* u, const double* f_ext, double* rf) {

@@ -194,6 +194,7 @@ struct Ctx {
   int32_t* dev_err = nullptr;
   int32_t* h_err = nullptr;     // pinned
 
+  double* fe = nullptr;  // [E][8][3] element forces of the matrix-free operators
   // Newton work vectors
   double *nr_fint = nullptr, *nr_R = nullptr, *nr_du = nullptr, *nr_dc = nullptr;
 
@@ -239,7 +240,7 @@ int export_csr(Ctx* c, const ufc_csr_export_arg* a);
 // c3d8.cu
 int element_lame(Ctx* c);  // Lame constants of the current material into c->lame
 int assemble(Ctx* c, int build, double* elapsed_ms);
-int apply_fp64(Ctx* c, const double* x, double* y, bool masked);  // y = K x matrix-free, FP64
+int apply_fp64(Ctx* c, const double* x, double* y);  // y = K x matrix-free, FP64, not eliminated
 int apply_fp64_eliminated(Ctx* c, const double* x, double* y);    // eliminated operator incl. identity rows
 int nr_norms(Ctx* c, const double* fext, const double* fint, double* R);  // R = fext - fint (free), norms
 int compute_fint(Ctx* c, const double* u, double* fint, bool update_state);
@@ -248,6 +249,7 @@ int mat_update_batch(Ctx* c, const ufc_mat_update_arg* a, const double* props, c
                      const double* dstrain, const double* sdv_n, double* stress, double* sdv, double* ddsdde,
                      int32_t* yielded);
 int stress_eval(Ctx* c, const double* u, double* sig, double* vm);
+int stress_at_nodes(Ctx* c, const double* u, double* fs, double* sig, double* vm);  // fs: [E][8][6] scratch
 int adjoint_sens(Ctx* c, int nrhs, const double* U, const double* L, double* g);
 
 // mg.cu
