@@ -1041,6 +1041,7 @@ void mg_release_graph(Ctx* c) {
 
 void mg_free(Ctx* c) {
   if (!c->mg) return;
+  cudaStreamSynchronize(c->stream);  // the levels' own contexts free in order of their streams, not of this one
   for (auto& L : c->mg->lv) free_level(L);
   dfree(&c->mg->dnorm);
   dfree(&c->mg->gj_flag);

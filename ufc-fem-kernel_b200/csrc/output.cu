@@ -122,17 +122,12 @@ __global__ void k_gather_rf(int32_t nfix, const int32_t* __restrict__ dofs, cons
 template <class T>
 struct AsyncBuf {
   T* p = nullptr;
-  cudaStream_t s = nullptr;
-  ~AsyncBuf() {
-    if (p) cudaFreeAsync(p, s);
-  }
+  ~AsyncBuf() { dfree(&p); }
 };
 
 template <class T>
 int async_alloc(Ctx* c, AsyncBuf<T>& b, int64_t count) {
-  b.s = c->stream;
-  UFC_CUDA(c, cudaMallocAsync((void**)&b.p, sizeof(T) * (size_t)std::max<int64_t>(count, 1), c->stream));
-  return UFC_STATUS_OK;
+  return dalloc(c, &b.p, count);
 }
 
 }  // namespace

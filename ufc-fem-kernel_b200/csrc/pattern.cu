@@ -538,9 +538,9 @@ int scan_exclusive(Ctx* c, const T* in, T* out, int64_t n) {
   size_t bytes = 0;
   UFC_CUDA(c, cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, (int)n, c->stream));
   void* tmp = nullptr;
-  UFC_CUDA(c, cudaMallocAsync(&tmp, bytes, c->stream));
+  UFC_CUDA(c, pool_alloc(c, &tmp, bytes));
   cudaError_t e = cub::DeviceScan::ExclusiveSum(tmp, bytes, in, out, (int)n, c->stream);
-  cudaFreeAsync(tmp, c->stream);
+  pool_free(tmp);
   if (e != cudaSuccess) return cuda_fail(c, e, "cub::DeviceScan::ExclusiveSum");
   return UFC_STATUS_OK;
 }

@@ -285,25 +285,29 @@ void release_graphs(Ctx* c);
 bool cg_resident_fits(const Ctx* c);  // small enough for all iterations in one kernel
 int cg_resident(Ctx* c, const double* dinv, int chunk);
 
-// device memory helper
+// Device memory: every array of a context and every temporary comes from one
+// stream-ordered pool per device (capi.cu), in stream order of the context.
+cudaError_t pool_alloc(Ctx* c, void** p, size_t bytes);
+void pool_free(void* p);  // in order on the stream of the API call being served
+
 template <class T>
 int dalloc(Ctx* c, T** p, int64_t count) {
   if (*p) {
-    cudaFree(*p);
+    pool_free(*p);
     *p = nullptr;
   }
   if (count <= 0) count = 1;
-  cudaError_t e = cudaMalloc((void**)p, sizeof(T) * (size_t)count);
+  cudaError_t e = pool_alloc(c, (void**)p, sizeof(T) * (size_t)count);
   if (e != cudaSuccess) {
     *p = nullptr;
-    return cuda_fail(c, e, "cudaMalloc");
+    return cuda_fail(c, e, "device allocation");
   }
   return UFC_STATUS_OK;
 }
 
 template <class T>
 void dfree(T** p) {
-  if (*p) cudaFree(*p);
+  if (*p) pool_free(*p);
   *p = nullptr;
 }
 
