@@ -66,8 +66,7 @@ __global__ void __launch_bounds__(kAsmWarps * 32)
                     const double* __restrict__ lame, const double* __restrict__ Dt, const int32_t* __restrict__ slot,
                     const int64_t* __restrict__ sptr, const int32_t* __restrict__ scol,
                     const int32_t* __restrict__ dpos, const uint8_t* __restrict__ fixed, int stride,
-                    T* __restrict__ val, T* __restrict__ dinv, float* __restrict__ val_r, float* __restrict__ dinv_r,
-                    int32_t* __restrict__ err) {
+                    const RowOutputs<T> to, int32_t* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char asm_smem[];
   using Warp = AsmWarp<T, kTangent>;
   Warp* wsm = reinterpret_cast<Warp*>(asm_smem);
@@ -240,7 +239,7 @@ __global__ void __launch_bounds__(kAsmWarps * 32)
   if (bad) atomicOr(err, (int)kDevBadJacobian);
   __syncthreads();
 
-  out.write(len, scol, fixed, acc, stride, val, dinv, val_r, dinv_r);
+  out.write(len, scol, fixed, acc, stride, to);
 }
 
 // The linear-elastic assembly with one thread per (block row, element): the
@@ -277,8 +276,7 @@ __global__ void __launch_bounds__(kIsoThreads, 2)
                    const double* __restrict__ lame, const int32_t* __restrict__ slot,
                    const int64_t* __restrict__ sptr, const int32_t* __restrict__ scol,
                    const int32_t* __restrict__ dpos, const uint8_t* __restrict__ fixed, int stride,
-                   T* __restrict__ val, T* __restrict__ dinv, float* __restrict__ val_r, float* __restrict__ dinv_r,
-                   int32_t* __restrict__ err) {
+                   const RowOutputs<T> to, int32_t* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char asm_smem[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* xs = reinterpret_cast<double*>(asm_smem) + w * (2 * 24 * 32) + lane;
@@ -437,7 +435,7 @@ __global__ void __launch_bounds__(kIsoThreads, 2)
   }
   if (bad) atomicOr(err, (int)kDevBadJacobian);
   __syncthreads();
-  out.write(len, scol, fixed, acc, stride, val, dinv, val_r, dinv_r);
+  out.write(len, scol, fixed, acc, stride, to);
 }
 
 // Lame constants of every element, [E][2].
@@ -745,7 +743,7 @@ int element_lame(Ctx* c) {
 }
 
 template <typename T, bool kTangent>
-static int launch_assemble(Ctx* c, T* val, T* dinv, float* val_r, float* dinv_r) {
+static int launch_assemble(Ctx* c, const RowOutputs<T>& to) {
   const int stride = (9 * c->max_row_blocks) | 1;  // odd: the rows of an entry lie in different banks
   if constexpr (!kTangent) {
     // while the slice's accumulators fit in shared memory
@@ -754,7 +752,7 @@ static int launch_assemble(Ctx* c, T* val, T* dinv, float* val_r, float* dinv_r)
       UFC_CUDA(c, cudaFuncSetAttribute(k_assemble_iso<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
       k_assemble_iso<T><<<(int)c->nslices, kIsoThreads, bytes, c->stream>>>(
           c->N, c->nptr, c->nelem, c->coords, c->conn, c->lame, c->slot, c->slice_ptr, c->sell_col, c->dpos, c->fixed,
-          stride, val, dinv, val_r, dinv_r, c->dev_err);
+          stride, to, c->dev_err);
       UFC_CUDA(c, cudaGetLastError());
       return UFC_STATUS_OK;
     }
@@ -763,7 +761,7 @@ static int launch_assemble(Ctx* c, T* val, T* dinv, float* val_r, float* dinv_r)
   UFC_CUDA(c, cudaFuncSetAttribute(k_assemble_rows<T, kTangent>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   k_assemble_rows<T, kTangent><<<(int)(2 * c->nslices), kAsmWarps * 32, bytes, c->stream>>>(
       c->N, c->nptr, c->nelem, c->coords, c->conn, c->lame, c->Dt, c->slot, c->slice_ptr, c->sell_col, c->dpos,
-      c->fixed, stride, val, dinv, val_r, dinv_r, c->dev_err);
+      c->fixed, stride, to, c->dev_err);
   UFC_CUDA(c, cudaGetLastError());
   return UFC_STATUS_OK;
 }
@@ -799,19 +797,35 @@ int assemble(Ctx* c, int build, double* elapsed_ms) {
     if (!c->dinv32) UFC_TRY(dalloc(c, &c->dinv32, c->n));
   }
   if (build & UFC_BUILD_FP64) {
-    // with `rounded` the FP32 values are the FP64 values rounded to nearest (Dirichlet rows included)
-    float *vr = rounded ? c->val32 : nullptr, *dr = rounded ? c->dinv32 : nullptr;
+    RowOutputs<double> to;
+    to.val = c->val64;
+    to.dinv = c->dinv64;
+    if (rounded) {  // the FP64 values rounded to nearest (Dirichlet rows included)
+      to.val_r = c->val32;
+      to.dinv_r = c->dinv32;
+    }
+    if (sym) {
+      UFC_TRY(alloc_symmetric(c, sym32));
+      to.uptr = c->uptr;
+      to.sval = c->sval64;
+      if (sym32) to.sval_r = c->sval32;
+    }
     if (tangent)
-      UFC_TRY((launch_assemble<double, true>(c, c->val64, c->dinv64, vr, dr)));
+      UFC_TRY((launch_assemble<double, true>(c, to)));
     else
-      UFC_TRY((launch_assemble<double, false>(c, c->val64, c->dinv64, vr, dr)));
+      UFC_TRY((launch_assemble<double, false>(c, to)));
+    c->has_sval64 = sym;
+    c->has_sval32 = sym32;
     c->has_val64 = true;
   }
   if (build & UFC_BUILD_FP32) {
+    RowOutputs<float> to;
+    to.val = c->val32;
+    to.dinv = c->dinv32;
     if (tangent)
-      UFC_TRY((launch_assemble<float, true>(c, c->val32, c->dinv32, nullptr, nullptr)));
+      UFC_TRY((launch_assemble<float, true>(c, to)));
     else
-      UFC_TRY((launch_assemble<float, false>(c, c->val32, c->dinv32, nullptr, nullptr)));
+      UFC_TRY((launch_assemble<float, false>(c, to)));
     c->has_val32 = true;
   }
   if (rounded) {
@@ -821,7 +835,6 @@ int assemble(Ctx* c, int build, double* elapsed_ms) {
     c->has_val32 = true;
     c->val32_diff = diff;
   }
-  if (sym) UFC_TRY(pack_symmetric(c, true, sym32));
   UFC_CUDA(c, cudaEventRecord(e1, c->stream));
   UFC_CUDA(c, cudaEventSynchronize(e1));
   float ms = 0.f;

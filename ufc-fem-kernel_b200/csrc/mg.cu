@@ -328,8 +328,7 @@ __global__ void __launch_bounds__(kMgRowThreads)
     k_mg_rows(int32_t N, const int32_t* __restrict__ nptr, const int32_t* __restrict__ nelem,
               const double* __restrict__ ke, const int32_t* __restrict__ slot, const int64_t* __restrict__ sptr,
               const int32_t* __restrict__ scol, const int32_t* __restrict__ dpos, const uint8_t* __restrict__ fixed,
-              int stride, double* __restrict__ val, double* __restrict__ dinv, float* __restrict__ val_r,
-              float* __restrict__ dinv_r) {
+              int stride, const RowOutputs<double> to) {
   extern __shared__ double mg_acc[];  // [row][stride]
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 7;
   const int64_t s = blockIdx.x >> 1;
@@ -359,7 +358,7 @@ __global__ void __launch_bounds__(kMgRowThreads)
     __syncwarp();  // the lanes of a row meet again at the same entries
   }
   __syncthreads();
-  out.write(len, scol, fixed, mg_acc, stride, val, dinv, val_r, dinv_r);
+  out.write(len, scol, fixed, mg_acc, stride, to);
 }
 
 // b = P^T r_f and d = D^-1 b / theta (the coarse smoother's first step): one
@@ -1110,9 +1109,13 @@ int mg_numeric(Ctx* c) {
     const int stride = (9 * lc->max_row_blocks) | 1;
     const int bytes = (int)sizeof(double) * kMgRows * stride;
     UFC_CUDA(c, cudaFuncSetAttribute(k_mg_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    RowOutputs<double> to;
+    to.val = lc->val64;
+    to.dinv = lc->dinv64;
+    to.val_r = L.val32;
+    to.dinv_r = L.dinv32;
     k_mg_rows<<<(int)(2 * lc->nslices), kMgRowThreads, bytes, c->stream>>>(
-        lc->N, lc->nptr, lc->nelem, L.ke, lc->slot, lc->slice_ptr, lc->sell_col, lc->dpos, lc->fixed, stride,
-        lc->val64, lc->dinv64, L.val32, L.dinv32);
+        lc->N, lc->nptr, lc->nelem, L.ke, lc->slot, lc->slice_ptr, lc->sell_col, lc->dpos, lc->fixed, stride, to);
     UFC_CUDA(c, cudaGetLastError());
     lc->has_val64 = true;
   }

@@ -451,23 +451,6 @@ __global__ void k_full_codes(int32_t N, int64_t nslices, const int64_t* __restri
   }
 }
 
-// Copy the upper blocks of the full SELL values into the symmetric storage.
-template <typename TO>
-__global__ void k_sym_pack(int32_t N, const int64_t* __restrict__ sptr, const int64_t* __restrict__ uptr,
-                           const int32_t* __restrict__ brow, const int32_t* __restrict__ lcnt,
-                           const double* __restrict__ v64, TO* __restrict__ out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const int64_t s = i / kSlice, t = i % kSlice;
-  const int32_t nl = lcnt[i], nu = brow[i + 1] - brow[i] - nl;
-  for (int32_t j = 0; j < nu; ++j) {
-    const int64_t src = sptr[s] + (int64_t)(nl + j) * kSlice + t;
-    const int64_t dst = uptr[s] + (int64_t)j * kSlice + t;
-#pragma unroll
-    for (int c = 0; c < 9; ++c) out[spos<TO>(dst, c)] = (TO)v64[vpos(src, c)];
-  }
-}
-
 // Scalar CSR export from the block pattern, one thread per (block row, entry).
 template <typename TV>
 __global__ void k_export(int32_t N, const int32_t* __restrict__ brow, const int32_t* __restrict__ bcol,
@@ -954,29 +937,22 @@ int build_sym_pattern(Ctx* c) {
   return build_sym_codes(c);
 }
 
-int pack_symmetric(Ctx* c, bool fp64, bool fp32) {
-  if (!c->has_val64) return fail(c, UFC_STATUS_INVALID, "symmetric storage: FP64 values not assembled");
+// The arrays of the symmetric storage; the assembly fills them.
+int alloc_symmetric(Ctx* c, bool fp32) {
   bool moved = !c->has_sym_pattern;  // arrays that captured graphs read
   UFC_TRY(build_sym_pattern(c));
-  // stored blocks plus one zero slice that padded lower references point at
+  // stored blocks plus one zero slice that padded lower references point at;
+  // padding stays zero from here on
   const int64_t nv = (c->s_ublocks + kSlice) * 9;
-  if (fp64) {
-    moved |= !c->sval64;
-    if (!c->sval64) UFC_TRY(dalloc(c, &c->sval64, nv));
+  if (!c->sval64) {
+    moved = true;
+    UFC_TRY(dalloc(c, &c->sval64, nv));
     UFC_CUDA(c, cudaMemsetAsync(c->sval64, 0, sizeof(double) * nv, c->stream));
-    k_sym_pack<double><<<grid_for(c->N, 128), 128, 0, c->stream>>>(c->N, c->slice_ptr, c->uptr, c->brow, c->s_lcnt,
-                                                                   c->val64, c->sval64);
-    UFC_CUDA(c, cudaGetLastError());
-    c->has_sval64 = true;
   }
-  if (fp32) {
-    moved |= !c->sval32;
-    if (!c->sval32) UFC_TRY(dalloc(c, &c->sval32, nv));
+  if (fp32 && !c->sval32) {
+    moved = true;
+    UFC_TRY(dalloc(c, &c->sval32, nv));
     UFC_CUDA(c, cudaMemsetAsync(c->sval32, 0, sizeof(float) * nv, c->stream));
-    k_sym_pack<float><<<grid_for(c->N, 128), 128, 0, c->stream>>>(c->N, c->slice_ptr, c->uptr, c->brow, c->s_lcnt,
-                                                                  c->val64, c->sval32);
-    UFC_CUDA(c, cudaGetLastError());
-    c->has_sval32 = true;
   }
   if (moved) release_graphs(c);
   return UFC_STATUS_OK;

@@ -375,7 +375,7 @@ int get_graph(const Run& R, const Vecs<TV, TX>& V, int batch, cudaGraphExec_t* o
   // (symmetric or full), the SpMV form (FP32 difference form, coded indices)
   // or the sizes baked into their launches (DOFs, slices) change; a reassembly
   // into the same arrays keeps them.  The vector and pattern buffers are not in
-  // the key: ensure_vectors, build_sym_pattern and pack_symmetric, which
+  // the key: ensure_vectors, build_sym_pattern and alloc_symmetric, which
   // reallocate them, release the graphs themselves.
   const void* key = (const void*)V.dinv;
   const void* val = (const void*)V.val;

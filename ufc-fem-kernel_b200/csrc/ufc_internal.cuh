@@ -234,7 +234,7 @@ int build_pattern(Ctx* c);
 int build_sym_pattern(Ctx* c);
 int build_sym_codes(Ctx* c);
 int build_full_codes(Ctx* c);
-int pack_symmetric(Ctx* c, bool fp64, bool fp32);  // full SELL values -> symmetric SpMV copies
+int alloc_symmetric(Ctx* c, bool fp32);  // arrays of the symmetric SpMV copies, filled by the assembly
 int export_csr(Ctx* c, const ufc_csr_export_arg* a);
 
 // c3d8.cu
