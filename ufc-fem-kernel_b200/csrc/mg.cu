@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(kBlk)
                   const double* __restrict__ coef, CgScalars* __restrict__ scal,
                   const double* __restrict__ pq_partials, int nb, double* __restrict__ partials) {
   pdl_enter();
-  if (scal->stop) return;
+  if (any_in_block(scal->stop != 0)) return;  // (block 0 may set it)
   double pq[1];
   sum_partials<1>(pq_partials, nb, pq);
   if (!(fabs(pq[0]) > 1e-300) || !isfinite(pq[0])) {
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(kBlk)
     k_mgcg_pupdate(int64_t n, const double* __restrict__ z, double* __restrict__ p, CgScalars* __restrict__ scal,
                    const double* __restrict__ partials, int nb) {
   pdl_enter();
-  if (scal->stop) return;
+  if (any_in_block(scal->stop != 0)) return;  // (block 0 may set it)
   double rz[1];
   sum_partials<1>(partials, nb, rz);
   const bool fresh = scal->fresh != 0, bad = !isfinite(rz[0]) || !(rz[0] > 0.0);  // M must stay positive definite

@@ -34,6 +34,12 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
   }
 }
 
+// A condition that another block may change while this one starts (block 0
+// records the end of a run in the kernel that finds it): true for the whole
+// block if any thread saw it.  Without that, the warps that saw it would leave
+// and the rest would sum without them and go on with the wrong total.
+__device__ __forceinline__ bool any_in_block(bool seen) { return __syncthreads_or(seen) != 0; }
+
 // The block's sums into partials[blockIdx.x * NV ..], for a following kernel to
 // add up (sum_partials): nothing waits for the store.
 template <int NV>

@@ -112,8 +112,9 @@ __global__ void __launch_bounds__(kVecBlock)
   };
   if (gid < n4) load(gid << 2);
   pdl_enter();
-  if (halted(scal)) return;
+  const bool seen = halted(scal);  // block 0 of this kernel may set it (breakdown)
   if (gid < n4) ld4_cg(q + (gid << 2), qv);
+  if (any_in_block(seen)) return;
   double pq[1];
   sum_partials<1>(pq_partials, nb, pq);
   const bool broken = !(fabs(pq[0]) > 1e-300) || !isfinite(pq[0]);
@@ -180,8 +181,9 @@ __global__ void __launch_bounds__(kVecBlock)
   };
   if (gid < n4) load(gid << 2);
   pdl_enter();
-  if (halted(scal)) return;
+  const bool seen = halted(scal);  // block 0 of this kernel may set it
   if (gid < n4) ld4_cg(r + (gid << 2), rv);
+  if (any_in_block(seen)) return;
   double b;
   if (nb > 0) {
     double tot[2];
