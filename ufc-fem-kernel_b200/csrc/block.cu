@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "c3d8_device.cuh"
+#include "pdl.cuh"
 #include "ufc_internal.cuh"
 
 namespace ufc {
@@ -47,6 +48,7 @@ struct BScalars {
   int32_t conv[kMaxRhs];    // recursive residual met the tolerance
   int32_t iters[kMaxRhs];
   int32_t iter, max_iter, stop, nr;
+  int32_t done;  // x holds the stopping iteration's update too
   uint32_t ticket[4];
 };
 
@@ -77,6 +79,37 @@ __device__ __forceinline__ void ld_g(const double* p, double (&o)[G]) {
       o[i + 1] = v.y;
     }
   }
+}
+
+// The same past L1, and as a line that leaves L2 first.
+template <int G>
+__device__ __forceinline__ void ldcg_g(const double* p, double (&o)[G]) {
+  if constexpr (G == 1) {
+    o[0] = __ldcg(p);
+  } else {
+    const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+    o[0] = v.x;
+    o[1] = v.y;
+  }
+}
+
+template <int G>
+__device__ __forceinline__ void ldcs_g(const double* p, double (&o)[G]) {
+  if constexpr (G == 1) {
+    o[0] = __ldcs(p);
+  } else {
+    const double2 v = __ldcs(reinterpret_cast<const double2*>(p));
+    o[0] = v.x;
+    o[1] = v.y;
+  }
+}
+
+template <int G>
+__device__ __forceinline__ void stcs_g(double* p, const double (&o)[G]) {
+  if constexpr (G == 1)
+    __stcs(p, o[0]);
+  else
+    __stcs(reinterpret_cast<double2*>(p), make_double2(o[0], o[1]));
 }
 
 template <int G>
@@ -132,6 +165,7 @@ __device__ bool rhs_grid_sum(double (&v)[NV][G], int tpr, int nr, double* __rest
   double acc[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q) acc[q] = 0.0;
+#pragma unroll 4
   for (int64_t b = gi; b < gridDim.x; b += groups)
 #pragma unroll
     for (int q = 0; q < NV; ++q) acc[q] += __ldcg(partials + (b * NV + q) * kMaxRhs + k);
@@ -151,6 +185,14 @@ __device__ bool rhs_grid_sum(double (&v)[NV][G], int tpr, int nr, double* __rest
   return false;
 }
 
+// The product after the stopping iteration marks x as complete (the direction
+// kernel adds alpha p to x, and must do so once more after the stop).
+__device__ __forceinline__ bool stopped(BScalars* s) {
+  if (!s->stop) return false;
+  if (blockIdx.x == 0 && threadIdx.x == 0) s->done = 1;
+  return true;
+}
+
 // y = K x for nr interleaved vectors (FP64 SELL values); MODE 1 also forms
 // p.q per rhs and alpha.  One warp task = 32/tpr rows of a slice.
 template <int G, int MODE>
@@ -158,7 +200,8 @@ __global__ void __launch_bounds__(kBlk, 4)
     k_bspmv(int32_t N, int64_t nslices, const int64_t* __restrict__ sptr, const int32_t* __restrict__ col,
             const double* __restrict__ val, const double* __restrict__ x, double* __restrict__ y, int nr, int tpr,
             BScalars* __restrict__ s, double* __restrict__ partials) {
-  if (MODE == 1 && s->stop) return;
+  pdl_enter();
+  if (MODE == 1 && stopped(s)) return;
   const int lane = threadIdx.x & 31;
   const int rpw = 32 / tpr;
   const int rl = lane / tpr;
@@ -299,7 +342,8 @@ __global__ void __launch_bounds__(kBlk, 3)
   constexpr int TPR = 32 / RPW;
   constexpr int D = kPipeD;
   extern __shared__ __align__(16) unsigned char bsm[];
-  if (MODE == 1 && s->stop) return;
+  pdl_enter();
+  if (MODE == 1 && stopped(s)) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int rl = lane / TPR;
   const int k0 = (lane % TPR) * 2;
@@ -431,6 +475,15 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                : "memory");
 }
 
+__device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, uint32_t bytes, uint64_t* bar,
+                                              uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::
+          "r"(smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
+      : "memory");
+}
+
 // The values of the full storage in tile order: half slice h of slice s holds
 // its len steps x 16 rows x kValPad doubles (the 9 of the block, row-major by
 // output component, then a zero) at 10 * sptr[s] + h * 160 * len, so that a
@@ -473,6 +526,8 @@ __global__ void k_tile_codes(int64_t rows, const uint8_t* __restrict__ code, con
 // consumer threads (8 per row, 2 rhs each) multiply from shared memory while
 // the next tile lands, then release the stage; a step costs them one byte
 // extract, one address and eight 16-byte shared loads besides the 18 FMAs.
+// Bound by what a tile moves from L2 (97 KB per 16 rows, 7 TB/s at 64x32x32):
+// eight consumer warps, each row's steps in two halves, changed nothing.
 // The same products in the same order as k_bspmv_pipe, so the same y.  Every
 // wait is bounded; a wait that gives up sets kDevTimeout.
 template <int MODE>
@@ -483,9 +538,9 @@ __global__ void __launch_bounds__(kTileBlk, 1)
                  int32_t* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char tsm[];
   __shared__ __align__(8) uint64_t full[2], empty[2];
-  if (MODE == 1 && s->stop) return;
   const size_t stage_bytes = tile_stage_bytes(T.nodes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool producer = warp == kTileCons / 32;
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
@@ -499,21 +554,48 @@ __global__ void __launch_bounds__(kTileBlk, 1)
   const int64_t tiles = nslices * 2;
   bool late = false;
   double dot[1][2] = {{0.0, 0.0}};
-  if (warp == kTileCons / 32) {
+  // the values are read once per product: they leave L2 to the vectors
+  uint64_t once = 0;
+  if (producer) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once));
+  auto issue_values = [&](int64_t tile, int st) {
+    unsigned char* sb = tsm + st * stage_bytes;
+    const int64_t sl = tile >> 1, base = sptr[sl];
+    const int h = (int)(tile & 1), len = (int)((sptr[sl + 1] - base) >> 5);
+    const uint32_t vbytes = (uint32_t)len * (16 * kValPad * 8);
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[st])),
+                 "r"((uint32_t)kStageCodes + vbytes)
+                 : "memory");
+    bulk_g2s(sb, tcode + (sl * kSlice + h * kTileRows) * 32, kStageCodes, &full[st]);
+    if (vbytes)
+      bulk_g2s_hint(sb + kStageCodes, tv + kValPad * base + (int64_t)h * (16 * kValPad) * len, vbytes, &full[st],
+                    once);
+  };
+  // the matrix is not written inside a chain: the first two tiles' values and
+  // codes come in behind the end of the kernel in front
+  if (producer && lane == 0)
+    for (int k = 0; k < 2 && blockIdx.x + k * (int64_t)gridDim.x < tiles; ++k)
+      issue_values(blockIdx.x + k * (int64_t)gridDim.x, k);
+  pdl_enter();
+  if (MODE == 1 && stopped(s)) {
+    if (producer && lane == 0)  // no block leaves while copies into its stages are in flight
+      for (int k = 0; k < 2 && blockIdx.x + k * (int64_t)gridDim.x < tiles; ++k) {
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[k])) : "memory");
+        if (!mbar_wait(&full[k], 0)) atomicOr(err, kDevTimeout);
+      }
+    return;
+  }
+  if (producer) {
     // producer: one lane issues the copies of the block's tiles in order
     if (lane == 0) {
       int k = 0;
       for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++k) {
         const int st = k & 1;
-        if (k >= 2 && !mbar_wait(&empty[st], (uint32_t)((k >> 1) - 1) & 1u)) late = true;
-        unsigned char* sb = tsm + st * stage_bytes;
-        const int64_t sl = tile >> 1;
-        const int h = (int)(tile & 1);
-        const int64_t r0 = sl * kSlice + h * kTileRows;
-        const int64_t base = sptr[sl];
-        const int len = (int)((sptr[sl + 1] - base) >> 5);
-        const uint32_t vbytes = (uint32_t)len * (16 * kValPad * 8);
-        uint32_t bytes = kStageCodes + vbytes;
+        if (k >= 2) {
+          if (!mbar_wait(&empty[st], (uint32_t)((k >> 1) - 1) & 1u)) late = true;
+          issue_values(tile, st);
+        }
+        const int64_t r0 = (tile >> 1) * kSlice + (tile & 1) * kTileRows;
+        uint32_t bytes = 0;
         for (int m = 0; m < T.nrange; ++m) {
           const int64_t lo = max(r0 + T.a[m], (int64_t)0), hi = min(r0 + T.a[m] + T.len[m], (int64_t)N);
           if (hi > lo) bytes += (uint32_t)(hi - lo) * kTileNodeBytes;
@@ -521,10 +603,7 @@ __global__ void __launch_bounds__(kTileBlk, 1)
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&full[st])),
                      "r"(bytes)
                      : "memory");
-        bulk_g2s(sb, tcode + r0 * 32, kStageCodes, &full[st]);
-        if (vbytes) bulk_g2s(sb + kStageCodes, tv + kValPad * base + (int64_t)h * (16 * kValPad) * len, vbytes,
-                             &full[st]);
-        double* xs = reinterpret_cast<double*>(sb + kStageCodes + kStageVals);
+        double* xs = reinterpret_cast<double*>(tsm + st * stage_bytes + kStageCodes + kStageVals);
         for (int m = 0; m < T.nrange; ++m) {
           // the runs clipped to the mesh; nodes outside it are never named by a code
           const int64_t lo = max(r0 + T.a[m], (int64_t)0), hi = min(r0 + T.a[m] + T.len[m], (int64_t)N);
@@ -619,42 +698,67 @@ __global__ void __launch_bounds__(kTileBlk, 1)
   }
 }
 
-// x += alpha p, r -= alpha q, then r.z and r.r per rhs, beta and the stop tests.
+// The two vector kernels read and write G right-hand sides of kVecU entries per
+// thread and pass, one pass's loads in flight together; what the kernel in
+// front does not write is loaded before waiting for it (past L1).  Blocks of
+// kVecBlk threads, two per SM: few enough that the last block's sum over the
+// blocks is short (with 8 blocks of 256 threads per SM it took 7 of the update's
+// 34 us at 64x32x32, 16 rhs).  Bound by memory; with x moved to the direction
+// kernel, the values marked as first to leave L2 and programmatic dependence
+// an iteration there takes 97 us (116 before; the product about 60 of it).
+constexpr int kVecBlk = 512;
+constexpr int kVecU = 2;
+
+// r -= alpha q, then r.z and r.r per rhs, beta and the stop tests.
 template <int G>
-__global__ void __launch_bounds__(kBlk)
-    k_bupdate(int64_t n, int nr, int tpr, const double* __restrict__ p, const double* __restrict__ q,
-              double* __restrict__ r, double* __restrict__ x, const double* __restrict__ dinv,
-              BScalars* __restrict__ s, double* __restrict__ partials) {
+__global__ void __launch_bounds__(kVecBlk, 2)
+    k_bupdate(int64_t n, int nr, int tpr, const double* __restrict__ q, double* __restrict__ r,
+              const double* __restrict__ dinv, BScalars* __restrict__ s, double* __restrict__ partials) {
+  constexpr int U = kVecU + 1;
+  const int64_t tid = (int64_t)blockIdx.x * kVecBlk + threadIdx.x, stride = (int64_t)gridDim.x * kVecBlk;
+  const int k0 = (int)(tid & (tpr - 1)) * G, sh = __ffs(tpr) - 1;
+  const int64_t groups = n * tpr;
+  double rv[U][G], d[U];
+  auto load_r = [&](int64_t i0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t idx = i0 + u * stride;
+      if (idx < groups) {
+        ldcg_g<G>(r + idx * G, rv[u]);
+        d[u] = dinv ? __ldg(dinv + (idx >> sh)) : 1.0;
+      }
+    }
+  };
+  load_r(tid);
+  pdl_enter();
   if (s->stop) return;
-  const int64_t tid = (int64_t)blockIdx.x * kBlk + threadIdx.x, stride = (int64_t)gridDim.x * kBlk;
-  const int k0 = (int)(tid % tpr) * G;
   double a[G];
 #pragma unroll
   for (int i = 0; i < G; ++i) a[i] = s->alpha[k0 + i];
   double v[2][G];
 #pragma unroll
   for (int i = 0; i < G; ++i) v[0][i] = v[1][i] = 0.0;
-  const int64_t groups = n * tpr;
-  for (int64_t idx = tid; idx < groups; idx += stride) {
-    const int64_t e = idx * G;
-    const double d = dinv ? __ldg(dinv + idx / tpr) : 1.0;
-    double pv[G], qv[G], rv[G], xv[G];
-    ldg_g<G>(p + e, pv);
-    ldg_g<G>(q + e, qv);
-    ld_g<G>(r + e, rv);
-    ld_g<G>(x + e, xv);
+  for (int64_t i0 = tid; i0 < groups;) {
+    double qv[U][G];
 #pragma unroll
-    for (int i = 0; i < G; ++i) {
-      xv[i] += a[i] * pv[i];
-      rv[i] -= a[i] * qv[i];
-      v[0][i] += rv[i] * (d * rv[i]);
-      v[1][i] += rv[i] * rv[i];
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * stride < groups) ldg_g<G>(q + (i0 + u * stride) * G, qv[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (i0 + u * stride >= groups) break;
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+        rv[u][i] -= a[i] * qv[u][i];
+        v[0][i] += rv[u][i] * (d[u] * rv[u][i]);
+        v[1][i] += rv[u][i] * rv[u][i];
+      }
+      st_g<G>(r + (i0 + u * stride) * G, rv[u]);
     }
-    st_g<G>(r + e, rv);
-    st_g<G>(x + e, xv);
+    i0 += U * stride;
+    if (i0 < groups) load_r(i0);
   }
   double tot[2];
-  if (rhs_grid_sum<G, 2>(v, tpr, nr, partials, &s->ticket[1], tot)) {
+  if (rhs_grid_sum<G, 2, kVecBlk>(v, tpr, nr, partials, &s->ticket[1], tot)) {
     const int kk = threadIdx.x;
     if (s->active[kk]) {
       s->rz_old[kk] = s->rz[kk];
@@ -681,34 +785,60 @@ __global__ void __launch_bounds__(kBlk)
   }
 }
 
-// p = D^-1 r + beta p for the rhs still active.
+// x += alpha p, and p = D^-1 r + beta p for the rhs still active: p is read
+// once for both.  x goes through L2 as first to leave; with the matrix values
+// so marked too, p, q and r of a mid-size problem stay in L2.
 template <int G>
-__global__ void __launch_bounds__(kBlk)
+__global__ void __launch_bounds__(kVecBlk, 2)
     k_bpupdate(int64_t n, int nr, int tpr, const double* __restrict__ r, const double* __restrict__ dinv,
-               double* __restrict__ p, const BScalars* __restrict__ s) {
-  if (s->stop) return;
-  const int64_t tid = (int64_t)blockIdx.x * kBlk + threadIdx.x, stride = (int64_t)gridDim.x * kBlk;
-  const int k0 = (int)(tid % tpr) * G;
-  double b[G];
+               double* __restrict__ p, double* __restrict__ x, const BScalars* __restrict__ s) {
+  constexpr int U = kVecU;
+  const int64_t tid = (int64_t)blockIdx.x * kVecBlk + threadIdx.x, stride = (int64_t)gridDim.x * kVecBlk;
+  const int k0 = (int)(tid & (tpr - 1)) * G, sh = __ffs(tpr) - 1;
+  const int64_t groups = n * tpr;
+  double pv[U][G], xv[U][G], d[U];
+  auto load_px = [&](int64_t i0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t idx = i0 + u * stride;
+      if (idx < groups) {
+        ldcg_g<G>(p + idx * G, pv[u]);
+        ldcs_g<G>(x + idx * G, xv[u]);
+        d[u] = dinv ? __ldg(dinv + (idx >> sh)) : 1.0;
+      }
+    }
+  };
+  load_px(tid);
+  pdl_enter();
+  if (s->done) return;
+  double a[G], b[G];
   bool act[G], any = false;
 #pragma unroll
   for (int i = 0; i < G; ++i) {
+    a[i] = s->alpha[k0 + i];
     b[i] = s->beta[k0 + i];
     act[i] = s->active[k0 + i] != 0;
-    any |= act[i];
+    any |= act[i] || a[i] != 0.0;
   }
   if (!any) return;
-  const int64_t groups = n * tpr;
-  for (int64_t idx = tid; idx < groups; idx += stride) {
-    const int64_t e = idx * G;
-    const double d = dinv ? __ldg(dinv + idx / tpr) : 1.0;
-    double rv[G], pv[G];
-    ldg_g<G>(r + e, rv);
-    ld_g<G>(p + e, pv);
+  for (int64_t i0 = tid; i0 < groups;) {
+    double rv[U][G];
 #pragma unroll
-    for (int i = 0; i < G; ++i)
-      if (act[i]) pv[i] = d * rv[i] + b[i] * pv[i];
-    st_g<G>(p + e, pv);
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * stride < groups) ldg_g<G>(r + (i0 + u * stride) * G, rv[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (i0 + u * stride >= groups) break;
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+        xv[u][i] += a[i] * pv[u][i];
+        if (act[i]) pv[u][i] = d[u] * rv[u][i] + b[i] * pv[u][i];
+      }
+      stcs_g<G>(x + (i0 + u * stride) * G, xv[u]);
+      st_g<G>(p + (i0 + u * stride) * G, pv[u]);
+    }
+    i0 += U * stride;
+    if (i0 < groups) load_px(i0);
   }
 }
 
@@ -796,7 +926,7 @@ struct BlockRun {
   double *bx, *xx, *rx, *px, *qx;
   BScalars* s;
   double* partials;
-  int g_spmv, g_vec;
+  int g_spmv, g_vec, g_upd;
   bool tile;  // k_bspmv_tile (16 rhs, coded full storage)
   BTile T;
   int g_tile;
@@ -837,8 +967,8 @@ void launch_bspmv_tile(const BlockRun& B, cudaStream_t st, int mode, const doubl
   Ctx* c = B.c;
   const size_t sm = 2 * tile_stage_bytes(B.T.nodes);
   if (mode == 1)
-    k_bspmv_tile<1><<<B.g_tile, kTileBlk, sm, st>>>(c->N, c->nslices, c->slice_ptr, B.tc, B.tv, B.T, x, y, B.s,
-                                                    B.partials, c->dev_err);
+    launch_pdl_smem(k_bspmv_tile<1>, B.g_tile, kTileBlk, sm, st, c->N, c->nslices, c->slice_ptr, B.tc, B.tv, B.T, x, y,
+                    B.s, B.partials, c->dev_err);
   else
     k_bspmv_tile<0><<<B.g_tile, kTileBlk, sm, st>>>(c->N, c->nslices, c->slice_ptr, B.tc, B.tv, B.T, x, y, B.s,
                                                     B.partials, c->dev_err);
@@ -856,8 +986,8 @@ void launch_bspmv_pipe(const BlockRun& B, cudaStream_t st, int mode, const doubl
   Ctx* c = B.c;
   constexpr size_t sm = bpipe_smem<RPW>();
   if (mode == 1)
-    k_bspmv_pipe<RPW, 1><<<B.g_spmv, kBlk, sm, st>>>(c->N, c->nslices, c->slice_ptr, c->sell_col, c->val64, x, y,
-                                                      B.nr, B.s, B.partials);
+    launch_pdl_smem(k_bspmv_pipe<RPW, 1>, B.g_spmv, kBlk, sm, st, c->N, c->nslices, c->slice_ptr, c->sell_col, c->val64,
+                    x, y, B.nr, B.s, B.partials);
   else
     k_bspmv_pipe<RPW, 0><<<B.g_spmv, kBlk, sm, st>>>(c->N, c->nslices, c->slice_ptr, c->sell_col, c->val64, x, y,
                                                       B.nr, B.s, B.partials);
@@ -903,8 +1033,8 @@ void launch_bspmv(const BlockRun& B, cudaStream_t st, int mode, const double* x,
     }
   }
   if (mode == 1)
-    k_bspmv<G, 1><<<B.g_spmv, kBlk, 0, st>>>(c->N, c->nslices, c->slice_ptr, c->sell_col, c->val64, x, y, B.nr,
-                                              B.tpr, B.s, B.partials);
+    launch_pdl(k_bspmv<G, 1>, B.g_spmv, kBlk, st, c->N, c->nslices, c->slice_ptr, c->sell_col, c->val64, x, y, B.nr,
+               B.tpr, B.s, B.partials);
   else
     k_bspmv<G, 0><<<B.g_spmv, kBlk, 0, st>>>(c->N, c->nslices, c->slice_ptr, c->sell_col, c->val64, x, y, B.nr,
                                               B.tpr, B.s, B.partials);
@@ -913,8 +1043,9 @@ void launch_bspmv(const BlockRun& B, cudaStream_t st, int mode, const double* x,
 template <int G>
 void launch_biteration(const BlockRun& B, cudaStream_t st) {
   launch_bspmv<G>(B, st, 1, B.px, B.qx);
-  k_bupdate<G><<<B.g_vec, kBlk, 0, st>>>(B.n, B.nr, B.tpr, B.px, B.qx, B.rx, B.xx, B.dinv, B.s, B.partials);
-  k_bpupdate<G><<<B.g_vec, kBlk, 0, st>>>(B.n, B.nr, B.tpr, B.rx, B.dinv, B.px, B.s);
+  launch_pdl(k_bupdate<G>, B.g_upd, kVecBlk, st, B.n, B.nr, B.tpr, (const double*)B.qx, B.rx, B.dinv, B.s, B.partials);
+  launch_pdl(k_bpupdate<G>, B.g_upd, kVecBlk, st, B.n, B.nr, B.tpr, (const double*)B.rx, B.dinv, B.px, B.xx,
+             (const BScalars*)B.s);
 }
 
 template <int G>
@@ -1047,6 +1178,7 @@ int pcg_solve_block(Ctx* c, int nrhs, const double* Bm, double* X, const ufc_sol
   B.g_tile = (int)std::min<int64_t>(2 * c->nslices, (int64_t)sm_count());
   if (B.tile) UFC_CUDA(c, prepare_tile(B.T));
   B.g_vec = grid_blocks(c->n * B.tpr);
+  B.g_upd = (int)std::min<int64_t>((c->n * B.tpr + kVecBlk - 1) / kVecBlk, 2 * (int64_t)sm_count());
   BScalars* hs = nullptr;
   int32_t* restart_dev = nullptr;
   auto cleanup = [&]() {
@@ -1076,7 +1208,7 @@ int pcg_solve_block(Ctx* c, int nrhs, const double* Bm, double* X, const ufc_sol
   BCUDA(cudaMemsetAsync(B.px, 0, sizeof(double) * B.nn, c->stream));
   BTRY(dalloc(c, &B.qx, B.nn));
   BTRY(dalloc(c, &B.s, 1));
-  BTRY(dalloc(c, &B.partials, (int64_t)std::max({B.g_spmv, B.g_vec, B.g_tile}) * kNvMax * kMaxRhs));
+  BTRY(dalloc(c, &B.partials, (int64_t)std::max({B.g_spmv, B.g_vec, B.g_upd, B.g_tile}) * kNvMax * kMaxRhs));
   BTRY(dalloc(c, &restart_dev, kMaxRhs));
   if (B.tile) {
     BTRY(dalloc(c, &B.tv, kValPad * c->sell_blocks));

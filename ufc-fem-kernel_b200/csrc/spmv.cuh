@@ -10,6 +10,7 @@
 #include <utility>
 
 #include "c3d8_device.cuh"
+#include "pdl.cuh"
 #include "reduce.cuh"
 #include "ufc_internal.cuh"
 
@@ -17,16 +18,6 @@ namespace ufc {
 namespace {
 
 constexpr int kSpmvBlock = 256;
-
-// Programmatic dependent launch between the kernels of a CG iteration: each
-// kernel lets its successor launch as soon as all of its own blocks are
-// running (launch_dependents), and waits for its predecessor's completion and
-// memory (wait) before it reads anything; both are no-ops for a kernel
-// launched without the attribute.
-__device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" :::);
-}
 
 // Stored steps that a warp of a split product loads (columns and values) before
 // it waits for the kernel in front: the matrix is not written inside a chain,
@@ -36,21 +27,6 @@ __device__ __forceinline__ void pdl_enter() {
 template <typename TV, int SPLIT>
 constexpr int split_ahead() {
   return SPLIT == 8 ? 4 : sizeof(TV) == 4 ? 4 : 2;
-}
-
-template <typename... K, typename... A>
-void launch_pdl(void (*kernel)(K...), int grid, int block, cudaStream_t st, A&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 // Products inside an iteration chain are launched with programmatic dependence.
