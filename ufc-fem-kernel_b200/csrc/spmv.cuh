@@ -421,11 +421,19 @@ __global__ void __launch_bounds__(kSpmvBlock)
 // two 16-byte loads when the warp starts, so the loop loads no indices at all.
 // Upper step j: column row + off[code], its x gathered at once.  Lower step j:
 // column row - off[code], and the block (col, row) at position
-// uptr[col / 32] + 32 rank + col % 32 of the upper storage (uptr from L1):
-// one dependent load (the slice start) instead of a streamed position and
-// column.  Same summation order as k_spmv_sym, so the same results bit for bit.
+// uptr[col / 32] + 32 rank + col % 32 of the upper storage.  The columns of a
+// slice at one offset lie in two slices, so a warp takes the starts of the (at
+// most 15) pairs into shared memory first: no step has a dependent global load.
+// Same summation order as k_spmv_sym, so the same results bit for bit.
+// Bound by the latency of the gathers (DRAM 53 %, FP32, 128x64x64).  FP32
+// values: two upper and two lower steps load together, without branches, in 3
+// blocks per SM (a padded upper step holds zeros itself, a padded lower step
+// takes the row's own diagonal block times 0): 198 -> 181 us at 192x96x96, 97.0
+// -> 94.5 us per CG iteration at 128x64x64.  FP64 values would fill the
+// registers that way (336 -> 479 us) and go step by step; the starts in shared
+// memory give 489 -> 476 and 160 -> 154 us per iteration.
 template <typename TV, typename TX, typename TA, class EPI>
-__global__ void __launch_bounds__(kSpmvBlock)
+__global__ void __launch_bounds__(kSpmvBlock, sizeof(TV) + sizeof(TX) == 8 ? 3 : 0)
     k_spmv_symc(int32_t N, int64_t nrows_pad, const int64_t* __restrict__ uptr, const int64_t* __restrict__ lptr,
                 const uint4* __restrict__ ucode, const uint4* __restrict__ lcode, SymOffsets tab,
                 const TV* __restrict__ val, const TX* __restrict__ x, EPI epi,
@@ -433,9 +441,11 @@ __global__ void __launch_bounds__(kSpmvBlock)
   pdl_enter();
   if (epi.halt()) return;
   __shared__ int32_t soff[16];
+  __shared__ int2 sbase[kSpmvBlock / 32][16];
   if (threadIdx.x < 16) soff[threadIdx.x] = tab.off[threadIdx.x];
   __syncthreads();
   double dot[1] = {0.0};
+  int2* sb = sbase[threadIdx.x >> 5];  // (block counts stay below 2^31: their FP64 values alone would be 154 GB)
   // FP64 values: a capped grid whose warps step through the slices (measured on
   // B200, 192x96x96: 400-402 us against 453 us with one slice per warp; FP32
   // values are faster with one slice per warp, 235 against 252-275 us)
@@ -453,6 +463,18 @@ __global__ void __launch_bounds__(kSpmvBlock)
     uint64_t ulo = uc.x | ((uint64_t)uc.y << 32), uhi = uc.z | ((uint64_t)uc.w << 32);
     uint64_t llo = lc.x | ((uint64_t)lc.y << 32), lhi = lc.z | ((uint64_t)lc.w << 32);
     const TV* uvp = val + 9 * ub;
+    __syncwarp();
+    if (t < 16) {
+      const int64_t sa = (32 * s - soff[t]) >> 5;
+      sb[t] = make_int2((int)__ldg(uptr + (sa < 0 ? 0 : sa)), (int)__ldg(uptr + (sa + 1 < 0 ? 0 : sa + 1)));
+    }
+    __syncwarp();
+    // first block of the slice of column row - off
+    auto slice_start = [&](unsigned code, int off) {
+      const int2 pb = sb[code];
+      const int sh = off & 31;
+      return (int64_t)(sh && t >= sh ? pb.y : pb.x);
+    };
     if (t == 0) {
       const int k1 = (sizeof(TV) == 8 ? 4 : 8) < ulen ? (sizeof(TV) == 8 ? 4 : 8) : ulen;
       if (k1 > 0)
@@ -482,8 +504,9 @@ __global__ void __launch_bounds__(kSpmvBlock)
       llo = (llo >> 8) | (lhi << 56);
       lhi >>= 8;
       if (b != 0xFFu) {
-        const int64_t cj = row - soff[b >> 4];
-        const int64_t P = __ldg(uptr + (cj >> 5)) + 32 * (int64_t)(b & 15u) + (cj & 31);
+        const int off = soff[b >> 4];
+        const int64_t cj = row - off;
+        const int64_t P = slice_start(b >> 4, off) + 32 * (int64_t)(b & 15u) + (cj & 31);
         const TA x0 = (TA)__ldg(x + 3 * cj), x1 = (TA)__ldg(x + 3 * cj + 1), x2 = (TA)__ldg(x + 3 * cj + 2);
         TV v[9];
         load_block(val + 9 * (P & ~int64_t(31)), (int)(P & 31), v);
@@ -494,12 +517,56 @@ __global__ void __launch_bounds__(kSpmvBlock)
     };
     const int mlen = ulen < llen ? ulen : llen;
     int j = 0;
+    if constexpr (sizeof(TV) + sizeof(TX) == 8) {
+      const int64_t rx = row < N ? row : 0;
 #pragma unroll 1
-    for (; j + 1 < mlen; j += 2) {
-      upper(j);
-      lower(j);
-      upper(j + 1);
-      lower(j + 1);
+      for (; j + 1 < mlen; j += 2) {
+        TV uv[2][9], lv[2][9];
+        TX ux[2][3], lx[2][3];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const unsigned code = (unsigned)(ulo & 0xFF), b = (unsigned)(llo & 0xFF);
+          ulo = (ulo >> 8) | (uhi << 56);
+          uhi >>= 8;
+          llo = (llo >> 8) | (lhi << 56);
+          lhi >>= 8;
+          const bool up = code != kSymCodes, low = b != 0xFFu;
+          const int off = low ? soff[b >> 4] : 0;
+          const int64_t cu = rx + (up ? soff[code] : 0), cl = rx - off;
+          const int64_t lstep = low ? slice_start(b >> 4, off) + 32 * (int64_t)(b & 15u) : ub;
+          load_block(uvp + 288 * (int64_t)(j + h), t, uv[h]);
+          load_block(val + 9 * lstep, (int)(cl & 31), lv[h]);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            ux[h][c] = __ldg(x + 3 * cu + c);
+            lx[h][c] = __ldg(x + 3 * cl + c);
+          }
+          if (!low) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) lx[h][c] = TX(0);
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const TV *u = uv[h], *v = lv[h];
+          TA x0 = (TA)ux[h][0], x1 = (TA)ux[h][1], x2 = (TA)ux[h][2];
+          a0 += (TA)u[0] * x0 + (TA)u[1] * x1 + (TA)u[2] * x2;
+          a1 += (TA)u[3] * x0 + (TA)u[4] * x1 + (TA)u[5] * x2;
+          a2 += (TA)u[6] * x0 + (TA)u[7] * x1 + (TA)u[8] * x2;
+          x0 = (TA)lx[h][0], x1 = (TA)lx[h][1], x2 = (TA)lx[h][2];
+          a0 += (TA)v[0] * x0 + (TA)v[3] * x1 + (TA)v[6] * x2;
+          a1 += (TA)v[1] * x0 + (TA)v[4] * x1 + (TA)v[7] * x2;
+          a2 += (TA)v[2] * x0 + (TA)v[5] * x1 + (TA)v[8] * x2;
+        }
+      }
+    } else {
+#pragma unroll 1
+      for (; j + 1 < mlen; j += 2) {
+        upper(j);
+        lower(j);
+        upper(j + 1);
+        lower(j + 1);
+      }
     }
     for (; j < mlen; ++j) {
       upper(j);
