@@ -809,8 +809,9 @@ int ufc_nr_increment(ufc_ctx* c, ufc_nr_arg* a) {
   // tangent rounded from its FP64 assembly, whose FP64 values give the
   // refinement residual
   if (lin.precision_mode != UFC_PRECISION_FP32_REFINE) lin.precision_mode = UFC_PRECISION_FP64;
-  const int build =
-      lin.precision_mode == UFC_PRECISION_FP64 ? UFC_BUILD_FP64 : (UFC_BUILD_FP64 | UFC_BUILD_FP32_ROUNDED);
+  int build = lin.precision_mode == UFC_PRECISION_FP64 ? UFC_BUILD_FP64 : (UFC_BUILD_FP64 | UFC_BUILD_FP32_ROUNDED);
+  if (lin.precision_mode == UFC_PRECISION_FP64 && tangent_symmetric(c, lin.precond_type == UFC_SOLV_PREC_MG))
+    build |= UFC_BUILD_SYMMETRIC;
   const int vg = std::min(grid_for(c->n, 256), 148 * 8);
   for (int it = 0; it < a->max_iterations; ++it) {
     UFC_TRY(compute_fint(c, c->u, c->nr_fint, true));

@@ -750,6 +750,32 @@ bool fp64_fits_l2(const Ctx* c) {
   return spmv_bytes(c, UFC_PRECISION_FP64) < (int64_t)l2 / 2;
 }
 
+// Whether the FP64 solves of a Newton increment take the symmetric storage of the
+// tangent: on a stencil-like numbering (on a random one the transposed blocks
+// are scattered reads), with Jacobi where the full values exceed half the L2,
+// with multigrid twice the L2.  Below, both forms come from L2 and the full one
+// reads no block twice.  Second increment of a J2 bar, full against symmetric,
+// ms: Jacobi 48x24x24 (59 MB) 26.9/26.5, 56x28x28 (93 MB) 40.0/37.0, 64x32x32
+// 58.4/52.7, 96x48x48 (456 MB) 311/206; multigrid 56x28x28 11.0/11.5, 64x32x32
+// (137 MB) 9.6/9.9, 96x48x48 25.5/19.6.  The first increment builds the
+// symmetric pattern, 2 ms at 64x32x32.
+// The storage is optional here, so it is taken only where device memory is
+// plentiful: a run that fits without it must not end for it.
+bool tangent_symmetric(Ctx* c, bool mg) {
+  int dev = 0, l2 = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess || l2 <= 0) return false;
+  const int64_t full = c->nnzb * 9 * 8;
+  if (!c->full_coded || full < (mg ? 2 * (int64_t)l2 : (int64_t)l2 / 2)) return false;
+  if (c->sval64) return true;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || (int64_t)free_b < 4 * full) return false;
+  if (alloc_symmetric(c, false) == UFC_STATUS_OK) return true;
+  cudaGetLastError();
+  c->err.clear();
+  return false;
+}
+
 int pcg_solve(Ctx* c, const double* b, double* x, const ufc_solver_algo* algo, ufc_solver_state* st) {
   if (!c->has_pattern) return fail(c, UFC_STATUS_INVALID, "ufc_pcg_solve: pattern not built");
   if (algo->method != UFC_SOLV_METHOD_CG) return fail(c, UFC_STATUS_UNSUPPORTED, "ufc_pcg_solve: method must be CG");
