@@ -4,6 +4,7 @@ the end of a graph of iterations, against the oracle's matrix and the
 single-right-hand-side solver."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 pytestmark = pytest.mark.gpu
 
@@ -57,4 +58,19 @@ def test_iteration_limit(pkg, nrhs, limit):
     # rounding at 1e-16 each, amplified by the vectors' decay, stay below 1e-9
     u, _ = m.solve(F[0], pkg.SolverAlgo(tolerance=1e-14, max_iter=limit), raise_on_not_converged=False)
     assert np.linalg.norm(u - X[0]) <= 1e-9 * np.linalg.norm(u)
+    m.close()
+
+
+@pytest.mark.parametrize("shape,nrhs", [((48, 24, 24), 8), ((64, 40, 32), 32)])
+def test_vectors_within_and_beyond_the_l2(pkg, shape, nrhs):
+    """p, q and r of 18 and 204 MB: either side of the direction kernel's rule."""
+    p = pkg.mesh.lognormal_cantilever(*shape, seed=8)
+    m = pkg.FemModel.from_problem(p)
+    m.assemble(pkg.BUILD_FP64)
+    F = _rhs(p, nrhs, 3)
+    X, st = m.solve_block(F, pkg.SolverAlgo(tolerance=1e-10))
+    rp, col, val, _ = m.csr_export(index_base=0)
+    K = sp.csr_matrix((val, col, rp), shape=(p.n_dof, p.n_dof))
+    for k in range(nrhs):
+        assert st[k].converged and np.linalg.norm(F[k] - K @ X[k]) <= 2e-10 * np.linalg.norm(F[k])
     m.close()

@@ -785,10 +785,12 @@ __global__ void __launch_bounds__(kVecBlk, 2)
   }
 }
 
-// x += alpha p, and p = D^-1 r + beta p for the rhs still active: p is read
-// once for both.  x goes through L2 as first to leave; with the matrix values
-// so marked too, p, q and r of a mid-size problem stay in L2.
-template <int G>
+// x += alpha p, and p = D^-1 r + beta p for the rhs still active: p is read once
+// for both.  kOnce: x goes through L2 as first to leave; with the matrix values
+// so marked too, p, q and r stay there if they fit.  16 rhs, us per iteration
+// with and without: 64x32x32 102.9/104.3, 96x48x48 (p, q, r 268 MB) 337/333,
+// 128x64x64 769/759.
+template <int G, bool kOnce>
 __global__ void __launch_bounds__(kVecBlk, 2)
     k_bpupdate(int64_t n, int nr, int tpr, const double* __restrict__ r, const double* __restrict__ dinv,
                double* __restrict__ p, double* __restrict__ x, const BScalars* __restrict__ s) {
@@ -803,7 +805,8 @@ __global__ void __launch_bounds__(kVecBlk, 2)
       const int64_t idx = i0 + u * stride;
       if (idx < groups) {
         ldcg_g<G>(p + idx * G, pv[u]);
-        ldcs_g<G>(x + idx * G, xv[u]);
+        if constexpr (kOnce) ldcs_g<G>(x + idx * G, xv[u]);
+        else ldcg_g<G>(x + idx * G, xv[u]);
         d[u] = dinv ? __ldg(dinv + (idx >> sh)) : 1.0;
       }
     }
@@ -834,7 +837,8 @@ __global__ void __launch_bounds__(kVecBlk, 2)
         xv[u][i] += a[i] * pv[u][i];
         if (act[i]) pv[u][i] = d[u] * rv[u][i] + b[i] * pv[u][i];
       }
-      stcs_g<G>(x + (i0 + u * stride) * G, xv[u]);
+      if constexpr (kOnce) stcs_g<G>(x + (i0 + u * stride) * G, xv[u]);
+      else st_g<G>(x + (i0 + u * stride) * G, xv[u]);
       st_g<G>(p + (i0 + u * stride) * G, pv[u]);
     }
     i0 += U * stride;
@@ -927,6 +931,7 @@ struct BlockRun {
   BScalars* s;
   double* partials;
   int g_spmv, g_vec, g_upd;
+  bool once;  // p, q and r fit the L2
   bool tile;  // k_bspmv_tile (16 rhs, coded full storage)
   BTile T;
   int g_tile;
@@ -1044,7 +1049,7 @@ template <int G>
 void launch_biteration(const BlockRun& B, cudaStream_t st) {
   launch_bspmv<G>(B, st, 1, B.px, B.qx);
   launch_pdl(k_bupdate<G>, B.g_upd, kVecBlk, st, B.n, B.nr, B.tpr, (const double*)B.qx, B.rx, B.dinv, B.s, B.partials);
-  launch_pdl(k_bpupdate<G>, B.g_upd, kVecBlk, st, B.n, B.nr, B.tpr, (const double*)B.rx, B.dinv, B.px, B.xx,
+  launch_pdl(B.once ? k_bpupdate<G, true> : k_bpupdate<G, false>, B.g_upd, kVecBlk, st, B.n, B.nr, B.tpr, (const double*)B.rx, B.dinv, B.px, B.xx,
              (const BScalars*)B.s);
 }
 
@@ -1173,6 +1178,9 @@ int pcg_solve_block(Ctx* c, int nrhs, const double* Bm, double* X, const ufc_sol
   B.nn = c->n * nr;
   B.dinv = algo->precond_type == UFC_SOLV_PREC_JACOBI ? c->dinv64 : nullptr;
   B.g_spmv = grid_blocks(c->nslices * B.tpr * 32);
+  int dev = 0, l2 = 0;
+  cudaGetDevice(&dev);
+  B.once = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) == cudaSuccess && 3 * 8 * B.nn <= (int64_t)l2;
   if (G == 2) UFC_CUDA(c, prepare_bspmv(B.tpr));
   B.tile = nr == kTileNr && make_tile(c, &B.T);
   B.g_tile = (int)std::min<int64_t>(2 * c->nslices, (int64_t)sm_count());
