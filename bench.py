@@ -795,10 +795,10 @@ def run_ours(args):
                      "with_storage_ms": build_ms,
                      "elements_per_s_fp32": p.n_elems / (asm32_ms / 1e3), "host_setup_s": setup_s},
         "roofline": {"bound": "hbm",
-                     "kernel": ("k_spmv_symc<float,float,float,kCg> (symmetric SELL-32 BSR3 SpMV, coded indices: "
+                     "kernel": ("k_spmv_symc<float,float,float,EpiCg> (symmetric SELL-32 BSR3 SpMV, coded indices: "
                                 "16 + 16 code bytes per row, + p.Ap)" if coded else
-                                "k_spmv_sym<float,float,float,kCg> (symmetric SELL-32 BSR3 SpMV + p.Ap)" if sym else
-                                "k_spmv<float,float,float,kCg> (SELL-32 BSR3 SpMV + p.Ap)"),
+                                "k_spmv_sym<float,float,float,EpiCg> (symmetric SELL-32 BSR3 SpMV + p.Ap)" if sym else
+                                "k_spmv<float,float,float,EpiCg> (SELL-32 BSR3 SpMV + p.Ap)"),
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "traffic": traffic,
                      "algorithmic_bytes_per_launch": tm["spmv_bytes"], "avg_launch_us": spmv_avg_s * 1e6,

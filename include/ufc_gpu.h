@@ -86,7 +86,7 @@ extern "C" {
 #define UFC_BUILD_FP32 2
 #define UFC_BUILD_FP32_ROUNDED 4
 #define UFC_BUILD_FP32_DIFF 8
-/* Also pack symmetric SpMV copies (upper-triangle blocks only; each row reads
+/* Also write symmetric SpMV copies (upper-triangle blocks only; each row reads
  * its lower blocks transposed from the rows that store them): FP64, and FP32
  * rounded from FP64 when an FP32 build is requested.  The solver and ufc_spmv
  * use them when present.  Implies UFC_BUILD_FP64. */
@@ -404,8 +404,8 @@ int ufc_load_faces(ufc_ctx* ctx, const ufc_face_load_arg* arg);
  * Gauss-point stress of each element extrapolated to its nodes with the
  * inverse of the Gauss-point interpolation matrix (PH_Elem_C3D8_GetExtrapMat /
  * PH_Elem_C3D8_MapToNode, PH_Elem_C3D8.f90:2782-2824, with N_a = (1/8)...),
- * then averaged over the elements that share the node (colour-ordered,
- * deterministic).  u as ufc_stress_eval; either output may be NULL. */
+ * then averaged over the elements that share the node (in ascending element
+ * order, deterministic).  u as ufc_stress_eval; either output may be NULL. */
 int ufc_stress_nodal(ufc_ctx* ctx, const double* u, double* stress_node, double* vm_node, int32_t mem);
 /* Reaction forces RF = F_int(u) - F_ext at the prescribed DOFs, in the order of
  * ufc_bc_desc (the constrained rows of R = F_ext - F_int of

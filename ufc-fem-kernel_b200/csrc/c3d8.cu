@@ -4,9 +4,8 @@
 //
 // Assembly is deterministic without floating-point atomics: the stiffness is
 // assembled by block rows, each value summed by one thread in ascending element
-// order and written once; the vector scatters process elements colour by colour
-// (no two elements of one colour share a node), so every entry receives its
-// contributions in the fixed colour order.
+// order and written once; element vectors (forces, nodal stresses) are written
+// per element node and summed by one thread per node in ascending element order.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -22,8 +22,8 @@
 // at set-up; the coarsest level is solved with its dense inverse (<= kDenseMax DOF)
 // or a high-degree Chebyshev polynomial.  Restriction and prolongation are
 // structured gathers, one thread per coarse or fine node, so they need no
-// atomics and are deterministic; the coarse matrices are assembled colour by
-// colour like the fine one.
+// atomics and are deterministic; the coarse matrices are assembled by block rows
+// like the fine one.
 //
 // Precision: the cycle runs in FP64, or (precision = UFC_PRECISION_FP32_REFINE)
 // in FP32 on values rounded from the FP64 operators, half the bytes; the PCG

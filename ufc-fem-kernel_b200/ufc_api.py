@@ -184,7 +184,7 @@ class PH_Element_Compute_Fe_Arg:
 def PH_Element_Compute_Ke(ctx: NM_Solver_Ctx, build=A.BUILD_FP64) -> ErrorStatusType:
     """Compute_Ke of every element with its scatter into the device CSR values
     (PH_Element_Compute_Ke_Arg, PH_Elem_Def.f90:331-341, called per element by
-    RT_Asm_Solv.f90:1883,1946): one batched launch set per colour."""
+    RT_Asm_Solv.f90:1883,1946): one batched launch over the block rows."""
     return _run("PH_Element_Compute_Ke", ctx.model.assemble, build)[1]
 
 
