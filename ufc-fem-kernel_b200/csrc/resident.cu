@@ -151,7 +151,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const ResArgs A)
 
   bool first = true;
   int done = 0;
-  __syncthreads();
+  // the first sum writes into the other CTAs' shared memory, which may not be
+  // touched before they have started
+  if constexpr (SYNC == kCluster)
+    cg::this_cluster().sync();
+  else
+    __syncthreads();
   while (done < A.chunk) {
     // direction: given on entry, then z + beta p
     if (!first && own)
