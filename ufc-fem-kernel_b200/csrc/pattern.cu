@@ -715,6 +715,7 @@ int build_pattern(Ctx* c) {
   dfree(&c->sval64); dfree(&c->sval32); dfree(&c->sym_ucode); dfree(&c->sym_lcode); dfree(&c->full_code);
   c->full_coded = false;
   c->has_sym_pattern = c->has_sval64 = c->has_sval32 = c->sym_coded = false;
+  c->res_ctas = -1;
   const int32_t N = c->N, E = c->E;
 
   // 1. node -> element adjacency on the device

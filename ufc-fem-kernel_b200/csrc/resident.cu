@@ -28,6 +28,7 @@
 #include <type_traits>
 
 #include "reduce.cuh"
+#include "resident_rule.h"
 #include "ufc_internal.cuh"
 
 namespace ufc {
@@ -38,8 +39,7 @@ namespace cg = cooperative_groups;
 
 constexpr int kResThreads = 512;
 constexpr int kResWarps = kResThreads / 32;
-constexpr int kResMaxRows1 = 5 * kSlice;   // rows of the one-CTA form
-constexpr int kResCluster = 16;            // CTAs of the cluster form (non-portable size)
+constexpr int kResMaxRows1 = (int)kOneCtaSlices * kSlice;  // rows of the one-CTA form
 
 enum ResSync { kOneCta = 0, kCluster = 1 };
 
@@ -275,17 +275,55 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const ResArgs A)
   }
 }
 
-// Largest systems of the two forms, in slices.
-constexpr int64_t kOneCtaSlices = 4;
-constexpr int64_t kClusterSlices = 48;
+// The launch of the form with g CTAs.
+struct ResLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  int32_t steps;
+  ResLaunch(const Ctx* c, int g) {
+    // no CTA has more steps than ceil(slices / CTAs) slices of the longest row
+    const int64_t most = (c->nslices + g - 1) / g * c->max_row_blocks;
+    steps = (int32_t)std::min<int64_t>(most, kResSmem / kStepBytes);
+    cfg.gridDim = dim3(g);
+    cfg.blockDim = dim3(kResThreads);
+    cfg.stream = c->stream;
+    cfg.dynamicSmemBytes = (size_t)steps * kStepBytes;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = g;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g > 1 ? 1 : 0;
+  }
+};
+
+template <int SYNC>
+cudaError_t allow_resident() {
+  const auto kernel = k_cg_resident<SYNC>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
+  if (e == cudaSuccess && SYNC == kCluster)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e;
+}
+
+bool cluster_placeable(const Ctx* c, int g) {
+  const ResLaunch L(c, g);
+  int n = 0;
+  cudaError_t e = allow_resident<kCluster>();
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, k_cg_resident<kCluster>, &L.cfg);
+  if (e != cudaSuccess) cudaGetLastError();  // not a failure of the solve: the chain of kernels takes over
+  return e == cudaSuccess && n > 0;
+}
 
 }  // namespace
 
-bool cg_resident_fits(const Ctx* c) { return c->nslices <= kClusterSlices; }
+int cg_resident_plan(Ctx* c) {
+  if (c->res_ctas < 0) c->res_ctas = resident_ctas(c->nslices, [c](int g) { return cluster_placeable(c, g); });
+  return c->res_ctas;
+}
 
 // At most `chunk` iterations from r64, p64 and the scalars, as the kernels of a
-// batch would leave them.
-int cg_resident(Ctx* c, const double* dinv, int chunk) {
+// batch would leave them, on the g CTAs of cg_resident_plan.
+int cg_resident(Ctx* c, const double* dinv, int chunk, int g) {
   ResArgs a{};
   a.N = c->N;
   a.nslices = (int32_t)c->nslices;
@@ -300,28 +338,15 @@ int cg_resident(Ctx* c, const double* dinv, int chunk) {
   a.zp = c->res_zp;
   a.scal = c->scal;
   a.chunk = chunk;
-  const bool cluster = c->nslices > kOneCtaSlices;
-  const int g = cluster ? (int)std::min<int64_t>(c->nslices, kResCluster) : 1;
-  // no CTA has more steps than ceil(slices / CTAs) slices of the longest row
-  const int64_t most = (c->nslices + g - 1) / g * c->max_row_blocks;
-  a.steps = (int32_t)std::min<int64_t>(most, kResSmem / kStepBytes);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(g);
-  cfg.blockDim = dim3(kResThreads);
-  cfg.stream = c->stream;
-  cfg.dynamicSmemBytes = (size_t)a.steps * kStepBytes;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = g;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = cluster ? 1 : 0;
-  const auto launch = [&](auto kernel) -> cudaError_t {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
-    if (e == cudaSuccess && cluster) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, kernel, a) : e;
-  };
-  UFC_CUDA(c, cluster ? launch(k_cg_resident<kCluster>) : launch(k_cg_resident<kOneCta>));
+  const ResLaunch L(c, g);
+  a.steps = L.steps;
+  if (g > 1) {
+    UFC_CUDA(c, allow_resident<kCluster>());
+    UFC_CUDA(c, cudaLaunchKernelEx(&L.cfg, k_cg_resident<kCluster>, a));
+  } else {
+    UFC_CUDA(c, allow_resident<kOneCta>());
+    UFC_CUDA(c, cudaLaunchKernelEx(&L.cfg, k_cg_resident<kOneCta>, a));
+  }
   c->launches += 1;
   return UFC_STATUS_OK;
 }

@@ -495,8 +495,8 @@ int pcg_run(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
     cudaGraphExec_t graph = nullptr;
     int64_t graph_launches = 0;
     // small FP64 systems: all iterations in one kernel (resident.cu)
-    bool resident = false;
-    if constexpr (sizeof(TV) == 8) resident = !c->instrument && cg_resident_fits(c);
+    int resident = 0;  // its CTAs
+    if constexpr (sizeof(TV) == 8) resident = c->instrument ? 0 : cg_resident_plan(c);
     if (!c->instrument && !resident) UFC_TRY((get_graph<TV, TX, TA>(R, V, batch, &graph, &graph_launches)));
     std::vector<cudaEvent_t> evs;
     if (c->instrument) {
@@ -521,7 +521,7 @@ int pcg_run(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
       CgScalars cur;
       if (resident) {
         if constexpr (sizeof(TV) == 8)
-          status = cg_resident(c, V.dinv, algo->check_every > 0 ? algo->check_every : kResidentChunk);
+          status = cg_resident(c, V.dinv, algo->check_every > 0 ? algo->check_every : kResidentChunk, resident);
         if (status == UFC_STATUS_OK) status = read_scalars(c);
         if (status != UFC_STATUS_OK) break;
         cur = *c->h_scal;

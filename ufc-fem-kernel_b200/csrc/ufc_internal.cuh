@@ -211,6 +211,7 @@ struct Ctx {
   double* z64 = nullptr;
 
   double* res_zp = nullptr;  // [N][6] z and p records of the resident CG
+  int res_ctas = -1;         // its CTAs for this pattern (cg_resident_plan), -1: not asked yet
 
   // cached CUDA graphs of CG batches
   cudaGraphExec_t cg_graph[kGraphSlots] = {};
@@ -283,8 +284,8 @@ int pcg_solve_block(Ctx* c, int nrhs, const double* B, double* X, const ufc_solv
 void release_graphs(Ctx* c);
 
 // resident.cu
-bool cg_resident_fits(const Ctx* c);  // small enough for all iterations in one kernel
-int cg_resident(Ctx* c, const double* dinv, int chunk);
+int cg_resident_plan(Ctx* c);  // CTAs that take all iterations in one kernel, 0: the chain of kernels
+int cg_resident(Ctx* c, const double* dinv, int chunk, int ctas);
 
 // Device memory: every array of a context and every temporary comes from one
 // stream-ordered pool per device (capi.cu), in stream order of the context.
