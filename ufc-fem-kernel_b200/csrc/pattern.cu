@@ -201,20 +201,25 @@ __global__ void k_row_fill(int32_t N, const int32_t* __restrict__ conn, const in
   for (int k = 0; k < u; ++k) bcol[brow[i] + k] = buf[k];
 }
 
-// Longest row of each slice, in blocks.
+// Longest row of each slice, in blocks.  A node that no element names has no
+// block in the canonical pattern, but one of its own in the storage (see
+// k_sell_fill), so every row counts for at least one.
 __global__ void k_slice_len(int32_t N, int64_t nslices, const int32_t* __restrict__ brow, int64_t* __restrict__ len) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nslices) return;
   int32_t m = 0;
   for (int t = 0; t < kSlice; ++t) {
     const int64_t r = s * kSlice + t;
-    if (r < N) m = max(m, brow[r + 1] - brow[r]);
+    if (r < N) m = max(m, max(brow[r + 1] - brow[r], 1));
   }
   len[s] = (int64_t)m * kSlice;
 }
 
 // SELL column array: real entries, then padding that points at the row itself
-// (zero values), one thread per padded row.
+// (zero values), one thread per padded row.  dpos: the diagonal's position; in a
+// row without entries (a node that no element names) the first padding block is
+// the diagonal, zero on free DOFs and 1 on fixed ones, so that such a node keeps
+// its value in a solve (zero, or the prescribed one) and D^-1 is set for it.
 __global__ void k_sell_fill(int32_t N, int64_t nslices, const int32_t* __restrict__ brow,
                             const int32_t* __restrict__ bcol, const int64_t* __restrict__ sptr,
                             int32_t* __restrict__ scol, int32_t* __restrict__ dpos) {
@@ -227,7 +232,7 @@ __global__ void k_sell_fill(int32_t N, int64_t nslices, const int32_t* __restric
   for (int64_t j = 0; j < len; ++j) {
     const int32_t cj = j < m ? bcol[b + j] : self;
     scol[base + j * kSlice + t] = cj;
-    if (r < N && j < m && cj == r) dpos[r] = (int32_t)(base + j * kSlice + t);
+    if (r < N && cj == r && (j < m || (m == 0 && j == 0))) dpos[r] = (int32_t)(base + j * kSlice + t);
   }
 }
 
@@ -276,14 +281,16 @@ __device__ __forceinline__ int find_in_row(const int32_t* __restrict__ brow, con
   return -1;
 }
 
-// Lower (j < i) and upper (j >= i) block counts of every row.
+// Lower (j < i) and upper (j >= i) block counts of every row; a row without
+// entries counts its diagonal (see k_sell_fill).
 __global__ void k_sym_counts(int32_t N, const int32_t* __restrict__ brow, const int32_t* __restrict__ bcol,
                              int32_t* __restrict__ lcnt, int32_t* __restrict__ ucnt) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const int d = find_in_row(brow, bcol, i, (int32_t)i);  // the diagonal is always present
+  const int m = brow[i + 1] - brow[i];
+  const int d = m > 0 ? find_in_row(brow, bcol, i, (int32_t)i) : 0;  // present in every row with entries
   lcnt[i] = d;
-  ucnt[i] = brow[i + 1] - brow[i] - d;
+  ucnt[i] = max(m, 1) - d;
 }
 
 __global__ void k_slice_len_counts(int32_t N, int64_t nslices, const int32_t* __restrict__ cnt,
