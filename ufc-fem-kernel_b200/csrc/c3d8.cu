@@ -42,11 +42,22 @@ namespace {
 // about 320 when D is applied at every Gauss point); the J2 block as
 // sum_gp (D B_a)^T B_b with D B_a formed once per (row, element, Gauss point).
 //
+// Rounding must not have one sign in every element: the response of an element
+// to a rigid translation, zero but for rounding, then adds up along a slender
+// box like an elastic foundation.  So (1) the Jacobian is summed over the nodes'
+// coordinates instead of taken from coordinate differences, which are exact and
+// the same in all elements of a regular box, and (2) the linear-elastic block of
+// the row's own node is minus the sum of the row's other seven.  Displacements
+// of 80x4x4 elements of one modulus against extended precision: 1e-9 with
+// differences and all eight blocks summed alike, 2e-11 now; 40x8x8 with lognormal
+// moduli 1.7e-12 and 2e-13.
+//
 // What bounds it: the shared-memory pipe (97 % busy, 400 wavefronts per element
 // of 4 rows; FP64 35 %).  It serves the J2 tangents, and linear-elastic rows too
-// long for the shared memory of the one-thread form below.  Recomputing an element's Jacobians for each of its 8 rows costs less
-// than the read-modify-write of the values that an element-wise scatter needs
-// (16.6 GB at 192x96x96, in 8 colour passes).
+// long for the shared memory of the one-thread form below.  Recomputing an
+// element's Jacobians for each of its 8 rows costs less than the
+// read-modify-write of the values that an element-wise scatter needs (16.6 GB at
+// 192x96x96, in 8 colour passes).
 constexpr int kAsmRows = 16;                // rows per CTA
 constexpr int kAsmWarps = kAsmRows / 4;
 constexpr int kAsmMaxSmem = 227 * 1024;     // dynamic shared memory of one CTA
@@ -57,6 +68,12 @@ struct AsmWarp {
   T X[4][26];                             // element coordinates by sign bits, [row][3 bits + i], padded
   T P[4][8][kTangent ? 28 : 10];          // [row][gp]: scaled inverse Jacobian (9), then D B_a (18) for J2
 };
+
+// Entry (i, j) of the symmetric part of a 3x3 block.
+template <typename T>
+__device__ __forceinline__ T sym_part(const T (&v)[9], int i, int j) {
+  return i == j ? v[4 * i] : T(0.5) * (v[3 * i + j] + v[3 * j + i]);
+}
 
 template <typename T, bool kTangent>
 __global__ void __launch_bounds__(kAsmWarps * 32)
@@ -137,18 +154,21 @@ __global__ void __launch_bounds__(kAsmWarps * 32)
     fetch(k + 1);
     __syncwarp();
     if (on) {
-      // Gauss point t: J_di = dx_i / dxi_d from the 4 edges along d
+      // Gauss point t: J_di = dx_i / dxi_d, summed over the nodes
       const T* X = sm.X[rr];
       T J[9];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        J[i] = J[3 + i] = J[6 + i] = T(0);
+      for (int i = 0; i < 9; ++i) J[i] = T(0);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const int m0 = m & 1, m1 = m >> 1;
-          J[i] += c[0][m] * (X[3 * (1 + 2 * m0 + 4 * m1) + i] - X[3 * (2 * m0 + 4 * m1) + i]);
-          J[3 + i] += c[1][m] * (X[3 * (m0 + 2 + 4 * m1) + i] - X[3 * (m0 + 4 * m1) + i]);
-          J[6 + i] += c[2][m] * (X[3 * (m0 + 2 * m1 + 4) + i] - X[3 * (m0 + 2 * m1) + i]);
+      for (int m = 0; m < 8; ++m) {
+        const T d0 = flip_if(c[0][m >> 1], !(m & 1)), d1 = flip_if(c[1][(m & 1) | ((m >> 1) & 2)], !(m & 2)),
+                d2 = flip_if(c[2][m & 3], !(m & 4));
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const T x = X[3 * m + i];
+          J[i] += d0 * x;
+          J[3 + i] += d1 * x;
+          J[6 + i] += d2 * x;
         }
       }
       const T a0 = J[4] * J[8] - J[5] * J[7], a3 = J[5] * J[6] - J[3] * J[8], a6 = J[3] * J[7] - J[4] * J[6];
@@ -216,22 +236,32 @@ __global__ void __launch_bounds__(kAsmWarps * 32)
           for (int jj = 0; jj < 3; ++jj) K[3 * i + jj] += ga[i] * gb[jj];
       }
     }
+    if (!kTangent) {
+      const T tr = mu * (K[0] + K[4] + K[8]);
+      T v[9], own[9];
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int jj = 0; jj < 3; ++jj) {
+          v[3 * i + jj] = lam * K[3 * i + jj] + mu * K[3 * jj + i];
+          if (i == jj) v[3 * i + jj] += tr;
+        }
+      // the row node's own block is minus the sum of the others
+#pragma unroll
+      for (int i = 0; i < 9; ++i) own[i] = t == ta ? T(0) : -v[i];
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+        for (int i = 0; i < 9; ++i) own[i] += __shfl_xor_sync(0xffffffffu, own[i], o, 8);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int jj = 0; jj < 3; ++jj) K[3 * i + jj] = t == ta ? sym_part(own, i, jj) : v[3 * i + jj];
+    }
     if (on) {
       T* d = arow + 9 * j;
-      if (kTangent) {
 #pragma unroll
-        for (int i = 0; i < 9; ++i) d[i] += K[i];
-      } else {
-        const T tr = mu * (K[0] + K[4] + K[8]);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int jj = 0; jj < 3; ++jj) {
-            T v = lam * K[3 * i + jj] + mu * K[3 * jj + i];
-            if (i == jj) v += tr;
-            d[3 * i + jj] += v;
-          }
-      }
+      for (int i = 0; i < 9; ++i) d[i] += K[i];
     }
     __syncwarp();  // the warp's shared memory is consumed
   }
@@ -249,10 +279,13 @@ __global__ void __launch_bounds__(kAsmWarps * 32)
 // warps add their blocks in turn (named barriers pass the turn on), so each
 // entry still receives its contributions in ascending element order.  The
 // coordinates of a thread's next element come by cp.async while the current one
-// is worked on.  128x64x64, FP64 with FP32 copies: 1.32 ms; 8 lanes per row and
-// element as above 1.57 ms (shared-memory pipe 97 % busy); the colour-ordered
-// element scatter before 5.03 ms.  Here FP64 is 40 % busy, the rest is latency
-// (8 warps per SM; the accumulators take the registers).
+// is worked on.  The Jacobian's node sums (see above) are taken per eta and zeta
+// for both faces xi = -1 and +1, so that they read the coordinates no oftener
+// than differences along the edges would.  128x64x64, FP64 with FP32 copies, the
+// call with its products: 1.78 ms (1.66 ms with edge differences; node sums
+// formed at every Gauss point 2.26 ms; the colour-ordered element scatter before
+// 6.26 ms).  The kernel is bound by latency and FP64 (8 warps per SM; the
+// accumulators take the registers).
 constexpr int kIsoWarps = 4;
 constexpr int kIsoThreads = kIsoWarps * 32;
 constexpr int kIsoXBytes = kIsoWarps * 2 * 24 * 32 * (int)sizeof(double);  // [warp][stage][coordinate][lane]
@@ -331,38 +364,36 @@ __global__ void __launch_bounds__(kIsoThreads, 2)
 #pragma unroll 1
     for (int iz = 0; iz < 2; ++iz) {
       const T fz = ((ta >> 2) == iz) ? hp : hm;  // factors (1 + s g) / 2 of the row's node
-      const T tz = iz ? hp : hm;                 // the Gauss point's position on the edge
 #pragma unroll 1
       for (int iy = 0; iy < 2; ++iy) {
         if (!on) continue;
-        const T fy = (((ta >> 1) & 1) == iy) ? hp : hm, ty = iy ? hp : hm;
-        // at the Gauss point's eta and zeta, for xi = -1 and +1: value, half
-        // eta-derivative, half zeta-derivative of the coordinates
-        T v[2][3], dy[2][3], dz[2][3];
+        const T fy = (((ta >> 1) & 1) == iy) ? hp : hm;
+        // products of the element nodes' factors in two directions, by the nodes' bits in them
+        const T y0 = iy ? hm : hp, y1 = iy ? hp : hm, z0 = iz ? hm : hp, z1 = iz ? hp : hm;
+        const T pyz[4] = {T(0.5) * (y0 * z0), T(0.5) * (y1 * z0), T(0.5) * (y0 * z1), T(0.5) * (y1 * z1)};
+        // node sums for the Jacobian: d x / d xi, and the eta and zeta derivatives on the faces xi = -1 and +1
+        T Jx[3], Je[2][3], Jz[2][3];
 #pragma unroll
-        for (int x = 0; x < 2; ++x)
+        for (int i = 0; i < 3; ++i) Jx[i] = Je[0][i] = Je[1][i] = Jz[0][i] = Jz[1][i] = T(0);
+#pragma unroll
+        for (int b = 0; b < 8; ++b)
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
-            const T x00 = (T)X[32 * (3 * x + i)], x10 = (T)X[32 * (3 * (x + 2) + i)],
-                    x01 = (T)X[32 * (3 * (x + 4) + i)], x11 = (T)X[32 * (3 * (x + 6) + i)];
-            const T d0 = x01 - x00, d1 = x11 - x10;
-            const T v0 = x00 + tz * d0, v1 = x10 + tz * d1;
-            dz[x][i] = T(0.5) * (d0 + ty * (d1 - d0));
-            dy[x][i] = T(0.5) * (v1 - v0);
-            v[x][i] = v0 + ty * (v1 - v0);
+            const T x = (T)X[32 * (3 * b + i)];
+            Jx[i] += flip_if(pyz[b >> 1], !(b & 1)) * x;
+            Je[b & 1][i] += flip_if(T(0.5) * ((b & 4) ? z1 : z0), !(b & 2)) * x;
+            Jz[b & 1][i] += flip_if(T(0.5) * ((b & 2) ? y1 : y0), !(b & 4)) * x;
           }
-        // products of the element nodes' factors in eta and zeta: [same or opposite side of the Gauss point]
-        const T pyz[4] = {T(0.5) * ((iy ? hm : hp) * (iz ? hm : hp)), T(0.5) * ((iy ? hp : hm) * (iz ? hm : hp)),
-                          T(0.5) * ((iy ? hm : hp) * (iz ? hp : hm)), T(0.5) * ((iy ? hp : hm) * (iz ? hp : hm))};
 #pragma unroll 1
         for (int ix = 0; ix < 2; ++ix) {
-          const T fx = ((ta & 1) == ix) ? hp : hm, tx = ix ? hp : hm;
+          const T fx = ((ta & 1) == ix) ? hp : hm;
+          const T x0 = ix ? hm : hp, x1 = ix ? hp : hm;
           T J[9];
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
-            J[i] = T(0.5) * (v[1][i] - v[0][i]);
-            J[3 + i] = dy[0][i] + tx * (dy[1][i] - dy[0][i]);
-            J[6 + i] = dz[0][i] + tx * (dz[1][i] - dz[0][i]);
+            J[i] = Jx[i];
+            J[3 + i] = x0 * Je[0][i] + x1 * Je[1][i];
+            J[6 + i] = x0 * Jz[0][i] + x1 * Jz[1][i];
           }
           const T c0 = J[4] * J[8] - J[5] * J[7], c3 = J[5] * J[6] - J[3] * J[8], c6 = J[3] * J[7] - J[4] * J[6];
           const T det = J[0] * c0 + J[1] * c3 + J[2] * c6;
@@ -378,10 +409,9 @@ __global__ void __launch_bounds__(kIsoThreads, 2)
           for (int i = 0; i < 3; ++i) ga[i] = inv[3 * i] * a0 + inv[3 * i + 1] * a1 + inv[3 * i + 2] * a2;
 #pragma unroll
           for (int b = 0; b < 8; ++b) {
-            const T bx = ((b & 1) == ix) ? hp : hm, by = (((b >> 1) & 1) == iy) ? hp : hm,
-                    bz = ((b >> 2) == iz) ? hp : hm;
-            const T b0 = flip_if(pyz[b >> 1], !(b & 1)), b1 = flip_if(T(0.5) * (bx * bz), !(b & 2)),
-                    b2 = flip_if(T(0.5) * (bx * by), !(b & 4));
+            const T b0 = flip_if(pyz[b >> 1], !(b & 1)),
+                    b1 = flip_if(T(0.5) * (((b & 1) ? x1 : x0) * ((b & 4) ? z1 : z0)), !(b & 2)),
+                    b2 = flip_if(T(0.5) * (((b & 1) ? x1 : x0) * ((b & 2) ? y1 : y0)), !(b & 4));
             T gb[3];
 #pragma unroll
             for (int i = 0; i < 3; ++i) gb[i] = inv[3 * i] * b0 + inv[3 * i + 1] * b1 + inv[3 * i + 2] * b2;
@@ -413,8 +443,17 @@ __global__ void __launch_bounds__(kIsoThreads, 2)
     if (r > 0 || w > 0) bar_sync(1 + w, 64);
     if (on) {
       const int32_t ps[8] = {s0.x, s0.y, s0.w, s0.z, s1.x, s1.y, s1.w, s1.z};
+      // the row node's own block is minus the sum of the others
+      T own[9];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) own[i] = T(0);
+      int pos = 0;
 #pragma unroll
       for (int b = 0; b < 8; ++b) {
+        if (b == ta) {
+          pos = ps[b];
+          continue;
+        }
         T* d = acc + lane * stride + 9 * (int)((ps[b] - base) >> 5);
         const T tr = mu * (G[b][0] + G[b][4] + G[b][8]);
 #pragma unroll
@@ -424,8 +463,14 @@ __global__ void __launch_bounds__(kIsoThreads, 2)
             T v = lam * G[b][3 * i + jj] + mu * G[b][3 * jj + i];
             if (i == jj) v += tr;
             d[3 * i + jj] += v;
+            own[3 * i + jj] -= v;
           }
       }
+      T* d = acc + lane * stride + 9 * (int)((pos - base) >> 5);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int jj = 0; jj < 3; ++jj) d[3 * i + jj] += sym_part(own, i, jj);
     }
     if (r + 1 < rounds || w + 1 < kIsoWarps) {
       __threadfence_block();
