@@ -7,6 +7,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <unordered_set>
 #include <vector>
 
 #include "ufc_internal.cuh"
@@ -48,35 +49,89 @@ int check_dev_err(Ctx* c, const char* where) {
 
 namespace {
 
-// The memory pool of each device, made at its first use and kept for the life
-// of the process.  cudaMalloc and cudaFree cost about 0.1 ms a call and stop the
-// device; a model has some 60 arrays, and the default pool gives its memory back
-// at every synchronisation, so that each staged buffer was mapped anew.  This one
-// keeps at most kPoolKeep bytes of freed memory; what is freed beyond that goes
-// back to the device at the next synchronisation.  The pool is the library's own
-// (no setting of the default pool is touched) and safe for contexts on several
-// threads and streams: the runtime orders a reuse behind the stream that freed.
-// 48x24x24 analysis from host arrays: 37.6 -> 20.0 ms.
+// Device memory.  Arrays below kPoolMost bytes come from a pool per device, made
+// at its first use: cudaMalloc and cudaFree cost about 0.1 ms a call and stop the
+// device, a model has some 60 arrays, and the default pool gives its memory back
+// at every synchronisation, so that each staged buffer was mapped anew.  Larger
+// arrays are allocated by themselves: the pool maps memory more slowly than
+// cudaMalloc and would keep gigabytes.  First assembly of a new model at
+// 128x64x64 and 192x96x96, all arrays in the pool / above 16 / 64 / 256 MiB by
+// themselves: 17, 56 / 5.0, 10.7 / 4.4, 10.1 / 4.4, 10.7 ms; 60 iterations of a
+// 16-case block solve at 128x64x64, 47 ms of kernels: 75 / 55 / 55 / 50 ms;
+// stresses and loads at 97x51x47 0.61 / 1.34 / 1.37 / 0.61 ms (their buffers have
+// 90 MiB, and 200 MiB at 128x64x64).
+//
+// The release threshold counts the memory in use too, so it is kept kPoolKeep
+// above that: freed memory beyond it goes back to the device at the next
+// synchronisation, and so does all that is left when the last context of a device
+// closes (a 48x24x24 analysis from host arrays takes 25 ms, 22.7 if 256 MiB stayed).
+// The pool is the library's own (no setting of the default pool is touched) and
+// safe for contexts on several threads and streams: the runtime orders a reuse
+// behind the stream that freed.
+constexpr size_t kPoolMost = 256u << 20;
 constexpr uint64_t kPoolKeep = 1ull << 30;
 constexpr int kMaxDevices = 64;
 
-cudaMemPool_t device_pool(int device) {
-  static std::mutex lock;
-  static cudaMemPool_t pools[kMaxDevices] = {};
-  if (device < 0 || device >= kMaxDevices) return nullptr;
-  std::lock_guard<std::mutex> hold(lock);
-  if (!pools[device]) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device;
-    cudaMemPool_t p = nullptr;
-    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
-    uint64_t keep = kPoolKeep;
-    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    pools[device] = p;
+struct DeviceMemory {
+  std::mutex lock;
+  cudaMemPool_t pool = nullptr;
+  uint64_t threshold = 0;          // of release, as set
+  int contexts = 0;                // open
+};
+
+// The allocations outside the pools, of all devices.
+struct OwnAllocations {
+  std::mutex lock;
+  std::unordered_set<void*> set;
+};
+OwnAllocations& own_allocations() {
+  static OwnAllocations own;
+  return own;
+}
+
+DeviceMemory* device_memory(int device) {
+  static DeviceMemory mem[kMaxDevices];
+  return device >= 0 && device < kMaxDevices ? &mem[device] : nullptr;
+}
+
+// (with the lock held)
+bool have_pool(DeviceMemory* d, int device) {
+  if (d->pool) return true;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  return cudaMemPoolCreate(&d->pool, &props) == cudaSuccess;
+}
+
+uint64_t pool_used(const DeviceMemory* d) {
+  uint64_t used = 0;
+  cudaMemPoolGetAttribute(d->pool, cudaMemPoolAttrUsedMemCurrent, &used);
+  return used;
+}
+
+void set_threshold(DeviceMemory* d, uint64_t bytes) {
+  if (d->threshold != bytes && cudaMemPoolSetAttribute(d->pool, cudaMemPoolAttrReleaseThreshold, &bytes) == cudaSuccess)
+    d->threshold = bytes;
+}
+
+void context_opened(int device) {
+  if (DeviceMemory* d = device_memory(device)) {
+    std::lock_guard<std::mutex> hold(d->lock);
+    ++d->contexts;
   }
-  return pools[device];
+}
+
+// After a context has freed its memory and its stream is idle.
+void context_closed(int device) {
+  DeviceMemory* d = device_memory(device);
+  if (!d) return;
+  std::lock_guard<std::mutex> hold(d->lock);
+  --d->contexts;
+  if (!d->pool) return;
+  const uint64_t keep = pool_used(d) + (d->contexts > 0 ? kPoolKeep : 0);
+  set_threshold(d, keep);
+  cudaMemPoolTrimTo(d->pool, keep);
 }
 
 // The stream of the API call that this thread is serving: frees are ordered on it.
@@ -85,15 +140,39 @@ thread_local cudaStream_t t_stream = nullptr;
 }  // namespace
 
 cudaError_t pool_alloc(Ctx* c, void** p, size_t bytes) {
-  cudaMemPool_t pool = device_pool(c->device);
-  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, c->stream) : cudaErrorMemoryAllocation;
+  DeviceMemory* d = device_memory(c->device);
+  if (!d) return cudaErrorMemoryAllocation;
+  std::lock_guard<std::mutex> hold(d->lock);
+  if (!have_pool(d, c->device)) return cudaErrorMemoryAllocation;
+  cudaError_t e = cudaSuccess;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    e = bytes >= kPoolMost ? cudaMalloc(p, bytes) : cudaMallocFromPoolAsync(p, bytes, d->pool, c->stream);
+    if (e != cudaErrorMemoryAllocation || attempt > 0) break;
+    cudaGetLastError();  // once more without what the pool keeps
+    cudaStreamSynchronize(c->stream);
+    cudaMemPoolTrimTo(d->pool, 0);
+  }
+  if (e != cudaSuccess) return e;
+  if (bytes >= kPoolMost) {
+    std::lock_guard<std::mutex> also(own_allocations().lock);
+    own_allocations().set.insert(*p);
+  } else {
+    const uint64_t used = pool_used(d);
+    if (used + kPoolKeep / 2 > d->threshold || used + 2 * kPoolKeep < d->threshold) set_threshold(d, used + kPoolKeep);
+  }
+  return e;
 }
 
 void pool_free(void* p) {
-  if (t_stream)
-    cudaFreeAsync(p, t_stream);
-  else
+  bool own;
+  {
+    std::lock_guard<std::mutex> hold(own_allocations().lock);
+    own = own_allocations().set.erase(p) > 0;
+  }
+  if (own || !t_stream)
     cudaFree(p);
+  else
+    cudaFreeAsync(p, t_stream);
 }
 
 namespace {
@@ -307,6 +386,7 @@ int ufc_ctx_create(int32_t device, ufc_ctx** out) {
     return UFC_STATUS_MEM_ERROR;
   }
   c->h_err = reinterpret_cast<int32_t*>(c->h_scal + 3);
+  context_opened(device);
   *out = c;
   return UFC_STATUS_OK;
 }
@@ -322,6 +402,8 @@ int ufc_ctx_destroy(ufc_ctx* c) {
   dfree(&c->partials);
   dfree(&c->dev_err);
   t_stream = outer;
+  cudaStreamSynchronize(c->stream);  // the frees have passed
+  context_closed(c->device);
   if (c->h_scal) cudaFreeHost(c->h_scal);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
   if (c->stream) cudaStreamDestroy(c->stream);

@@ -287,8 +287,9 @@ void release_graphs(Ctx* c);
 int cg_resident_plan(Ctx* c);  // CTAs that take all iterations in one kernel, 0: the chain of kernels
 int cg_resident(Ctx* c, const double* dinv, int chunk, int ctas);
 
-// Device memory: every array of a context and every temporary comes from one
-// stream-ordered pool per device (capi.cu), in stream order of the context.
+// Device memory: every array of a context and every temporary (capi.cu).  Small
+// ones come from one stream-ordered pool per device, in stream order of the
+// context; large ones are allocated by themselves.
 cudaError_t pool_alloc(Ctx* c, void** p, size_t bytes);
 void pool_free(void* p);  // in order on the stream of the API call being served
 
