@@ -577,7 +577,12 @@ __global__ void k_diag_rowsum(int32_t N, const int64_t* __restrict__ sptr, const
 // now 50.5 + 12.8 us; 192x96x96: 801 us, now 465 + 96.  The octets are bound by
 // the shuffles (108 a lane), the node sums by the 192 bytes per element between
 // the two.  J2 at 64x32x32, return map and forces: 151 + 8 x 13 us, now 75 + 6.
+// The array holds at most kFeElems elements (50 MB): larger meshes go through it
+// in element order, each node adding to the sum of the passes before, so that
+// the result is the same to the last bit and the scratch does not grow with the
+// mesh (192 bytes per element would be a twentieth of a refined model).
 constexpr int kOctBlock = 256;
+constexpr int32_t kFeElems = 1 << 18;
 
 // The octet's element of this thread, clamped (all lanes take part in the
 // exchanges; `real` says whether to write), its node and coordinates.
@@ -587,10 +592,12 @@ struct OctElem {
   int64_t node;
   bool real;
   double X[3];
-  __device__ __forceinline__ OctElem(int32_t E, const double* __restrict__ coords, const int32_t* __restrict__ conn) {
-    const int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-    real = k < E;
-    e = real ? k : E - 1;
+  // elements [e0, e1)
+  __device__ __forceinline__ OctElem(int32_t e0, int32_t e1, const double* __restrict__ coords,
+                                     const int32_t* __restrict__ conn) {
+    const int64_t k = e0 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3);
+    real = k < e1;
+    e = real ? k : e1 - 1;
     t = threadIdx.x & 7;
     a = bits_node(t);
     node = conn[e * 8 + a];
@@ -599,7 +606,7 @@ struct OctElem {
   }
 };
 
-// Nodal forces of every element, fe[(8 e + a) 3 + i]:
+// Nodal forces of the elements [e0, e1), fe[(8 (e - e0) + a) 3 + i]:
 //   kIso      B^T D B x with the linear-elastic D (masked by `fixed` when given);
 //             the internal force of the material (PH_Elem_C3D8_IntForce, PH_Elem_C3D8.f90:734-757)
 //   kTangent  B^T D_gp B x with the tangents of the last return map (unmasked);
@@ -608,10 +615,10 @@ enum ForceMode { kIso, kTangent };
 
 template <int MODE>
 __global__ void __launch_bounds__(kOctBlock)
-    k_oct_force(int32_t E, const double* __restrict__ coords, const int32_t* __restrict__ conn,
+    k_oct_force(int32_t e0, int32_t e1, const double* __restrict__ coords, const int32_t* __restrict__ conn,
                 const double* __restrict__ lame, const double* __restrict__ Dt, const double* __restrict__ x,
                 const uint8_t* __restrict__ fixed, double* __restrict__ fe, int32_t* __restrict__ err) {
-  const OctElem el(E, coords, conn);
+  const OctElem el(e0, e1, coords, conn);
   const Octet oct(el.t);
   double u[3], inv[9], eps[6], s[6], f[3];
 #pragma unroll
@@ -639,20 +646,20 @@ __global__ void __launch_bounds__(kOctBlock)
   oct.nodal_force(inv, det, s, f);
   if (el.real)
 #pragma unroll
-    for (int i = 0; i < 3; ++i) fe[(el.e * 8 + el.a) * 3 + i] = f[i];
+    for (int i = 0; i < 3; ++i) fe[((el.e - e0) * 8 + el.a) * 3 + i] = f[i];
 }
 
 // J2 return map at every Gauss point: strain increment from du = u - u_n,
 // committed state (sig_n, epeq_n, epl_n) -> trial state, consistent tangent and
 // the element's nodal forces of the trial stress.
 __global__ void __launch_bounds__(kOctBlock)
-    k_oct_j2(int32_t E, const double* __restrict__ coords, const int32_t* __restrict__ conn,
+    k_oct_j2(int32_t e0, int32_t e1, const double* __restrict__ coords, const int32_t* __restrict__ conn,
              const double* __restrict__ props, int nprops, const double* __restrict__ u,
              const double* __restrict__ u_n, const double* __restrict__ sig_n, const double* __restrict__ epeq_n,
              const double* __restrict__ epl_n, double* __restrict__ sig_t, double* __restrict__ epeq_t,
              double* __restrict__ epl_t, double* __restrict__ Dt, double* __restrict__ fe,
              int32_t* __restrict__ err) {
-  const OctElem el(E, coords, conn);
+  const OctElem el(e0, e1, coords, conn);
   const Octet oct(el.t);
   const int64_t g = el.e * 8 + el.t;
   double du[3], inv[9], de[6], s[6], epl[6], D[36], epeq, f[3];
@@ -681,23 +688,37 @@ __global__ void __launch_bounds__(kOctBlock)
   oct.nodal_force(inv, det, s, f);
   if (el.real)
 #pragma unroll
-    for (int i = 0; i < 3; ++i) fe[(el.e * 8 + el.a) * 3 + i] = f[i];
+    for (int i = 0; i < 3; ++i) fe[((el.e - e0) * 8 + el.a) * 3 + i] = f[i];
 }
 
-// y_i = sum of the element forces at DOF i, elements ascending.  With `x` the
-// eliminated operator: y = x on fixed DOFs (identity rows).
+// y_i = sum of the element forces at DOF i, elements ascending; PART: of the
+// elements [e0, e1), added to what the passes before them left (e0 = 0: none).
+// With `x` the eliminated operator: y = x on fixed DOFs (identity rows).
+template <bool PART>
 __global__ void __launch_bounds__(256)
-    k_node_sum(int64_t n, const int32_t* __restrict__ nptr, const int32_t* __restrict__ nelem,
+    k_node_sum(int64_t n, int32_t e0, int32_t e1, const int32_t* __restrict__ nptr, const int32_t* __restrict__ nelem,
                const double* __restrict__ fe, const uint8_t* __restrict__ fixed, const double* __restrict__ x,
                double* __restrict__ y) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t node = i / 3;
   const int c = (int)(i - 3 * node);
-  double s = 0.0;
   const int32_t k0 = nptr[node], k1 = nptr[node + 1];
+  double s = 0.0;
+  if constexpr (PART) {
+    const int64_t lo = 8 * (int64_t)e0, hi = 8 * (int64_t)e1;
+    if (e0 > 0) {
+      if (k0 == k1 || nelem[k1 - 1] < lo || nelem[k0] >= hi) return;  // the node has none of these elements
+      s = y[i];
+    }
+    for (int32_t k = k0; k < k1; ++k) {
+      const int64_t el = nelem[k];
+      if (el >= lo && el < hi) s += fe[3 * (el - lo) + c];
+    }
+  } else {
 #pragma unroll 4
-  for (int32_t k = k0; k < k1; ++k) s += fe[3 * (int64_t)nelem[k] + c];
+    for (int32_t k = k0; k < k1; ++k) s += fe[3 * (int64_t)nelem[k] + c];
+  }
   y[i] = (x && fixed[i]) ? x[i] : s;
 }
 
@@ -717,7 +738,7 @@ __global__ void __launch_bounds__(kOctBlock)
     k_oct_stress(int32_t E, const double* __restrict__ coords, const int32_t* __restrict__ conn,
                  const double* __restrict__ lame, const double* __restrict__ u, const double* __restrict__ s6,
                  double* __restrict__ sig, double* __restrict__ vm) {
-  const OctElem el(E, coords, conn);
+  const OctElem el(0, E, coords, conn);
   const Octet oct(el.t);
   const int64_t g = el.e * 8 + el.t;
   double s[6];
@@ -808,7 +829,7 @@ __global__ void __launch_bounds__(kOctBlock)
     k_adjoint_sens(int32_t E, int64_t n, int nrhs, const double* __restrict__ coords,
                    const int32_t* __restrict__ conn, const double* __restrict__ props, int nprops,
                    const double* __restrict__ U, const double* __restrict__ L, double* __restrict__ g) {
-  const OctElem el(E, coords, conn);
+  const OctElem el(0, E, coords, conn);
   const Octet oct(el.t);
   double inv[9], lam, mu;
   const double det = oct.jacobian(el.X, inv);
@@ -949,36 +970,41 @@ namespace {
 
 int oct_grid(const Ctx* c) { return grid_for(8 * (int64_t)c->E, kOctBlock); }
 
-// y = node sums of the element forces in c->fe; x: identity rows on fixed DOFs
-int node_sum(Ctx* c, const double* x, double* y) {
-  k_node_sum<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->nptr, c->nelem, c->fe, c->fixed, x, y);
-  UFC_CUDA(c, cudaGetLastError());
-  c->launches += 1;
+// y = node sums of the element forces that `forces(e0, e1)` leaves in c->fe; x:
+// identity rows on fixed DOFs
+template <class Forces>
+int sum_forces(Ctx* c, const double* x, double* y, Forces forces) {
+  if (!c->fe) UFC_TRY(dalloc(c, &c->fe, 24 * (int64_t)std::min(c->E, kFeElems)));
+  for (int32_t e0 = 0; e0 < c->E; e0 += kFeElems) {
+    const int32_t e1 = std::min(c->E - e0, kFeElems) + e0;
+    forces(e0, e1);
+    UFC_CUDA(c, cudaGetLastError());
+    const int grid = grid_for(c->n, 256);
+    if (c->E <= kFeElems)
+      k_node_sum<false><<<grid, 256, 0, c->stream>>>(c->n, e0, e1, c->nptr, c->nelem, c->fe, c->fixed, x, y);
+    else
+      k_node_sum<true><<<grid, 256, 0, c->stream>>>(c->n, e0, e1, c->nptr, c->nelem, c->fe, c->fixed, x, y);
+    UFC_CUDA(c, cudaGetLastError());
+    c->launches += 2;
+  }
   return UFC_STATUS_OK;
 }
 
-int ensure_fe(Ctx* c) { return c->fe ? UFC_STATUS_OK : dalloc(c, &c->fe, 24 * (int64_t)c->E); }
+int part_grid(int32_t e0, int32_t e1) { return grid_for(8 * (int64_t)(e1 - e0), kOctBlock); }
+
+int apply_iso(Ctx* c, const double* x, const uint8_t* fixed, const double* identity, double* y) {
+  return sum_forces(c, identity, y, [&](int32_t e0, int32_t e1) {
+    k_oct_force<kIso><<<part_grid(e0, e1), kOctBlock, 0, c->stream>>>(e0, e1, c->coords, c->conn, c->lame, nullptr, x,
+                                                                      fixed, c->fe, c->dev_err);
+  });
+}
 
 }  // namespace
 
 // y = K x matrix-free, FP64, without elimination (the linear-elastic internal force).
-int apply_fp64(Ctx* c, const double* x, double* y) {
-  UFC_TRY(ensure_fe(c));
-  k_oct_force<kIso><<<oct_grid(c), kOctBlock, 0, c->stream>>>(c->E, c->coords, c->conn, c->lame, nullptr, x, nullptr,
-                                                              c->fe, c->dev_err);
-  UFC_CUDA(c, cudaGetLastError());
-  c->launches += 1;
-  return node_sum(c, nullptr, y);
-}
+int apply_fp64(Ctx* c, const double* x, double* y) { return apply_iso(c, x, nullptr, nullptr, y); }
 
-int apply_fp64_eliminated(Ctx* c, const double* x, double* y) {
-  UFC_TRY(ensure_fe(c));
-  k_oct_force<kIso><<<oct_grid(c), kOctBlock, 0, c->stream>>>(c->E, c->coords, c->conn, c->lame, nullptr, x, c->fixed,
-                                                              c->fe, c->dev_err);
-  UFC_CUDA(c, cudaGetLastError());
-  c->launches += 1;
-  return node_sum(c, x, y);
-}
+int apply_fp64_eliminated(Ctx* c, const double* x, double* y) { return apply_iso(c, x, c->fixed, x, y); }
 
 // Newton residual R = f_ext - F_int on free DOFs (0 on fixed) and the norms
 // ||R||^2, ||F_int||^2, ||F_ext||^2 into the scalars (RT_Asm_ComputeResidual,
@@ -1015,22 +1041,21 @@ int compute_fint(Ctx* c, const double* u, double* fint, bool update_state) {
   if (!c->has_material) return fail(c, UFC_STATUS_INVALID, "ufc_elem_compute_fint: material not set");
   if (c->ncol == 0) return fail(c, UFC_STATUS_INVALID, "ufc_elem_compute_fint: pattern not built");
   if (c->mat_model != UFC_MAT_J2_ISO) return apply_fp64(c, u, fint);
-  UFC_TRY(ensure_fe(c));
-  k_oct_j2<<<oct_grid(c), kOctBlock, 0, c->stream>>>(c->E, c->coords, c->conn, c->props, c->nprops, u, c->u_n,
-                                                     c->sig_n, c->epeq_n, c->epl_n, c->sig_t, c->epeq_t, c->epl_t,
-                                                     c->Dt, c->fe, c->dev_err);
-  UFC_CUDA(c, cudaGetLastError());
+  UFC_TRY(sum_forces(c, nullptr, fint, [&](int32_t e0, int32_t e1) {
+    k_oct_j2<<<part_grid(e0, e1), kOctBlock, 0, c->stream>>>(e0, e1, c->coords, c->conn, c->props, c->nprops, u,
+                                                             c->u_n, c->sig_n, c->epeq_n, c->epl_n, c->sig_t, c->epeq_t,
+                                                             c->epl_t, c->Dt, c->fe, c->dev_err);
+  }));
   c->has_trial = true;
-  return node_sum(c, nullptr, fint);
+  return UFC_STATUS_OK;
 }
 
 int apply_tangent(Ctx* c, const double* x, double* y) {
   if (!c->has_trial) return fail(c, UFC_STATUS_INVALID, "tangent operator needs a return map first");
-  UFC_TRY(ensure_fe(c));
-  k_oct_force<kTangent><<<oct_grid(c), kOctBlock, 0, c->stream>>>(c->E, c->coords, c->conn, nullptr, c->Dt, x, nullptr,
-                                                                  c->fe, c->dev_err);
-  UFC_CUDA(c, cudaGetLastError());
-  return node_sum(c, nullptr, y);
+  return sum_forces(c, nullptr, y, [&](int32_t e0, int32_t e1) {
+    k_oct_force<kTangent><<<part_grid(e0, e1), kOctBlock, 0, c->stream>>>(e0, e1, c->coords, c->conn, nullptr, c->Dt, x,
+                                                                          nullptr, c->fe, c->dev_err);
+  });
 }
 
 int mat_update_batch(Ctx* c, const ufc_mat_update_arg* a, const double* props, const double* stress_n,

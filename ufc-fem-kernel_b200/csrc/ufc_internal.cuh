@@ -194,7 +194,7 @@ struct Ctx {
   int32_t* dev_err = nullptr;
   int32_t* h_err = nullptr;     // pinned
 
-  double* fe = nullptr;  // [E][8][3] element forces of the matrix-free operators
+  double* fe = nullptr;  // [at most 2^18 elements][8][3] element forces of the matrix-free operators
   // Newton work vectors
   double *nr_fint = nullptr, *nr_R = nullptr, *nr_du = nullptr, *nr_dc = nullptr;
 
