@@ -1130,10 +1130,17 @@ int mg_numeric(Ctx* c) {
       if (l == 0) {
         UFC_TRY(mg_alloc(c, &L.dinv32, n));
         k_mg_round<<<grid_n(n), kBlk, 0, c->stream>>>(n, c->dinv64, L.dinv32);
-        if (c->has_sval64 && c->sym_coded && spmv_split(c) == 1) {
-          // the coded symmetric product reads half the bytes (128x64x64: 62 against 89 us)
-          const int64_t nb = c->s_ublocks + kSlice;
-          UFC_TRY(mg_alloc(c, &L.sval32, nb * 9));
+        // the coded symmetric product reads half the bytes (128x64x64: 62 against 89 us)
+        const int64_t nb = c->s_ublocks + kSlice;
+        bool sym = c->has_sval64 && c->sym_coded && spmv_split(c) == 1;
+        if (sym && mg_alloc(c, &L.sval32, nb * 9) != UFC_STATUS_OK) {
+          // (the tangent's symmetric storage is taken where it fits; its copy need not fit too)
+          if (!L.val32) return UFC_STATUS_MEM_ERROR;
+          cudaGetLastError();
+          c->err.clear();
+          sym = false;
+        }
+        if (sym) {
           k_mg_round_sym<<<grid_n(nb), kBlk, 0, c->stream>>>(nb, c->sval64, L.sval32);
         } else {
           const int64_t nv = c->sell_blocks * 9;

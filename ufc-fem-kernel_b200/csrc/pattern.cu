@@ -715,13 +715,19 @@ int build_full_codes(Ctx* c) {
   return done(UFC_STATUS_OK);
 }
 
-int build_pattern(Ctx* c) {
-  if (c->E <= 0 || c->N <= 0) return fail(c, UFC_STATUS_INVALID, "ufc_pattern_build: mesh not set");
+// The symmetric storage and its index arrays; graphs that read them go with them.
+void free_symmetric(Ctx* c) {
   release_graphs(c);
   dfree(&c->uptr); dfree(&c->ucol); dfree(&c->lptr); dfree(&c->lpos); dfree(&c->lcol); dfree(&c->s_lcnt);
-  dfree(&c->sval64); dfree(&c->sval32); dfree(&c->sym_ucode); dfree(&c->sym_lcode); dfree(&c->full_code);
-  c->full_coded = false;
+  dfree(&c->sval64); dfree(&c->sval32); dfree(&c->sym_ucode); dfree(&c->sym_lcode);
   c->has_sym_pattern = c->has_sval64 = c->has_sval32 = c->sym_coded = false;
+}
+
+int build_pattern(Ctx* c) {
+  if (c->E <= 0 || c->N <= 0) return fail(c, UFC_STATUS_INVALID, "ufc_pattern_build: mesh not set");
+  free_symmetric(c);
+  dfree(&c->full_code);
+  c->full_coded = false;
   c->res_ctas = -1;
   const int32_t N = c->N, E = c->E;
 
@@ -908,8 +914,16 @@ int build_sym_pattern(Ctx* c) {
   if (!c->has_pattern) return fail(c, UFC_STATUS_INVALID, "symmetric storage: pattern not built");
   if (c->has_sym_pattern) return UFC_STATUS_OK;
   const int32_t N = c->N;
-  int32_t* ucnt = nullptr;
-  int64_t* len = nullptr;
+  struct Temporaries {  // freed on every way out: the caller may go on without the storage
+    int32_t* ucnt = nullptr;
+    int64_t* len = nullptr;
+    ~Temporaries() {
+      dfree(&len);
+      dfree(&ucnt);
+    }
+  } tmp;
+  int32_t*& ucnt = tmp.ucnt;
+  int64_t*& len = tmp.len;
   UFC_TRY(dalloc(c, &c->s_lcnt, N));
   UFC_TRY(dalloc(c, &ucnt, N));
   UFC_TRY(dalloc(c, &len, c->nslices + 1));
@@ -928,8 +942,6 @@ int build_sym_pattern(Ctx* c) {
   UFC_CUDA(c, cudaMemcpyAsync(&c->s_lblocks, c->lptr + c->nslices, sizeof(int64_t), cudaMemcpyDeviceToHost,
                               c->stream));
   UFC_CUDA(c, cudaStreamSynchronize(c->stream));
-  dfree(&len);
-  dfree(&ucnt);
   if (c->s_ublocks + kSlice >= ((int64_t)1 << 31))
     return fail(c, UFC_STATUS_UNSUPPORTED, "symmetric storage: more than 2^31 stored blocks");
   UFC_TRY(dalloc(c, &c->ucol, c->s_ublocks));

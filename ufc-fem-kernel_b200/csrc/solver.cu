@@ -759,8 +759,11 @@ bool fp64_fits_l2(const Ctx* c) {
 // 58.4/52.7, 96x48x48 (456 MB) 311/206; multigrid 56x28x28 11.0/11.5, 64x32x32
 // (137 MB) 9.6/9.9, 96x48x48 25.5/19.6.  The first increment builds the
 // symmetric pattern, 2 ms at 64x32x32.
-// The storage is optional here, so it is taken only where device memory is
-// plentiful: a run that fits without it must not end for it.
+// The rule looks at sizes only, so that the same increment takes the same
+// products whatever else the device holds.  The storage is optional here and
+// must not end a run that fits without it: it is not taken where four times the
+// full values would fill the device, what the increment needs in either form is
+// allocated first, and if the storage does not fit then the full form stays.
 bool tangent_symmetric(Ctx* c, bool mg) {
   int dev = 0, l2 = 0;
   cudaGetDevice(&dev);
@@ -769,8 +772,15 @@ bool tangent_symmetric(Ctx* c, bool mg) {
   if (!c->full_coded || full < (mg ? 2 * (int64_t)l2 : (int64_t)l2 / 2)) return false;
   if (c->sval64) return true;
   size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || (int64_t)free_b < 4 * full) return false;
-  if (alloc_symmetric(c, false) == UFC_STATUS_OK) return true;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || (int64_t)total_b < 4 * full) return false;
+  int st = UFC_STATUS_OK;
+  if (!c->val64) st = dalloc(c, &c->val64, c->sell_blocks * 9);
+  if (st == UFC_STATUS_OK && !c->dinv64) st = dalloc(c, &c->dinv64, c->n);
+  if (st == UFC_STATUS_OK && mg && !c->z64) st = dalloc(c, &c->z64, c->n);
+  if (st == UFC_STATUS_OK) st = ensure_vectors(c, UFC_PRECISION_FP64);
+  if (st == UFC_STATUS_OK) st = alloc_symmetric(c, false);
+  if (st == UFC_STATUS_OK) return true;
+  free_symmetric(c);
   cudaGetLastError();
   c->err.clear();
   return false;

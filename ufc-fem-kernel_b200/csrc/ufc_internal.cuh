@@ -237,6 +237,7 @@ int build_sym_codes(Ctx* c);
 int build_full_codes(Ctx* c);
 bool tangent_symmetric(Ctx* c, bool mg);  // storage of the tangent in a Newton increment
 int alloc_symmetric(Ctx* c, bool fp32);  // arrays of the symmetric SpMV copies, filled by the assembly
+void free_symmetric(Ctx* c);
 int export_csr(Ctx* c, const ufc_csr_export_arg* a);
 
 // c3d8.cu
