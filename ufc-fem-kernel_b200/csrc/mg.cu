@@ -79,7 +79,7 @@ struct Mg {
   bool stale = false;
   bool fp32 = false;         // the cycle runs in FP32 (values, vectors); the PCG around it in FP64
   int cheb_coarse = 0;       // degree of the coarsest Chebyshev solve (0: dense inverse)
-  double lmax_scale = 1.0;   // raised when the smoother's interval proved too short
+  double lmax_scale = 1.0;   // of the coefficients in place: above 1 inside a solve whose cycle was indefinite
   double* dnorm = nullptr;   // ||v||^2 of the power iteration, on the device
   int32_t* gj_flag = nullptr;  // set when the coarsest elimination met a pivot that is not positive
   // the PCG iteration as a graph, and what it baked in
@@ -554,8 +554,8 @@ __global__ void __launch_bounds__(kBlk) k_mg_sum(const double* __restrict__ part
 
 // The smoother's interval [1.1 lambda_max / ratio, 1.1 lambda_max] and the
 // coefficients of m steps.  nb > 0: lambda_max = ||v_k|| / ||v_{k-1}|| of the
-// power iteration (partials of ||v_k||^2 and *prev = ||v_{k-1}||^2); nb = 0: the
-// stored one, times scale.
+// power iteration (partials of ||v_k||^2 and *prev = ||v_{k-1}||^2), kept in
+// coef[0]; nb = 0: from the kept one, times scale.
 __global__ void __launch_bounds__(kBlk)
     k_mg_coef(const double* __restrict__ partials, int nb, const double* __restrict__ prev, double scale, double ratio,
               int m, double* __restrict__ coef) {
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(kBlk)
   if (nb > 0) sum_partials<1>(partials, nb, tot);
   if (threadIdx.x != 0) return;
   const double lambda = nb > 0 ? (*prev > 0.0 ? sqrt(tot[0] / *prev) : 0.0) : coef[0] * scale;
-  coef[0] = lambda;
+  if (nb > 0) coef[0] = lambda;
   const double lmax = 1.1 * lambda, lmin = lmax / ratio;
   const double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin);
   const double sigma = theta / delta;
@@ -1351,6 +1351,24 @@ static int pcg_mg_graph(Ctx* c, Mg& mg, int batch) {
   return UFC_STATUS_OK;
 }
 
+// The smoothers' intervals for a solve: as estimated, or widened by set().  A
+// solve leaves them as it found them, so that it gives the same bits on a
+// hierarchy that others have used before.
+struct Widening {
+  Ctx* c;
+  Mg& mg;
+  ~Widening() {
+    if (mg.lmax_scale != 1.0) set(1.0);
+  }
+  void set(double scale) {
+    mg.lmax_scale = scale;
+    for (size_t l = 0; l < mg.lv.size(); ++l)
+      if (mg.lv[l].coef && lv_degree(mg, l) > 0)
+        k_mg_coef<<<1, kBlk, 0, c->stream>>>(nullptr, 0, nullptr, scale, lv_ratio(mg, l), lv_degree(mg, l),
+                                             mg.lv[l].coef);
+  }
+};
+
 int pcg_mg(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
   if (!c->mg) return fail(c, UFC_STATUS_INVALID, "ufc_pcg_solve: multigrid not set up (ufc_mg_setup)");
   if (c->mg->stale) UFC_TRY(mg_refresh(c));
@@ -1393,6 +1411,7 @@ int pcg_mg(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
   int flag = 0, restarts = 0;
   const int batch = algo->check_every > 0 ? algo->check_every : 2;
   int status = UFC_STATUS_OK;
+  Widening widening{c, mg};
   cudaEvent_t done[2] = {nullptr, nullptr};
   if (!converged) {
     UFC_TRY(pcg_mg_graph(c, mg, batch));
@@ -1453,11 +1472,7 @@ int pcg_mg(Ctx* c, const ufc_solver_algo* algo, ufc_solver_state* st) {
       // the cycle was not positive definite: lambda_max was underestimated, so
       // the smoothers' intervals are widened before the restart
       constexpr double kWiden = 1.3;
-      mg.lmax_scale *= kWiden;
-      for (size_t l = 0; l < mg.lv.size(); ++l)
-        if (mg.lv[l].coef && lv_degree(mg, l) > 0)
-          k_mg_coef<<<1, kBlk, 0, c->stream>>>(nullptr, 0, nullptr, kWiden, lv_ratio(mg, l), lv_degree(mg, l),
-                                               mg.lv[l].coef);
+      widening.set(mg.lmax_scale * kWiden);
       UFC_CUDA(c, cudaGetLastError());
     }
   }
