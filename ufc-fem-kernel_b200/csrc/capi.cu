@@ -84,13 +84,15 @@ struct OwnAllocations {
   std::mutex lock;
   std::unordered_set<void*> set;
 };
+// (Never destroyed, like device_memory's: a program may close its last context
+// from a destructor that runs at exit, after this library's.)
 OwnAllocations& own_allocations() {
-  static OwnAllocations own;
-  return own;
+  static OwnAllocations* own = new OwnAllocations;
+  return *own;
 }
 
 DeviceMemory* device_memory(int device) {
-  static DeviceMemory mem[kMaxDevices];
+  static DeviceMemory* mem = new DeviceMemory[kMaxDevices];
   return device >= 0 && device < kMaxDevices ? &mem[device] : nullptr;
 }
 
