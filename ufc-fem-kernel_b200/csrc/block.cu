@@ -940,7 +940,7 @@ struct BlockRun {
 };
 
 // The tile of k_bspmv_tile from the offsets of the coded storage (ascending);
-// false when the pattern's tile would not fit three blocks per SM.
+// false when its two stages would not fit the shared memory of one block per SM.
 bool make_tile(const Ctx* c, BTile* T) {
   *T = BTile{};
   if (!c->full_coded || c->full_ntab <= 0) return false;

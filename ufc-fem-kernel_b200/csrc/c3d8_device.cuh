@@ -32,38 +32,6 @@ __device__ __forceinline__ void dN_dxi(int ip, int a, T& d0, T& d1, T& d2) {
   d2 = T(0.125) * s2 * f0 * f1;
 }
 
-// Jacobian J_ij = sum_a dN_a/dxi_i x_aj at Gauss point ip; returns detJ and J^-1.
-template <typename T>
-__device__ __forceinline__ T jacobian_inv(const T* X, int ip, T inv[9]) {
-  T J[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) J[k] = T(0);
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    T d0, d1, d2;
-    dN_dxi<T>(ip, a, d0, d1, d2);
-    const T x = X[a * 3], y = X[a * 3 + 1], z = X[a * 3 + 2];
-    J[0] += d0 * x; J[1] += d0 * y; J[2] += d0 * z;
-    J[3] += d1 * x; J[4] += d1 * y; J[5] += d1 * z;
-    J[6] += d2 * x; J[7] += d2 * y; J[8] += d2 * z;
-  }
-  const T c0 = J[4] * J[8] - J[5] * J[7];
-  const T c1 = J[5] * J[6] - J[3] * J[8];
-  const T c2 = J[3] * J[7] - J[4] * J[6];
-  const T det = J[0] * c0 + J[1] * c1 + J[2] * c2;
-  const T id = T(1) / det;
-  inv[0] = c0 * id;
-  inv[1] = (J[2] * J[7] - J[1] * J[8]) * id;
-  inv[2] = (J[1] * J[5] - J[2] * J[4]) * id;
-  inv[3] = c1 * id;
-  inv[4] = (J[0] * J[8] - J[2] * J[6]) * id;
-  inv[5] = (J[2] * J[3] - J[0] * J[5]) * id;
-  inv[6] = c2 * id;
-  inv[7] = (J[1] * J[6] - J[0] * J[7]) * id;
-  inv[8] = (J[0] * J[4] - J[1] * J[3]) * id;
-  return det;
-}
-
 // dN_a/dx = J^-1 dN_a/dxi.
 template <typename T>
 __device__ __forceinline__ void grad_x(const T inv[9], int ip, int a, T g[3]) {
@@ -72,42 +40,6 @@ __device__ __forceinline__ void grad_x(const T inv[9], int ip, int a, T g[3]) {
   g[0] = inv[0] * d0 + inv[1] * d1 + inv[2] * d2;
   g[1] = inv[3] * d0 + inv[4] * d1 + inv[5] * d2;
   g[2] = inv[6] * d0 + inv[7] * d1 + inv[8] * d2;
-}
-
-// Voigt strain (engineering shear) of element displacements ue at Gauss point ip.
-template <typename T>
-__device__ __forceinline__ void strain_at(const T inv[9], int ip, const T* ue, T eps[6]) {
-  T H[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) H[k] = T(0);
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    T g[3];
-    grad_x<T>(inv, ip, a, g);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) H[i * 3 + j] += ue[a * 3 + i] * g[j];
-  }
-  eps[0] = H[0];
-  eps[1] = H[4];
-  eps[2] = H[8];
-  eps[3] = H[1] + H[3];
-  eps[4] = H[5] + H[7];
-  eps[5] = H[6] + H[2];
-}
-
-// fe += wdet * B^T sigma.
-template <typename T>
-__device__ __forceinline__ void add_bt_sigma(const T inv[9], int ip, T wdet, const T s[6], T* fe) {
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    T g[3];
-    grad_x<T>(inv, ip, a, g);
-    fe[a * 3 + 0] += wdet * (g[0] * s[0] + g[1] * s[3] + g[2] * s[5]);
-    fe[a * 3 + 1] += wdet * (g[1] * s[1] + g[0] * s[3] + g[2] * s[4]);
-    fe[a * 3 + 2] += wdet * (g[2] * s[2] + g[1] * s[4] + g[0] * s[5]);
-  }
 }
 
 // Isotropic sigma = D eps (PH_Elem_C3D8_ConstMatrix, PH_Elem_C3D8.f90:603-625).

@@ -92,24 +92,14 @@ struct Mg {
 namespace {
 
 constexpr int kBlk = 256;
-// largest coarsest level inverted densely (on the host, O(n^3), at every set-up
-// and refresh); larger ones get a degree-24 Chebyshev solve
+// largest coarsest level inverted densely (block Gauss-Jordan on the device at
+// every set-up and refresh); larger ones get a degree-24 Chebyshev solve
 constexpr int64_t kDenseMax = 1200;
 
 int grid_n(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + kBlk - 1) / kBlk, 148 * 16)); }
 
 __host__ __device__ inline int64_t box_node(int64_t i, int64_t j, int64_t k, int32_t nx, int32_t ny) {
   return i + (int64_t)(nx + 1) * (j + (int64_t)(ny + 1) * k);
-}
-
-// Weight of coarse node A (its signs) at a fine node with coarse parametric
-// coordinates xi in {-1, 0, 1}: the trilinear hat, prod_d (1 + s_d xi_d) / 2.
-__device__ __forceinline__ double hat(int A, int x0, int x1, int x2) {
-  const int xi[3] = {x0, x1, x2};
-  double w = 1.0;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) w *= 0.5 * (1.0 + (double)(node_sign(A, d) * xi[d]));
-  return w;
 }
 
 // Galerkin element matrices of one coarse level: one CTA per coarse element, one

@@ -9,11 +9,15 @@
 namespace ufc {
 namespace {
 
-// Programmatic dependent launch between the kernels of a CG iteration: each
-// kernel lets its successor launch as soon as all of its own blocks are
-// running (launch_dependents), and waits for its predecessor's completion and
-// memory (wait) before it reads anything; both are no-ops for a kernel
-// launched without the attribute.
+// Programmatic dependent launch between the kernels of a chain: each kernel waits
+// for its predecessor's completion and memory (wait), then lets its successor
+// launch as soon as all of its own blocks are running (launch_dependents); both
+// are no-ops for a kernel launched without the attribute.  Before the wait a
+// kernel may read only what its direct predecessor does not write: the matrix,
+// flags, and vectors of earlier kernels.  Those are complete, because every
+// kernel of a chain waits before it triggers its dependents, so the
+// predecessor's own wait has seen them done; a kernel that triggered first, or
+// left out the wait, would break that for the one after next.
 __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" :::);

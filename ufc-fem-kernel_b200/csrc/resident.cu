@@ -5,9 +5,11 @@
 // a CTA owns a run of SELL slices and holds their values and columns in shared
 // memory as far as they fit, a thread owns a block row and keeps the row's x, r,
 // p, q and D^-1 in registers across iterations, and what crosses CTAs is z and p
-// (one 48-byte record per row) and two sums per iteration.  An iteration has two
-// synchronisations: rows gather z_j + beta p_j (the previous direction), so the
-// new direction needs no barrier of its own.
+// (one 48-byte record per row) and two sums per iteration.  Those two sums are the
+// only synchronisations between CTAs: rows gather z_j + beta p_j (the previous
+// direction), so the new direction needs none of its own.  Inside a CTA a barrier
+// stands before each sum's last part and before the warps' parts of a row are
+// added, in the one-CTA form also between the direction and its gathers.
 //
 // Two forms by size:
 //   one CTA       up to 4 slices: __syncthreads, the direction in shared memory;

@@ -54,20 +54,9 @@ int vec_grid(int64_t n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * 8));
 }
 
-// 4 consecutive entries through 16-byte loads and stores (cudaMalloc bases are
-// 256-byte aligned; callers pass offsets that are multiples of 4 entries).
-template <typename T>
-__device__ __forceinline__ void ld4(const T* __restrict__ p, T (&o)[4]) {
-  if constexpr (sizeof(T) == 4) {
-    const float4 v = *reinterpret_cast<const float4*>(p);
-    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-  } else {
-    const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
-    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-  }
-}
-
-// The same past L1, for loads before griddepcontrol.wait.
+// 4 consecutive entries through 16-byte loads and stores (allocations are
+// 256-byte aligned; callers pass offsets that are multiples of 4 entries); the
+// loads past L1, for those before griddepcontrol.wait.
 template <typename T>
 __device__ __forceinline__ void ld4_cg(const T* __restrict__ p, T (&o)[4]) {
   if constexpr (sizeof(T) == 4) {

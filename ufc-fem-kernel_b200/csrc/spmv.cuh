@@ -214,23 +214,20 @@ __global__ void __launch_bounds__(kSpmvBlock)
 // y = K x on the full SELL storage with coded indices (see build_full_codes):
 // each row loads its 32 code bytes with two 16-byte loads when the warp
 // starts, and block j's column is row + off[code j], so no column index is
-// loaded inside the loop.  The launcher takes it with one warp per slice
-// (SPLIT = 1, as k_spmv); the SPLIT form follows k_spmv_split.  Same summation
-// order as those kernels, so the same results bit for bit.
-template <typename TV, typename TX, typename TA, class EPI, int SPLIT>
+// loaded inside the loop.  One warp per slice, as k_spmv, and the same order of
+// sums, so the same results bit for bit.
+template <typename TV, typename TX, typename TA, class EPI>
 __global__ void __launch_bounds__(kSpmvBlock)
     k_spmvc(int32_t N, int64_t nslices, const int64_t* __restrict__ sptr, const uint4* __restrict__ code,
             FullOffsets tab, const TV* __restrict__ val, const TX* __restrict__ x, EPI epi,
-           double* __restrict__ partials) {
+            double* __restrict__ partials) {
   pdl_enter();
   if (epi.halt()) return;
   __shared__ int32_t soff[32];
   if (threadIdx.x < 32) soff[threadIdx.x] = tab.off[threadIdx.x];
   __syncthreads();
-  constexpr int kWarps = kSpmvBlock / 32;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int part = warp % SPLIT;
-  const int64_t s = (int64_t)blockIdx.x * (kWarps / SPLIT) + warp / SPLIT;
+  const int lane = threadIdx.x & 31;
+  const int64_t s = (int64_t)blockIdx.x * (kSpmvBlock / 32) + (threadIdx.x >> 5);
   const int64_t row = s * kSlice + lane;
   TA a0 = TA(0), a1 = TA(0), a2 = TA(0);
   if (s < nslices) {
@@ -239,12 +236,11 @@ __global__ void __launch_bounds__(kSpmvBlock)
     const uint4 c0 = __ldcs(code + 2 * row), c1 = __ldcs(code + 2 * row + 1);
     Code256 cw{c0.x | ((uint64_t)c0.y << 32), c0.z | ((uint64_t)c0.w << 32), c1.x | ((uint64_t)c1.y << 32),
                c1.z | ((uint64_t)c1.w << 32)};
-    for (int q = 0; q < part; ++q) cw.template drop<1>();
     const TV* vp = val + 9 * base + lane;
 #pragma unroll 2
-    for (int j = part; j < len; j += SPLIT) {
+    for (int j = 0; j < len; ++j) {
       const unsigned cd = cw.front();
-      cw.template drop<SPLIT>();
+      cw.drop();
       TA x0 = TA(0), x1 = TA(0), x2 = TA(0);
       if (cd != 255u) {
         const int64_t cj = row + soff[cd];
@@ -258,25 +254,8 @@ __global__ void __launch_bounds__(kSpmvBlock)
       a2 += (TA)__ldcs(v + 192) * x0 + (TA)__ldcs(v + 224) * x1 + (TA)__ldcs(v + 256) * x2;
     }
   }
-  if constexpr (SPLIT > 1) {
-    __shared__ TA sh[kWarps][3][32];
-    sh[warp][0][lane] = a0;
-    sh[warp][1][lane] = a1;
-    sh[warp][2][lane] = a2;
-    __syncthreads();
-    if (part == 0) {
-#pragma unroll
-      for (int q = 1; q < SPLIT; ++q) {
-        a0 += sh[warp + q][0][lane];
-        a1 += sh[warp + q][1][lane];
-        a2 += sh[warp + q][2][lane];
-      }
-    }
-  }
   double dot[1] = {0.0};
-  if (part == 0 && s < nslices && row < N) {
-    dot[0] = epi(row, a0, a1, a2, x);
-  }
+  if (s < nslices && row < N) dot[0] = epi(row, a0, a1, a2, x);
   if (EPI::kDot && epi.want_dot()) block_partial<1>(dot, partials);
 }
 
@@ -705,11 +684,13 @@ int launch_spmv_split(const Ctx* c, cudaStream_t st, const TV* val, const TX* x,
   // with SPLIT warps per slice each warp loads the row's 32 code bytes, more
   // than its share of 4-byte columns: J2 bar 53.7 against 51.8 us per CG
   // iteration)
-  if (!DIFF && SPLIT == 1 && sizeof(TV) == 4 && c->full_coded) {
-    constexpr int per_block = kSpmvBlock / 32 / SPLIT;
-    const int grid = (int)((c->nslices + per_block - 1) / per_block);
-    return launch_product<EPI::kPdl>(k_spmvc<TV, TX, TA, EPI, SPLIT>, grid, kSpmvBlock, st, c->N, c->nslices, c->slice_ptr,
-                             reinterpret_cast<const uint4*>(c->full_code), c->full_tab, val, x, epi, c->partials);
+  if constexpr (!DIFF && SPLIT == 1 && sizeof(TV) == 4) {
+    if (c->full_coded) {
+      constexpr int per_block = kSpmvBlock / 32;
+      const int grid = (int)((c->nslices + per_block - 1) / per_block);
+      return launch_product<EPI::kPdl>(k_spmvc<TV, TX, TA, EPI>, grid, kSpmvBlock, st, c->N, c->nslices, c->slice_ptr,
+                               reinterpret_cast<const uint4*>(c->full_code), c->full_tab, val, x, epi, c->partials);
+    }
   }
   if constexpr (SPLIT == 1) {
     const int grid = (int)((c->nslices * kSlice + kSpmvBlock - 1) / kSpmvBlock);
@@ -770,7 +751,6 @@ int launch_spmv_sym(const Ctx* c, cudaStream_t st, const TV* val, const TX* x, c
     default: return launch_spmv_sym_split<TV, TX, TA, 8>(c, st, val, x, epi);
   }
 }
-
 
 // Sum of the nb per-block partials of the product, for grids too large to be
 // summed again by every block of the update: one block, result in out[0].

@@ -64,20 +64,11 @@ enum DevErr : int32_t {
 struct Code256 {
   uint64_t w0, w1, w2, w3;
   __device__ __forceinline__ unsigned front() const { return (unsigned)(w0 & 0xFFu); }
-  template <int B>
   __device__ __forceinline__ void drop() {
-    if constexpr (B >= 8) {
-      w0 = w1;
-      w1 = w2;
-      w2 = w3;
-      w3 = 0;
-    } else {
-      constexpr int sh = 8 * B;
-      w0 = (w0 >> sh) | (w1 << (64 - sh));
-      w1 = (w1 >> sh) | (w2 << (64 - sh));
-      w2 = (w2 >> sh) | (w3 << (64 - sh));
-      w3 >>= sh;
-    }
+    w0 = (w0 >> 8) | (w1 << 56);
+    w1 = (w1 >> 8) | (w2 << 56);
+    w2 = (w2 >> 8) | (w3 << 56);
+    w3 >>= 8;
   }
 };
 
@@ -222,7 +213,6 @@ struct Ctx {
   const void* cg_graph_key[kGraphSlots] = {};
   int cg_graph_form[kGraphSlots] = {};
   int64_t cg_graph_n[kGraphSlots] = {}, cg_graph_slices[kGraphSlots] = {};
-  std::vector<cudaEvent_t> ev_pool;
 };
 
 int grid_for(int64_t work, int block);
@@ -272,13 +262,10 @@ int face_loads(Ctx* c, int32_t n_faces, const int32_t* h_elem, const int32_t* h_
                const double* pressure, double* f);  // h_elem 0-based, h_face 1..6 (host); others device
 int stress_nodal(Ctx* c, const double* u, double* sig_node, double* vm_node);
 int reactions(Ctx* c, const double* u, const double* f_ext, double* rf);
-int build_dinv(Ctx* c, int precision);
 
-// spmv.cu
+// solver.cu, block.cu
 int spmv(Ctx* c, int precision, const void* x, void* y);
 int64_t spmv_bytes(const Ctx* c, int precision);
-
-// pcg.cu
 int pcg_solve(Ctx* c, const double* b, double* x, const ufc_solver_algo* algo, ufc_solver_state* st);
 int pcg_solve_block(Ctx* c, int nrhs, const double* B, double* X, const ufc_solver_algo* algo,
                     ufc_solver_state* st);
