@@ -442,11 +442,29 @@ void orc_spmv(int64_t n, const int64_t* row_ptr, const int32_t* col, const doubl
   }
 }
 
-static double orc_dot(int64_t n, const double* a, const double* b) {
+/* Dot products are summed over blocks of fixed size, and the blocks' sums in
+ * order, so that a solve gives the same bits whatever the number of threads and
+ * the order in which they finish: at the yield surface of a homogeneous bar the
+ * last bit of the displacement decides which points are plastic. */
+enum { ORC_BLOCK = 4096 };
+
+static int64_t orc_block_end(int64_t k, int64_t n) { return (k + 1) * ORC_BLOCK < n ? (k + 1) * ORC_BLOCK : n; }
+
+static double orc_sum(int64_t m, const double* part) {
   double s = 0.0;
-#pragma omp parallel for schedule(static) reduction(+ : s)
-  for (int64_t i = 0; i < n; ++i) s += a[i] * b[i];
+  for (int64_t k = 0; k < m; ++k) s += part[k];
   return s;
+}
+
+static double orc_dot(int64_t n, const double* a, const double* b, double* part) {
+  const int64_t m = (n + ORC_BLOCK - 1) / ORC_BLOCK;
+#pragma omp parallel for schedule(static)
+  for (int64_t k = 0; k < m; ++k) {
+    double s = 0.0;
+    for (int64_t i = k * ORC_BLOCK; i < orc_block_end(k, n); ++i) s += a[i] * b[i];
+    part[k] = s;
+  }
+  return orc_sum(m, part);
 }
 
 /* Jacobi-PCG, iter_pcg semantics (NM_Solv_IterSolver.f90:713-846):
@@ -471,6 +489,8 @@ static int pcg_impl(int64_t n, const int64_t* row_ptr, const int32_t* col, const
   double* p = (double*)malloc(sizeof(double) * (size_t)n);
   double* q = (double*)malloc(sizeof(double) * (size_t)n);
   double* dinv = (double*)malloc(sizeof(double) * (size_t)n);
+  const int64_t nblk = (n + ORC_BLOCK - 1) / ORC_BLOCK;
+  double* part = (double*)malloc(sizeof(double) * (size_t)nblk);
   int fixed_count = max_iter <= 0;
   int maxit = fixed_count ? -max_iter : max_iter;
 #pragma omp parallel for schedule(static)
@@ -483,8 +503,8 @@ static int pcg_impl(int64_t n, const int64_t* row_ptr, const int32_t* col, const
   orc_spmv(n, row_ptr, col, val, x, r);
 #pragma omp parallel for schedule(static)
   for (int64_t i = 0; i < n; ++i) r[i] = b[i] - r[i];
-  double bnorm = sqrt(orc_dot(n, b, b));
-  double rnorm = sqrt(orc_dot(n, r, r));
+  double bnorm = sqrt(orc_dot(n, b, b, part));
+  double rnorm = sqrt(orc_dot(n, r, r, part));
   if (res_init) *res_init = rnorm;
   if (bnorm < 1e-30) bnorm = 1.0;
   double tol = rtol * bnorm > atol ? rtol * bnorm : atol;
@@ -499,23 +519,26 @@ static int pcg_impl(int64_t n, const int64_t* row_ptr, const int32_t* col, const
     z[i] = dinv[i] * r[i];
     p[i] = z[i];
   }
-  double rho = orc_dot(n, r, z);
+  double rho = orc_dot(n, r, z, part);
   for (k = 1; k <= maxit; ++k) {
     orc_spmv(n, row_ptr, col, val, p, q);
-    double pq = orc_dot(n, p, q);
+    double pq = orc_dot(n, p, q, part);
     if (fabs(pq) < 1e-300) {
       status = ORC_ERROR;
       break;
     }
     double alpha = rho / pq;
-    double rr = 0.0;
-#pragma omp parallel for schedule(static) reduction(+ : rr)
-    for (int64_t i = 0; i < n; ++i) {
-      x[i] += alpha * p[i];
-      r[i] -= alpha * q[i];
-      rr += r[i] * r[i];
+#pragma omp parallel for schedule(static)
+    for (int64_t j = 0; j < nblk; ++j) {
+      double rr = 0.0;
+      for (int64_t i = j * ORC_BLOCK; i < orc_block_end(j, n); ++i) {
+        x[i] += alpha * p[i];
+        r[i] -= alpha * q[i];
+        rr += r[i] * r[i];
+      }
+      part[j] = rr;
     }
-    rnorm = sqrt(rr);
+    rnorm = sqrt(orc_sum(nblk, part));
     if (mark_tol > 0.0 && rnorm <= mark_tol) {
       if (t_mark) *t_mark = omp_get_wtime() - t_start;
       if (it_mark) *it_mark = k;
@@ -526,12 +549,16 @@ static int pcg_impl(int64_t n, const int64_t* row_ptr, const int32_t* col, const
       status = ORC_OK;
       break;
     }
-    double rho_new = 0.0;
-#pragma omp parallel for schedule(static) reduction(+ : rho_new)
-    for (int64_t i = 0; i < n; ++i) {
-      z[i] = dinv[i] * r[i];
-      rho_new += r[i] * z[i];
+#pragma omp parallel for schedule(static)
+    for (int64_t j = 0; j < nblk; ++j) {
+      double s = 0.0;
+      for (int64_t i = j * ORC_BLOCK; i < orc_block_end(j, n); ++i) {
+        z[i] = dinv[i] * r[i];
+        s += r[i] * z[i];
+      }
+      part[j] = s;
     }
+    const double rho_new = orc_sum(nblk, part);
     if (fabs(rho) < 1e-300) {
       status = ORC_ERROR;
       break;
@@ -545,7 +572,7 @@ static int pcg_impl(int64_t n, const int64_t* row_ptr, const int32_t* col, const
 done:
   if (iters) *iters = k;
   if (res_final) *res_final = rnorm;
-  free(r); free(z); free(p); free(q); free(dinv);
+  free(r); free(z); free(p); free(q); free(dinv); free(part);
   return status;
 }
 
