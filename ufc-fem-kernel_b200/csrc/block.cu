@@ -979,8 +979,10 @@ void launch_bspmv_tile(const BlockRun& B, cudaStream_t st, int mode, const doubl
                                                     B.partials, c->dev_err);
 }
 
-cudaError_t prepare_tile(const BTile& T) {
-  const int sm = (int)(2 * tile_stage_bytes(T.nodes));
+// The limit of the largest tile, whatever this one takes: it belongs to the process
+// (another thread may be about to launch).
+cudaError_t prepare_tile() {
+  constexpr int sm = (int)(2 * tile_stage_bytes(kTileMaxNodes));
   cudaError_t e = cudaFuncSetAttribute(k_bspmv_tile<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_bspmv_tile<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   return e;
@@ -1184,7 +1186,7 @@ int pcg_solve_block(Ctx* c, int nrhs, const double* Bm, double* X, const ufc_sol
   if (G == 2) UFC_CUDA(c, prepare_bspmv(B.tpr));
   B.tile = nr == kTileNr && make_tile(c, &B.T);
   B.g_tile = (int)std::min<int64_t>(2 * c->nslices, (int64_t)sm_count());
-  if (B.tile) UFC_CUDA(c, prepare_tile(B.T));
+  if (B.tile) UFC_CUDA(c, prepare_tile());
   B.g_vec = grid_blocks(c->n * B.tpr);
   B.g_upd = (int)std::min<int64_t>((c->n * B.tpr + kVecBlk - 1) / kVecBlk, 2 * (int64_t)sm_count());
   BScalars* hs = nullptr;

@@ -861,6 +861,9 @@ int element_lame(Ctx* c) {
   return UFC_STATUS_OK;
 }
 
+// The kernels' limit of dynamic shared memory is set to the most there is and not to
+// what a launch takes: it belongs to the process, so another thread that assembles
+// a mesh with shorter rows would lower it between this thread's setting and launch.
 template <typename T, bool kTangent>
 static int launch_assemble(Ctx* c, const RowOutputs<T>& to) {
   const int stride = (9 * c->max_row_blocks) | 1;  // odd: the rows of an entry lie in different banks
@@ -868,7 +871,7 @@ static int launch_assemble(Ctx* c, const RowOutputs<T>& to) {
     // while the slice's accumulators fit in shared memory
     const int bytes = kIsoXBytes + (int)sizeof(T) * kSlice * stride;
     if (bytes <= kAsmMaxSmem) {
-      UFC_CUDA(c, cudaFuncSetAttribute(k_assemble_iso<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+      UFC_CUDA(c, cudaFuncSetAttribute(k_assemble_iso<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAsmMaxSmem));
       k_assemble_iso<T><<<(int)c->nslices, kIsoThreads, bytes, c->stream>>>(
           c->N, c->nptr, c->nelem, c->coords, c->conn, c->lame, c->slot, c->slice_ptr, c->sell_col, c->dpos, c->fixed,
           stride, to, c->dev_err);
@@ -877,7 +880,8 @@ static int launch_assemble(Ctx* c, const RowOutputs<T>& to) {
     }
   }
   const int bytes = (int)(sizeof(AsmWarp<T, kTangent>) * kAsmWarps + sizeof(T) * kAsmRows * stride);
-  UFC_CUDA(c, cudaFuncSetAttribute(k_assemble_rows<T, kTangent>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  UFC_CUDA(c, cudaFuncSetAttribute(k_assemble_rows<T, kTangent>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   kAsmMaxSmem));
   k_assemble_rows<T, kTangent><<<(int)(2 * c->nslices), kAsmWarps * 32, bytes, c->stream>>>(
       c->N, c->nptr, c->nelem, c->coords, c->conn, c->lame, c->Dt, c->slot, c->slice_ptr, c->sell_col, c->dpos,
       c->fixed, stride, to, c->dev_err);

@@ -1097,8 +1097,7 @@ int mg_numeric(Ctx* c) {
       UFC_TRY(mg_alloc(c, &L.dinv32, lc->n));
     }
     const int stride = (9 * lc->max_row_blocks) | 1;
-    const int bytes = (int)sizeof(double) * kMgRows * stride;
-    UFC_CUDA(c, cudaFuncSetAttribute(k_mg_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    const int bytes = (int)sizeof(double) * kMgRows * stride;  // (27 blocks a row at most: 31 KB, no limit to raise)
     RowOutputs<double> to;
     to.val = lc->val64;
     to.dinv = lc->dinv64;
