@@ -505,33 +505,42 @@ __global__ void __launch_bounds__(kIsoThreads, 2)
 
 // Lower blocks from the upper ones, transposed.  The J2 block (a, b) is formed as
 // (D B_a)^T B_b and (b, a) as (D B_b)^T B_a, the same but for rounding; the upper
-// one stands for both, as in the symmetric storage.  One thread per block row; a
-// Newton increment at 64x32x32 takes 188.8 ms with it, 188.2 without.
+// one stands for both, as in the symmetric storage.  A CTA per slice, its warps
+// take the rows' entries in turn, so that a thread's chain (column, search in that
+// column's row, block) is short and the stores of an entry's 32 rows lie together:
+// bound by the latency of that chain.  Tangent assembly at 16x8x8, 32x16x16 and
+// 64x32x32 without it / with it / with one thread per row: 62 / 70 / 115, 120 / 126
+// / 173 and 436 / 467 / 524 us.
+constexpr int kMirrorWarps = 8;
+
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kMirrorWarps * 32)
     k_mirror_lower(int32_t N, const int32_t* __restrict__ brow, const int32_t* __restrict__ bcol,
                    const int64_t* __restrict__ sptr, T* __restrict__ val, float* __restrict__ val_r) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t s = blockIdx.x, r = s * kSlice + (threadIdx.x & 31);
   if (r >= N) return;
-  const int64_t P0 = sptr[r >> 5] + (r & 31);
+  const int64_t P0 = sptr[s] + (threadIdx.x & 31);
   const int32_t b = brow[r], e = brow[r + 1];
-  for (int32_t k = b; k < e; ++k) {
+  for (int32_t k = b + (int32_t)(threadIdx.x >> 5); k < e; k += kMirrorWarps) {
     const int32_t c = bcol[k];
     if (c >= r) break;
     int32_t lo = brow[c], hi = brow[c + 1] - 1;  // row c holds column r: the pattern is symmetric
+    const int32_t first = lo;
     while (lo < hi) {
       const int32_t mid = (lo + hi) >> 1;
       if (bcol[mid] < r) lo = mid + 1;
       else hi = mid;
     }
-    const int64_t src = sptr[c >> 5] + 32 * (int64_t)(lo - brow[c]) + (c & 31), dst = P0 + 32 * (int64_t)(k - b);
+    const int64_t src = sptr[c >> 5] + 32 * (int64_t)(lo - first) + (c & 31), dst = P0 + 32 * (int64_t)(k - b);
+    T v[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) v[q] = val[vpos(src, q)];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
-        const T v = val[vpos(src, 3 * j + i)];
-        val[vpos(dst, 3 * i + j)] = v;
-        if (val_r) val_r[vpos(dst, 3 * i + j)] = (float)v;
+        val[vpos(dst, 3 * i + j)] = v[3 * j + i];
+        if (val_r) val_r[vpos(dst, 3 * i + j)] = (float)v[3 * j + i];
       }
   }
 }
@@ -886,7 +895,8 @@ static int launch_assemble(Ctx* c, const RowOutputs<T>& to) {
       c->N, c->nptr, c->nelem, c->coords, c->conn, c->lame, c->Dt, c->slot, c->slice_ptr, c->sell_col, c->dpos,
       c->fixed, stride, to, c->dev_err);
   if (kTangent)
-    k_mirror_lower<T><<<grid_for(c->N, 128), 128, 0, c->stream>>>(c->N, c->brow, c->bcol, c->slice_ptr, to.val, to.val_r);
+    k_mirror_lower<T><<<(int)c->nslices, kMirrorWarps * 32, 0, c->stream>>>(c->N, c->brow, c->bcol, c->slice_ptr, to.val,
+                                                                            to.val_r);
   UFC_CUDA(c, cudaGetLastError());
   return UFC_STATUS_OK;
 }
