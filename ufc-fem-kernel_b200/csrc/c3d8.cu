@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kAsmWarps * 32)
 // is worked on.  The Jacobian's node sums (see above) are taken per eta and zeta
 // for both faces xi = -1 and +1, so that they read the coordinates no oftener
 // than differences along the edges would.  128x64x64, FP64 with FP32 copies, the
-// call with its products: 1.78 ms (1.66 ms with edge differences; node sums
+// call with its products: 1.80 ms (1.66 ms with edge differences; node sums
 // formed at every Gauss point 2.26 ms; the colour-ordered element scatter before
 // 6.26 ms).  The kernel is bound by latency and FP64 (8 warps per SM; the
 // accumulators take the registers).
